@@ -1,41 +1,37 @@
 // fast_rcp.cuh -- reciprocal and square root for the fast floating-point mode.
 //
-// 1/d by Newton-Raphson iteration from the hardware's approximate reciprocal
-// (PTX rcp.approx.ftz.f64): y <- y + y*(1 - d*y), twice, each step an FMA pair
-// (the FMA form of Newton's iteration for 1/d, P. Markstein, IBM J. Res. Dev.
-// 34(1):111-119, 1990).  Each step squares the relative error, so the result
-// is within a few ulp of 1/d for normal d; it is not correctly rounded.  Four
-// FP64 pipe instructions against about seven and a half for an IEEE division.
-// A zero or subnormal d gives NaN (the approximation flushes it to zero).
+// Both correct the hardware's approximation once, with the residual's series
+// to third order instead of two Newton steps: on this part an FP64 instruction
+// costs an SM 16-19 cycles and a lone warp 64, so their number is what counts.
 //
-// sqrt(x) from the hardware's approximate reciprocal square root y ~ 1/sqrt(x)
-// (PTX rsqrt.approx.ftz.f64) by the coupled iteration of the same paper: with
-// g ~ sqrt(x) = x*y and h ~ 1/(2 sqrt(x)) = y/2, the residual r = 1/2 - g*h
-// corrects both (g += g*r, h += h*r), which squares the relative error; a last
-// step g += h*(x - g*g) (Newton's step for g^2 = x, its residual by one FMA)
-// squares it again.  Seven FP64 pipe instructions and one approximation, no
-// branch; within a few ulp of sqrt(x) for positive normal x, not correctly
-// rounded.  Zero, subnormal and infinite x give NaN, and so do negative x (as
-// sqrt does); the solver takes it only of a pressure over a density that it
-// has already tested, or will test, for positivity.
+// 1/d from y ~ 1/d (PTX rcp.approx.ftz.f64): with e = 1 - d*y,
+// 1/d = y/(1 - e) = y + y*(e + e^2) + O(e^3), the cubic ("hyperpower")
+// iteration of M. Altman, Pacific J. Math. 10(4):1107-1113, 1960.  Measured
+// |e| <= 2^-19.9, so the remainder is 2^-59.8: within an ulp or so of 1/d for
+// normal d, not correctly rounded.  Three FP64 instructions; the two Newton
+// steps it replaces took four, an IEEE division takes about seven and a half.
+// A zero or subnormal d gives NaN.
+//
+// sqrt(x) from y ~ 1/sqrt(x) (PTX rsqrt.approx.ftz.f64): with g = x*y and
+// e = 1 - g*y, sqrt(x) = g*(1 - e)^(-1/2) = g + g*e*(1/2 + 3/8 e) + O(e^3)
+// (the binomial series).  Measured |e| <= 2^-19, remainder 2^-58.7.  Five FP64
+// instructions and no branch (seven before); within an ulp or so for positive
+// normal x, not correctly rounded.  Zero, negative and infinite x give NaN;
+// the solver takes it only of a pressure over a density that it has already
+// tested, or will test, for positivity.
 #pragma once
 
 __device__ __forceinline__ double gpm_fast_rcp(double d) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    double e = fma(-d, y, 1.0);
-    y = fma(y, e, y);
-    e = fma(-d, y, 1.0);
-    return fma(y, e, y);
+    const double e = fma(-d, y, 1.0);
+    return fma(y, fma(e, e, e), y);
 }
 
 __device__ __forceinline__ double gpm_fast_sqrt(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    double g = x * y, h = 0.5 * y;
-    const double r = fma(-g, h, 0.5);
-    g = fma(g, r, g);
-    h = fma(h, r, h);
-    const double e = fma(-g, g, x);
-    return fma(h, e, g);
+    const double g = x * y;
+    const double e = fma(-g, y, 1.0);
+    return fma(g * e, fma(0.375, e, 0.5), g);
 }
