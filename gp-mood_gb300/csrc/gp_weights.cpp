@@ -270,14 +270,39 @@ extern "C" int gpm_gp_presim(double ell_o_dx, double lx, double ly, int lf, int 
             c13[11] = 0.25 * (za + zb - zc - zd);
             c13[12] = 0.25 * (za - zb - zc + zd);
         };
+        GpOrbit& d = out->orbd;
         double c[13];
-        split(out->zt[2][0][0], out->orb.x0);
+        split(out->zt[2][0][0], d.x0);
         split(out->zt[2][0][1], c);
-        for (int k = 0; k < 9; k++) out->orb.x1[k] = c[k];  // y-symmetric: groups 3, 4 vanish
-        split(out->zt[2][3][0], out->orb.y0);
+        for (int k = 0; k < 9; k++) d.x1[k] = c[k];  // y-symmetric: groups 3, 4 vanish
+        split(out->zt[2][3][0], d.y0);
         split(out->zt[2][3][1], c);
-        for (int k = 0; k < 6; k++) out->orb.y1[k] = c[k];  // x-symmetric: groups 2, 4 vanish
-        for (int k = 0; k < 3; k++) out->orb.y1[6 + k] = c[9 + k];
+        for (int k = 0; k < 6; k++) d.y1[k] = c[k];  // x-symmetric: groups 2, 4 vanish
+        for (int k = 0; k < 3; k++) d.y1[6 + k] = c[9 + k];
+        // w * 2^58, split in two signed halves; nc: stencil cells in each component
+        static const int nc[13] = {1, 2, 2, 2, 2, 4, 2, 2, 4, 2, 2, 4, 4};
+        static const int id[13] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12};
+        static const int swap[13] = {0, 3, 4, 1, 2, 5, 9, 10, 11, 6, 7, 8, 12};  // y faces: n is y, t is x
+        static const int swap9[9] = {0, 3, 4, 1, 2, 5, 6, 7, 8};
+        FixOrbit& orb = out->orb;
+        orb.ok = 1;
+        auto store = [&](const double* w, const int* order, int n, FixWeight* fw) {
+            double sum = 0.0;
+            for (int i = 0; i < n; i++) sum += fabs(w[order[i]]) * nc[i];
+            if (!(sum <= 4.0)) {
+                orb.ok = 0;
+                return;
+            }
+            for (int i = 0; i < n; i++) {
+                const long long v = llrint(ldexp(w[order[i]], 58));
+                fw[i].h = (int)((v + (1LL << 29)) >> 30);
+                fw[i].l = (int)(v - ((long long)fw[i].h << 30));
+            }
+        };
+        store(d.x0, id, 13, orb.w0[0]);
+        store(d.x1, id, 9, orb.w1[0]);
+        store(d.y0, swap, 13, orb.w0[1]);
+        store(d.y1, swap9, 9, orb.w1[1]);
     }
     return 0;
 }

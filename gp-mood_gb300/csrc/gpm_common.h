@@ -62,6 +62,19 @@ __host__ __device__ constexpr int gpm_sym_pair(int dir, int k, int side) {
 struct GpOrbit {
     double x0[13], x1[9], y0[13], y1[9];
 };
+// The same weights in 58-bit fixed point, split for 32-bit multiplies:
+// w = (h * 2^30 + l) * 2^-58, |l| <= 2^29 (fixed_recon.cuh).  [axis 0: x faces,
+// 1: y faces]; components in the axis's own frame (n: along it, t: across it):
+// [Q0 Q1p Q2p Q3p Q4p Q5pp | Q1m Q2m Q5mp | Q3m Q4m Q5pm | Q5mm] with Q1, Q2 the
+// pairs along n and Q3, Q4 along t.
+struct FixWeight {
+    int h, l;
+};
+struct FixOrbit {
+    FixWeight w0[2][13], w1[2][9];
+    int ok;  // the weights are in the fixed-point form's range; 0: the fast first pass runs per face instead
+    int pad;
+};
 
 struct GpSym {
     double a0[5], a1[5];         // axis weights of Gauss points 0 and 1
@@ -75,7 +88,8 @@ struct GpWeights {
     double gw[GPM_MAXGP];            // gauss_weight(ngp, :)
     double d2x[5], d2y[5];           // GP_d2x_sp(3,:), GP_d2y_sp(3,:)
     GpSym sym[3][4];                 // ngp = 3 split of zt (fast mode); zero otherwise
-    GpOrbit orb;                     // ngp = 3 order-5 cell-wise split (fast mode); zero otherwise
+    FixOrbit orb;                    // ngp = 3 order-5 cell-wise split (fast mode); zero otherwise
+    GpOrbit orbd;                    // ... in doubles (batched form)
 };
 
 struct GridGeom {

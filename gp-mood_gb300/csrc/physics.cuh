@@ -269,14 +269,20 @@ __device__ __forceinline__ bool hllc_normal(double rL, double nL, double tL, dou
                         __double_as_longlong(vR) >= __double_as_longlong(cR);              // S_L >= 0
     const bool superR = bits_of(vL) > bits_of(-cL) && bits_of(vR) > bits_of(-cR);          // S_R < 0
     const bool left = superL || !(bits_of(us) > 0x8000000000000000ULL);                    // u* >= 0 (-0 too)
+    const bool super = superL || (superR && !left);
+    // A supersonic side's flux must not feel the other side, not even in its
+    // rounding, and its mass flux is the momentum itself: a cell upwind of a
+    // jump keeps its density exactly then, and the density bounds of DETECTION
+    // hold with equality.  So S - v := 1 there, a = rho and q = 1.
     const double v = left ? vL : vR;
-    us = superL || (superR && !left) ? v : us;
-    const double w = us - v, a = left ? aL : aR, d = left ? dL : dR;
+    us = super ? v : us;
+    const double w = us - v;
+    const double a = super ? (left ? rL : rR) : (left ? aL : aR), d = super ? 1. : (left ? dL : dR);
     const double p = left ? pL : pR, vt = left ? wL : wR, e = left ? eL : eR;
     const double ps = fma(a, w, p);
     const double q = gpm_fast_rcp(d - w);  // 1 / (S - u*)
     const double m = a * q * us;
-    F.r = m;
+    F.r = super ? (left ? nL : nR) : m;
     F.n = fma(m, us, ps);
     F.t = m * vt;
     F.e = us * fma(fma(w, fma(a, us, p), e * d), q, ps);

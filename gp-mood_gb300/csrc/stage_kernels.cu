@@ -32,6 +32,7 @@
 // cell's Uout from Uin and its four current face fluxes, in the reference's
 // accumulation order, reproduces the reference bit for bit.
 #include "physics.cuh"
+#include "fixed_recon.cuh"
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -292,226 +293,194 @@ __global__ void __launch_bounds__(TX * TY) k_flux_tile(StageArgs a, const __grid
     st_cell(out, Cell{F[0], F[1], F[2], F[3]});
 }
 
-template <int DIR, int NP, int NGP>
+// The Riemann solve and quadrature a face function uses; the batched form has
+// its own in fast mode (batch_fast.cuh).
+struct FaceMath {
+    template <int DIR, int NGP>
+    static __device__ __forceinline__ void quad(const double (*uL)[4], const double (*uR)[4], const double* gw,
+                                                double* F, int nflux) {
+        quad_flux<DIR, NGP>(uL, uR, gw, F, nflux);
+    }
+    template <int DIR>
+    static __device__ __forceinline__ void solve(int nflux, const double* uL, const double* uR, double* F) {
+        riemann<DIR>(nflux, uL, uR, F);
+    }
+};
+
+template <int DIR, int NP, int NGP, class M = FaceMath>
 __device__ __forceinline__ void face_global(const GridGeom& g, const GpWeights& w, int o, const double* __restrict__ uin,
                                             size_t c0, double* F);
 
 #if !GPM_EXACT
 // ---------------------------------------------------------------------------
 // Fast first pass at uniform order 5 with ngp = 3: both face directions of a
-// tile of cells in one CTA.  Every cell's 12 face states (left/right/bottom/
-// top faces at 3 Gauss points) come from the mirror-symmetry components of its
-// 13-point stencil (GpOrbit): 16 operations form the components, 32 give the
-// six x-face states and 32 the six y-face states, per variable -- 80 FP64
-// operations for 12 states, against 128 when each face gathers its two states
-// on its own.  A cell passes its left and bottom states to its neighbours
-// through shared memory, keeps its right states in registers and parks its
-// top states in shared memory too (registers for the three Gauss points'
-// Riemann solves, which run together); then every thread solves the x face
-// and the y face of which its cell is the low side.  Tiles own the interior cells (l0..l0+XT-1, n0..n0+XY-1), l0, n0 >= 1;
-// one extra column (left states) and row (bottom states) is computed by two
-// warps.  The faces whose low cell is a ghost -- x faces (0,n), y faces (l,0)
-// -- are 32-face edge items computed face by face (edge_faces).
-constexpr int XT = 32, XY = 8;          // cells per tile
-constexpr int XS = 13;                  // doubles per published state set (12 used, padded)
-
-struct XyOut {
-    double lo[3][4];  // left (x) or bottom (y) face states
-    double hi[3][4];  // right (x) or top (y) face states
-};
-
-__device__ __forceinline__ double tile_var(const Cell* t, int k) { return cell_var(*t, k); }
-
-// Components of the stencil values of variable k around tile position (cx, cy).
-struct Comp {
-    double v[13];  // [Q0 Q1p Q2p Q3p Q4p Q5pp Q1m Q2m Q5mp Q3m Q4m Q5pm Q5mm]
-};
-
-__device__ __forceinline__ void components(const Cell (*tile)[XT + 5], int cx, int cy, int k, Comp& c) {
-    auto q = [&](int ox, int oy) { return cell_var(tile[cy + oy][cx + ox], k); };
-    const double qm1 = q(-1, 0), qp1 = q(1, 0), qm2 = q(-2, 0), qp2 = q(2, 0);
-    const double qb1 = q(0, -1), qt1 = q(0, 1), qb2 = q(0, -2), qt2 = q(0, 2);
-    const double a = q(-1, -1), b = q(1, -1), cc = q(-1, 1), d = q(1, 1);
-    c.v[0] = q(0, 0);
-    c.v[1] = qm1 + qp1;
-    c.v[2] = qm2 + qp2;
-    c.v[3] = qb1 + qt1;
-    c.v[4] = qb2 + qt2;
-    const double s1 = a + b, s2 = cc + d, d1 = a - b, d2 = cc - d;
-    c.v[5] = s1 + s2;
-    c.v[6] = qm1 - qp1;
-    c.v[7] = qm2 - qp2;
-    c.v[8] = d1 + d2;
-    c.v[9] = qb1 - qt1;
-    c.v[10] = qb2 - qt2;
-    c.v[11] = s1 - s2;
-    c.v[12] = d1 - d2;
-}
-
-// x family: left (lo) and right (hi) face states at Gauss points 0, 1, 2.
-__device__ __forceinline__ void x_family(const GpOrbit& o, const Comp& c, int k, XyOut& r) {
-    const double Ppp = o.x0[0] * c.v[0] + o.x0[1] * c.v[1] + o.x0[2] * c.v[2] + o.x0[3] * c.v[3] +
-                       o.x0[4] * c.v[4] + o.x0[5] * c.v[5];
-    const double Pmp = o.x0[6] * c.v[6] + o.x0[7] * c.v[7] + o.x0[8] * c.v[8];
-    const double Ppm = o.x0[9] * c.v[9] + o.x0[10] * c.v[10] + o.x0[11] * c.v[11];
-    const double Pmm = o.x0[12] * c.v[12];
-    const double A = Ppp + Ppm, B = Pmp + Pmm, C = Ppp - Ppm, D = Pmp - Pmm;
-    r.lo[0][k] = A + B;
-    r.hi[0][k] = A - B;
-    r.lo[2][k] = C + D;
-    r.hi[2][k] = C - D;
-    const double P1pp = o.x1[0] * c.v[0] + o.x1[1] * c.v[1] + o.x1[2] * c.v[2] + o.x1[3] * c.v[3] +
-                        o.x1[4] * c.v[4] + o.x1[5] * c.v[5];
-    const double P1mp = o.x1[6] * c.v[6] + o.x1[7] * c.v[7] + o.x1[8] * c.v[8];
-    r.lo[1][k] = P1pp + P1mp;
-    r.hi[1][k] = P1pp - P1mp;
-}
-
-// y family: bottom (lo) and top (hi) face states at Gauss points 0, 1, 2.
-__device__ __forceinline__ void y_family(const GpOrbit& o, const Comp& c, int k, XyOut& r) {
-    const double Ppp = o.y0[0] * c.v[0] + o.y0[1] * c.v[1] + o.y0[2] * c.v[2] + o.y0[3] * c.v[3] +
-                       o.y0[4] * c.v[4] + o.y0[5] * c.v[5];
-    const double Pmp = o.y0[6] * c.v[6] + o.y0[7] * c.v[7] + o.y0[8] * c.v[8];
-    const double Ppm = o.y0[9] * c.v[9] + o.y0[10] * c.v[10] + o.y0[11] * c.v[11];
-    const double Pmm = o.y0[12] * c.v[12];
-    const double A = Ppp + Ppm, B = Pmp + Pmm, C = Ppp - Ppm, D = Pmp - Pmm;
-    r.lo[0][k] = A + B;
-    r.lo[2][k] = A - B;
-    r.hi[0][k] = C + D;
-    r.hi[2][k] = C - D;
-    const double P1pp = o.y1[0] * c.v[0] + o.y1[1] * c.v[1] + o.y1[2] * c.v[2] + o.y1[3] * c.v[3] +
-                        o.y1[4] * c.v[4] + o.y1[5] * c.v[5];
-    const double P1pm = o.y1[6] * c.v[9] + o.y1[7] * c.v[10] + o.y1[8] * c.v[11];
-    r.lo[1][k] = P1pp + P1pm;
-    r.hi[1][k] = P1pp - P1pm;
-}
-
-__device__ __forceinline__ void publish(double* dst, const double (*st)[4]) {
-#pragma unroll
-    for (int g = 0; g < 3; g++)
-#pragma unroll
-        for (int k = 0; k < 4; k++) dst[4 * g + k] = st[g][k];
-}
+// tile of cells in one CTA.  A cell's six states on an axis's two faces come
+// from the mirror-symmetry components of its 13-point stencil (FixOrbit) in
+// fixed point, on the integer pipe (fixed_recon.cuh), so the FP64 pipe, which
+// bounds this kernel, runs only the Riemann solves: 192 FP64 instructions per
+// face instead of 350 with FP64 sums.  After staging, a CTA turns its tile
+// into signed mantissas (in place) and 16-bit exponents once.  Then, for x and
+// for y: every cell's states go to shared memory, its far-face (right, top)
+// states in its own slot and its near-face (left, bottom) states in the slot
+// of the neighbour that shares the face, and every thread solves the face of
+// which its cell is the low side.  Both axes and all four variables run the
+// same code (an axis's frame is a pair of strides): unrolled, the kernel
+// outgrew the instruction cache.  128-thread CTAs of 32 x 4 cells, five on an
+// SM, keep some CTAs in the FP64 phase while others are in the integer phase.
+// Tiles own the interior cells (l0..l0+XT-1, n0..n0+FY-1), l0, n0 >= 1; the
+// near-face states of the next column and row are computed by one warp in a
+// second turn.  The faces whose low cell is a ghost -- x faces (0,n), y faces
+// (l,0) -- are 32-face edge items computed face by face (edge_faces).
+constexpr int XT = 32, XY = 8;  // cells per tile of the batched form; XT is also the width here
+constexpr int FY = 4;           // rows of the single-problem tile
+constexpr int FCTAS = 5;        // CTAs per SM (40 KB of shared memory and 102 registers a thread)
+constexpr int XS = 13;          // doubles per published state set (12 used, padded)
+constexpr int TW = XT + 5;      // tile width with halo
 
 struct XySmem {
-    Cell tile[XY + 5][XT + 5];
-    double left[XY][XT][XS];    // left-face states of cells l0+1 .. l0+XT
-    double bottom[XY][XT][XS];  // bottom-face states of rows n0+1 .. n0+XY
-    double top[XY][XT][XS];     // each cell's own top-face states, parked during its x-face solve
+    Cell tile[FY + 5][TW];       // staged doubles, then their signed mantissas (fix_decode)
+    ushort4 ex[FY + 5][TW];      // biased exponents of the four variables
+    double far[FY][XT][XS];      // each cell's right (top) face states
+    double near[FY][XT][XS];     // the left (bottom) face states of its right (upper) neighbour
 };
 
+// Variable k's states on the two faces of one axis of the cell at tile
+// position `at`; sn, st: strides in cells along and across the axis.
+__device__ __forceinline__ void recon_axis(const XySmem& sm, const FixWeight* w0, const FixWeight* w1, int at, int sn,
+                                           int st, int k, double* lo, double* hi) {
+    const int off[13] = {0, -sn, sn, -2 * sn, 2 * sn, -st, st, -2 * st, 2 * st, -sn - st, sn - st, st - sn, sn + st};
+    const unsigned short* ex = reinterpret_cast<const unsigned short*>(&sm.ex[0][0] + at) + k;
+    const long long* q = reinterpret_cast<const long long*>(&sm.tile[0][0] + at) + k;
+    int e[13], E = 0;
+#pragma unroll
+    for (int i = 0; i < 13; i++) {
+        e[i] = ex[4 * off[i]];
+        E = max(E, e[i]);
+    }
+    long long v[13];
+#pragma unroll
+    for (int i = 0; i < 13; i++) v[i] = fix_shift(q[4 * off[i]], (unsigned)(E - e[i]));
+    FixHalves c[13];
+    fix_components(v, c);
+    long long l[3], h[3];
+    fix_family(w0, w1, c, l, h);
+    const bool ok = fix_exponent_ok(E);
+    const double special = __longlong_as_double(fix_special_bits(E));
+#pragma unroll
+    for (int g = 0; g < 3; g++) {
+        lo[g] = ok ? fix_value(l[g], E) : special;
+        hi[g] = ok ? fix_value(h[g], E) : special;
+    }
+}
+
 // staged: the halo tile is already in sm.tile (TMA); otherwise load it here.
-__device__ __forceinline__ void xy_tile(const GridGeom& g, const GpWeights& w, const double* __restrict__ uin,
-                                        double* __restrict__ fx, double* __restrict__ fy, int l0, int n0,
-                                        XySmem& sm, bool staged) {
+__device__ __forceinline__ void xy_tile(const GridGeom& g, const FixOrbit& o, const double* gw,
+                                        const double* __restrict__ uin, double* __restrict__ fx,
+                                        double* __restrict__ fy, int l0, int n0, XySmem& sm, bool staged) {
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * XT + tx;
     if (!staged)
-        for (int i = tid; i < (XT + 5) * (XY + 5); i += XT * XY) {
-            const int cy = i / (XT + 5), cx = i - cy * (XT + 5);
+        for (int i = tid; i < TW * (FY + 5); i += XT * FY) {
+            const int cy = i / TW, cx = i - cy * TW;
             const int l = l0 - 2 + cx, n = n0 - 2 + cy;
             if (l >= -3 && l <= g.lf + 4 && n >= -3 && n <= g.nf + 4)
                 sm.tile[cy][cx] = ld_cell(uin + 4 * cidx(g, l, n));
         }
     __syncthreads();
+    for (int i = tid; i < TW * (FY + 5); i += XT * FY) {
+        long long* c = reinterpret_cast<long long*>(&sm.tile[0][0] + i);
+        int e[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) c[k] = fix_decode(c[k], &e[k]);
+        (&sm.ex[0][0])[i] = make_ushort4((unsigned short)e[0], (unsigned short)e[1], (unsigned short)e[2],
+                                         (unsigned short)e[3]);
+    }
     const int l = l0 + tx, n = n0 + ty;
-    // a cell up to (lf+1, nf+1) provides states: its stencil stays inside the padded grid
-    const bool live = l <= g.lf + 1 && n <= g.nf + 1;
-    XyOut xs, ys;
-    if (live) {
+#pragma unroll 1
+    for (int axis = 0; axis < 2; axis++) {
+        __syncthreads();  // the tile is decoded; the previous axis is done with the states
+        const int sn = axis == 0 ? 1 : TW, st = axis == 0 ? TW : 1;
+        // turn 0: every cell of the tile; turn 1: the next column (axis 0) or row (axis 1).
+        // A cell up to (lf+1, nf+1) provides states: its stencil stays inside the padded grid.
+        int cx = tx, cy = ty;
+        bool live = l <= g.lf + 1 && n <= g.nf + 1;
+#pragma unroll 1
+        for (int turn = 0; turn < 2; turn++) {
+            if (live) {
+                const int px = cx - (axis == 0), py = cy - (axis != 0);  // the low neighbour's slot
+                const bool give = px >= 0 && py >= 0, keep = turn == 0;
+#pragma unroll 1
+                for (int k = 0; k < 4; k++) {
+                    double lo[3], hi[3];
+                    recon_axis(sm, o.w0[axis], o.w1[axis], (cy + 2) * TW + cx + 2, sn, st, k, lo, hi);
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            Comp c;
-            components(sm.tile, tx + 2, ty + 2, k, c);
-            x_family(w.orb, c, k, xs);
-            y_family(w.orb, c, k, ys);
-        }
-        if (tx > 0) publish(sm.left[ty][tx - 1], xs.lo);
-        if (ty > 0) publish(sm.bottom[ty - 1][tx], ys.lo);
-        publish(sm.top[ty][tx], ys.hi);
-    }
-    // the extra column (left states of cells l0+XT) and row (bottom states of n0+XY)
-    if (ty == XY - 1 && l <= g.lf + 1 && n0 + XY <= g.nf + 1) {
-        XyOut e;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            Comp c;
-            components(sm.tile, tx + 2, XY + 2, k, c);
-            y_family(w.orb, c, k, e);
-        }
-        publish(sm.bottom[XY - 1][tx], e.lo);
-    }
-    if (ty == XY - 2 && tx < XY && l0 + XT <= g.lf + 1 && n0 + tx <= g.nf + 1) {
-        XyOut e;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            Comp c;
-            components(sm.tile, XT + 2, tx + 2, k, c);
-            x_family(w.orb, c, k, e);
-        }
-        publish(sm.left[tx][XT - 1], e.lo);
-    }
-    __syncthreads();
-    if (l <= g.lf && n <= g.nf) {  // x face between (l,n) and (l+1,n)
-        double uR[3][4], F[4];
-        const double* src = sm.left[ty][tx];
-#pragma unroll
-        for (int gp = 0; gp < 3; gp++)
-#pragma unroll
-            for (int k = 0; k < 4; k++) uR[gp][k] = src[4 * gp + k];
-        quad_flux<0, 3>(xs.hi, uR, w.gw, F);
-        st_cell(fx + 4 * cidx(g, l, n), Cell{F[0], F[1], F[2], F[3]});
-    }
-    if (l <= g.lf && n <= g.nf) {  // y face between (l,n) and (l,n+1)
-        double uL[3][4], uR[3][4], F[4];
-        const double* src = sm.bottom[ty][tx];
-        const double* own = sm.top[ty][tx];
-#pragma unroll
-        for (int gp = 0; gp < 3; gp++)
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                uL[gp][k] = own[4 * gp + k];
-                uR[gp][k] = src[4 * gp + k];
+                    for (int gp = 0; gp < 3; gp++) {
+                        if (give) sm.near[py][px][4 * gp + k] = lo[gp];
+                        if (keep) sm.far[cy][cx][4 * gp + k] = hi[gp];
+                    }
+                }
             }
-        quad_flux<1, 3>(uL, uR, w.gw, F);
-        st_cell(fy + 4 * cidx(g, l, n), Cell{F[0], F[1], F[2], F[3]});
+            cx = axis == 0 ? XT : tid;
+            cy = axis == 0 ? tid : FY;
+            live = tid < (axis == 0 ? FY : XT) && l0 + cx <= g.lf + 1 && n0 + cy <= g.nf + 1;
+        }
+        __syncthreads();
+        if (l <= g.lf && n <= g.nf) {  // the face between (l,n) and its upper neighbour on the axis
+            const double* uL = sm.far[ty][tx];
+            const double* uR = sm.near[ty][tx];
+            const int kn = 1 + axis, kt = 2 - axis;  // normal and tangential momentum
+            NormalFlux acc{0., 0., 0., 0.};
+            bool adm = true;
+#pragma unroll
+            for (int gp = 0; gp < 3; gp++) {
+                NormalFlux f;
+                const double *a = uL + 4 * gp, *b = uR + 4 * gp;
+                adm = hllc_normal(a[0], a[kn], a[kt], a[3], b[0], b[kn], b[kt], b[3], f) && adm;
+                if (gp == 0) acc = NormalFlux{f.r * gw[0], f.n * gw[0], f.t * gw[0], f.e * gw[0]};
+                else acc = NormalFlux{acc.r + f.r * gw[gp], acc.n + f.n * gw[gp], acc.t + f.t * gw[gp], acc.e + f.e * gw[gp]};
+            }
+            double F[4] = {acc.r, axis == 0 ? acc.n : acc.t, axis == 0 ? acc.t : acc.n, acc.e};
+            nan_flux(!adm, F);
+            st_cell((axis == 0 ? fx : fy) + 4 * cidx(g, l, n), Cell{F[0], F[1], F[2], F[3]});
+        }
     }
 }
 
 // Edge item: faces k0 .. k0+EDGE_T-1 of the list [x faces (0,1..nf), y faces
 // (1..lf,0)], one warp per item so that the few edge faces spread over many SMs.
 constexpr int EDGE_T = 32;
+template <class M>
 __device__ __forceinline__ void edge_faces(const GridGeom& g, const GpWeights& w, const double* __restrict__ uin,
                                            double* __restrict__ fx, double* __restrict__ fy, int k0) {
     const int k = k0 + (int)threadIdx.x;
     double F[4];
     if (k < g.nf) {
         const size_t c0 = cidx(g, 0, k + 1);
-        face_global<0, 13, 3>(g, w, 2, uin, c0, F);
+        face_global<0, 13, 3, M>(g, w, 2, uin, c0, F);
         st_cell(fx + 4 * c0, Cell{F[0], F[1], F[2], F[3]});
     } else if (k < g.nf + g.lf) {
         const size_t c0 = cidx(g, k - g.nf + 1, 0);
-        face_global<1, 13, 3>(g, w, 2, uin, c0, F);
+        face_global<1, 13, 3, M>(g, w, 2, uin, c0, F);
         st_cell(fy + 4 * c0, Cell{F[0], F[1], F[2], F[3]});
     }
 }
 
 // One cell tile per block (x fastest).
-__global__ void __launch_bounds__(XT * XY, 2) k_flux_xy(StageArgs a, const __grid_constant__ GpWeights w, int tiles_x) {
+__global__ void __launch_bounds__(XT * FY, FCTAS) k_flux_xy(StageArgs a, const __grid_constant__ GpWeights w, int tiles_x) {
     extern __shared__ __align__(16) unsigned char xy_raw[];
     XySmem& sm = *reinterpret_cast<XySmem*>(xy_raw);
     const int by = blockIdx.x / tiles_x, bx = blockIdx.x - by * tiles_x;
-    xy_tile(a.g, w, a.uin, a.fx, a.fy, 1 + bx * XT, 1 + by * XY, sm, false);
+    xy_tile(a.g, w.orb, w.gw, a.uin, a.fx, a.fy, 1 + bx * XT, 1 + by * FY, sm, false);
 }
 
 // ---- the same kernel with the halo tile staged by the Tensor Memory Accelerator
 // The padded state is a 2-D tensor of ny rows by 4*nx doubles; one
-// cp.async.bulk.tensor copies the tile's (XY+5) rows of 4*(XT+5) doubles --
+// cp.async.bulk.tensor copies the tile's (FY+5) rows of 4*(XT+5) doubles --
 // exactly the row-major layout of XySmem::tile -- into this CTA's own shared
 // memory and completes on an mbarrier.  The innermost start coordinate is
 // 4*(l0+1) doubles, a multiple of 32 bytes; boxes that reach past the padded
 // grid on the right or top are zero-filled, and those cells feed no live
 // cell's stencil.
-constexpr unsigned XY_TILE_BYTES = (unsigned)sizeof(Cell) * (XT + 5) * (XY + 5);
+constexpr unsigned XY_TILE_BYTES = (unsigned)sizeof(Cell) * (XT + 5) * (FY + 5);
 static_assert(sizeof(XySmem::tile) == XY_TILE_BYTES, "TMA box = staged tile");
 static_assert(sizeof(XySmem) % 8 == 0, "mbarrier after the tile data");
 
@@ -531,13 +500,13 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, uint32_t pari
     return false;
 }
 
-__global__ void __launch_bounds__(XT * XY, 2) k_flux_xy_tma(StageArgs a, const __grid_constant__ GpWeights w,
+__global__ void __launch_bounds__(XT * FY, FCTAS) k_flux_xy_tma(StageArgs a, const __grid_constant__ GpWeights w,
                                                          const __grid_constant__ CUtensorMap tm, int tiles_x) {
     extern __shared__ __align__(1024) unsigned char xy_raw[];
     XySmem& sm = *reinterpret_cast<XySmem*>(xy_raw);
     unsigned long long* bar = reinterpret_cast<unsigned long long*>(xy_raw + sizeof(XySmem));
     const int by = blockIdx.x / tiles_x, bx = blockIdx.x - by * tiles_x;
-    const int l0 = 1 + bx * XT, n0 = 1 + by * XY;
+    const int l0 = 1 + bx * XT, n0 = 1 + by * FY;
     if (threadIdx.x == 0 && threadIdx.y == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -561,7 +530,7 @@ __global__ void __launch_bounds__(XT * XY, 2) k_flux_xy_tma(StageArgs a, const _
         }
         return;
     }
-    xy_tile(a.g, w, a.uin, a.fx, a.fy, l0, n0, sm, true);
+    xy_tile(a.g, w.orb, w.gw, a.uin, a.fx, a.fy, l0, n0, sm, true);
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no -lcuda).
@@ -579,7 +548,7 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
-// The tile map of a padded state: ny rows of 4*nx doubles, boxes of XY+5 rows
+// The tile map of a padded state: ny rows of 4*nx doubles, boxes of FY+5 rows
 // by 4*(XT+5) doubles.  False if the CUDA driver refuses it or the state is not
 // 16-byte aligned (TMA's rule for the global address).
 static bool encode_tile_map(CUtensorMap* m, const double* u, const GridGeom& g) {
@@ -587,7 +556,7 @@ static bool encode_tile_map(CUtensorMap* m, const double* u, const GridGeom& g) 
     if (!enc || (reinterpret_cast<uintptr_t>(u) & 15)) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)4 * g.nx, (cuuint64_t)g.ny};
     const cuuint64_t strides[1] = {(cuuint64_t)4 * g.nx * sizeof(double)};
-    const cuuint32_t box[2] = {4 * (XT + 5), XY + 5};
+    const cuuint32_t box[2] = {4 * (XT + 5), FY + 5};
     const cuuint32_t estr[2] = {1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<double*>(u), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -596,7 +565,7 @@ static bool encode_tile_map(CUtensorMap* m, const double* u, const GridGeom& g) 
 
 // The faces whose low cell is a ghost, EDGE_T per block.
 __global__ void __launch_bounds__(EDGE_T) k_flux_edge(StageArgs a, const __grid_constant__ GpWeights w) {
-    edge_faces(a.g, w, a.uin, a.fx, a.fy, blockIdx.x * EDGE_T);
+    edge_faces<FaceMath>(a.g, w, a.uin, a.fx, a.fy, blockIdx.x * EDGE_T);
 }
 
 bool launch_flux_xy(const StageArgs& a, const GpWeights& w, cudaStream_t s) {
@@ -608,13 +577,13 @@ bool launch_flux_xy(const StageArgs& a, const GpWeights& w, cudaStream_t s) {
         cudaFuncSetAttribute(k_flux_xy_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, tma_smem);
         attr[dev].store(true, std::memory_order_relaxed);
     }
-    const int tx = (a.g.lf + XT - 1) / XT, ty = (a.g.nf + XY - 1) / XY;
+    const int tx = (a.g.lf + XT - 1) / XT, ty = (a.g.nf + FY - 1) / FY;
     const int edges = (a.g.lf + a.g.nf + EDGE_T - 1) / EDGE_T;
     CUtensorMap tm;
     if (a.g.flux_tma && encode_tile_map(&tm, a.uin, a.g))
-        k_flux_xy_tma<<<tx * ty, dim3(XT, XY), tma_smem, s>>>(a, w, tm, tx);
+        k_flux_xy_tma<<<tx * ty, dim3(XT, FY), tma_smem, s>>>(a, w, tm, tx);
     else
-        k_flux_xy<<<tx * ty, dim3(XT, XY), sizeof(XySmem), s>>>(a, w, tx);
+        k_flux_xy<<<tx * ty, dim3(XT, FY), sizeof(XySmem), s>>>(a, w, tx);
     k_flux_edge<<<edges, EDGE_T, 0, s>>>(a, w);
     return true;
 }
@@ -639,7 +608,7 @@ void launch_flux_ngp(const StageArgs& a, const GpWeights& w, cudaStream_t s) {
 
 int launch_flux_all(const StageArgs& a, const GpWeights& w, cudaStream_t s) {
 #if !GPM_EXACT
-    if (a.uniform_order && a.g.mord == 5 && a.g.ngp == 3 && a.g.num_flux == 100 && launch_flux_xy(a, w, s))
+    if (a.uniform_order && a.g.mord == 5 && a.g.ngp == 3 && a.g.num_flux == 100 && w.orb.ok && launch_flux_xy(a, w, s))
         return 2;
 #endif
     switch (a.g.ngp) {
@@ -745,7 +714,7 @@ constexpr int LIST_CTAS_PER_SM = 4;
 
 // One face of the face list at its current order (min of the two cells),
 // with stencils read straight from global memory.
-template <int DIR, int NP, int NGP>
+template <int DIR, int NP, int NGP, class M>
 __device__ __forceinline__ void face_global(const GridGeom& g, const GpWeights& w, int o, const double* __restrict__ uin,
                                             size_t c0, double* F) {
     constexpr int FL = DIR == 0 ? 2 : 1;
@@ -765,7 +734,7 @@ __device__ __forceinline__ void face_global(const GridGeom& g, const GpWeights& 
         for (int m = 0; m < NP; m++) q[m] = ld_cell(uin + 4 * (c1 + st_ox(m) + row * st_oy(m)));
         recon_face<DIR, NP, NGP>(w, o, FH, q, uR);
     }
-    quad_flux<DIR, NGP>(uL, uR, w.gw, F, g.num_flux);
+    M::template quad<DIR, NGP>(uL, uR, w.gw, F, g.num_flux);
 }
 
 // The MOOD face phase, split by Gauss point.  A pass's face list is short
@@ -826,7 +795,7 @@ __device__ __forceinline__ void face_gp_states(const GridGeom& g, const GpWeight
 // the whole warp after the branches rejoin (an FP64 warp instruction costs
 // its SM partition ~64 cycles however many lanes are active, so a solve in
 // each branch would double the pass's critical path).
-template <int DIR>
+template <int DIR, class M = FaceMath>
 __device__ __forceinline__ void face_gp_any(const StageArgs& a, const GpWeights& w, size_t c0, int gp, FaceGp& f) {
     const GridGeom& g = a.g;
     const size_t c1 = DIR == 0 ? c0 + 1 : c0 + g.nx;
@@ -835,7 +804,7 @@ __device__ __forceinline__ void face_gp_any(const StageArgs& a, const GpWeights&
     if (o >= 5) face_gp_states<DIR, 13>(g, w, 2, a.uin, c0, gp, uL, uR, nullptr);
     else if (o >= 3) face_gp_states<DIR, 5>(g, w, 1, a.uin, c0, gp, uL, uR, a.ccw);
     else face_gp_states<DIR, 1>(g, w, 0, a.uin, c0, gp, uL, uR, a.ccw);
-    riemann<DIR>(g.num_flux, uL, uR, f.F);
+    M::template solve<DIR>(g.num_flux, uL, uR, f.F);
     f.out = (DIR == 0 ? a.fx : a.fy) + 4 * c0;
     f.gw = w.gw;
 }
@@ -1438,6 +1407,26 @@ const KernelTable table = {launch_bc,          launch_flux_all,  launch_update_d
 
 namespace GPM_NS {
 
+#if GPM_EXACT
+using EnsMath = FaceMath;
+namespace ens {
+using GPM_NS::cell_dt;
+}
+#else
+#include "batch_fast.cuh"
+struct EnsMath {
+    template <int DIR, int NGP>
+    static __device__ __forceinline__ void quad(const double (*uL)[4], const double (*uR)[4], const double* gw,
+                                                double* F, int nflux) {
+        ens::quad_flux<DIR, NGP>(uL, uR, gw, F, nflux);
+    }
+    template <int DIR>
+    static __device__ __forceinline__ void solve(int nflux, const double* uL, const double* uR, double* F) {
+        ens::solve<DIR>(nflux, uL, uR, F);
+    }
+};
+#endif
+
 __device__ __forceinline__ GridGeom bgeom(const BatchArgs& a, const BProb& p) {
     GridGeom g;
     g.lf = p.lf; g.nf = p.nf; g.nx = p.nx; g.ny = p.ny;
@@ -1525,7 +1514,7 @@ __device__ __forceinline__ void face_tile_b(const GpWeights& w, int o, const Cel
         for (int m = 0; m < NP; m++) q[m] = tile[(ty + hy + st_oy(m)) * HXB + tx + hx + st_ox(m)];
         recon_face<DIR, NP, NGP>(w, o, FH, q, uR);
     }
-    quad_flux<DIR, NGP>(uL, uR, w.gw, F, nflux);
+    EnsMath::template quad<DIR, NGP>(uL, uR, w.gw, F, nflux);
 }
 
 template <int TXB, int TYB, int NGP, int ORD>
@@ -1560,12 +1549,12 @@ __global__ void __launch_bounds__(TXB* TYB) kb_flux(BatchArgs a) {
 // The two-direction cell tiles of every problem (xy_tile), persistent CTAs.
 __global__ void __launch_bounds__(XT * XY, 2) kb_flux_xy(BatchArgs a) {
     extern __shared__ __align__(16) unsigned char xy_raw[];
-    XySmem& sm = *reinterpret_cast<XySmem*>(xy_raw);
+    ens::XySmem& sm = *reinterpret_cast<ens::XySmem*>(xy_raw);
     for (int item = blockIdx.x; item < a.nftiles; item += gridDim.x) {
         const int4 it = a.ftiles[item];
         const BProb P = a.prob[it.x];
         __syncthreads();  // the previous tile is done with the shared buffers
-        xy_tile(bgeom(a, P), a.wtab[P.wc], a.uin + 4 * P.off, a.fx + 4 * P.off, a.fy + 4 * P.off, it.z, it.w, sm, false);
+        ens::xy_tile(bgeom(a, P), a.wtab[P.wc], a.uin + 4 * P.off, a.fx + 4 * P.off, a.fy + 4 * P.off, it.z, it.w, sm);
     }
 }
 
@@ -1574,7 +1563,7 @@ __global__ void __launch_bounds__(EDGE_T) kb_flux_edge(BatchArgs a) {
     for (int item = blockIdx.x; item < a.netiles; item += gridDim.x) {
         const int4 it = a.etiles[item];
         const BProb P = a.prob[it.x];
-        edge_faces(bgeom(a, P), a.wtab[P.wc], a.uin + 4 * P.off, a.fx + 4 * P.off, a.fy + 4 * P.off, it.z);
+        edge_faces<EnsMath>(bgeom(a, P), a.wtab[P.wc], a.uin + 4 * P.off, a.fx + 4 * P.off, a.fy + 4 * P.off, it.z);
     }
 }
 #endif
@@ -1607,11 +1596,11 @@ static void blaunch_flux_n(const BatchArgs& a, cudaStream_t s) {
         static std::atomic<bool> attr[GPM_MAX_DEVICES];
         const int dev = gpm_device();
         if (!attr[dev].load(std::memory_order_relaxed)) {
-            cudaFuncSetAttribute(kb_flux_xy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(XySmem));
+            cudaFuncSetAttribute(kb_flux_xy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ens::XySmem));
             attr[dev].store(true, std::memory_order_relaxed);
         }
         const int grid = a.nftiles < sm_count() * 2 ? a.nftiles : sm_count() * 2;
-        kb_flux_xy<<<grid, dim3(XT, XY), sizeof(XySmem), s>>>(a);
+        kb_flux_xy<<<grid, dim3(XT, XY), sizeof(ens::XySmem), s>>>(a);
         const int ge = a.netiles < sm_count() * 16 ? a.netiles : sm_count() * 16;
         if (ge > 0) kb_flux_edge<<<ge, EDGE_T, 0, s>>>(a);
         return;
@@ -1695,8 +1684,8 @@ __device__ __forceinline__ void kb_face_gp(const BatchArgs& a, int cur, int nt, 
     sa.order = a.order + P.off;
     const GpWeights& w = a.wtab[P.wc];
     const size_t c = (size_t)e.y;
-    if (dir == 0) face_gp_any<0>(sa, w, side == 0 ? c - 1 : c, gp, f);
-    else face_gp_any<1>(sa, w, side == 0 ? c - sa.g.nx : c, gp, f);
+    if (dir == 0) face_gp_any<0, EnsMath>(sa, w, side == 0 ? c - 1 : c, gp, f);
+    else face_gp_any<1, EnsMath>(sa, w, side == 0 ? c - sa.g.nx : c, gp, f);
 }
 
 __global__ void kb_mood_mark(BatchArgs a, int cur) {  // the listed cells' orders are already lowered
@@ -1901,7 +1890,7 @@ __global__ void __launch_bounds__(256) kb_combine(BatchArgs a, const double* __r
         if (k < P.nx * P.ny) {
             const long long c = P.off + k;
             if (only_cfl) {
-                v = cell_dt(ld_cell(x + 4 * c), P.dx, P.dy);
+                v = ens::cell_dt(ld_cell(x + 4 * c), P.dx, P.dy);
             } else {
                 const Cell p = ld_cell(x + 4 * c);
                 const Cell q = ld_cell_cg(y + 4 * c);
@@ -1911,7 +1900,7 @@ __global__ void __launch_bounds__(256) kb_combine(BatchArgs a, const double* __r
                 o.my = ca * p.my + cb * q.my;
                 o.e = ca * p.e + cb * q.e;
                 st_cell(y + 4 * c, o);
-                if (with_cfl) v = cell_dt(o, P.dx, P.dy);
+                if (with_cfl) v = ens::cell_dt(o, P.dx, P.dy);
             }
         }
         if (with_cfl || only_cfl) bdt_reduce(v, &a.sc[it.x]);

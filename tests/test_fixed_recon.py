@@ -1,0 +1,149 @@
+"""The fixed-point reconstruction of the fast first pass (csrc/fixed_recon.cuh,
+csrc/gp_weights.cpp) on the CPU: its error against binary128 sums of the same
+stencils and weights, beside the error of the FP64 symmetry sums it stands in
+for (GpOrbit), over smooth, rough, discontinuous and sign-changing stencils;
+and its special exponents."""
+from __future__ import annotations
+
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parents[1] / "gp-mood_gb300" / "csrc"
+
+SOURCE = r"""
+#include <math.h>
+#include <stdio.h>
+#include <string.h>
+#include <random>
+#include "fixed_recon.cuh"
+typedef __float128 f128;
+static const int v_to_st[2][13] = {{0, 1, 3, 10, 12, 4, 2, 9, 11, 5, 8, 6, 7}, {0, 4, 2, 9, 11, 1, 3, 10, 12, 5, 6, 8, 7}};
+static void fixed(const GpWeights& w, int axis, const double* q, double lo[3], double hi[3]) {
+    long long m[13], v[13], l[3], h[3];
+    int e[13], E = 0;
+    for (int i = 0; i < 13; i++) {
+        long long b;
+        memcpy(&b, &q[v_to_st[axis][i]], 8);
+        m[i] = fix_decode(b, &e[i]);
+        E = e[i] > E ? e[i] : E;
+    }
+    for (int i = 0; i < 13; i++) v[i] = fix_shift(m[i], E - e[i]);
+    FixHalves c[13];
+    fix_components(v, c);
+    fix_family(w.orb.w0[axis], w.orb.w1[axis], c, l, h);
+    for (int g = 0; g < 3; g++) {
+        double sp;
+        long long b = fix_special_bits(E);
+        memcpy(&sp, &b, 8);
+        lo[g] = fix_exponent_ok(E) ? fix_value(l[g], E) : sp;
+        hi[g] = fix_exponent_ok(E) ? fix_value(h[g], E) : sp;
+    }
+}
+// the FP64 form: components and fused multiply-adds in the order of the cell tile
+static void fp64(const GpWeights& w, int axis, const double* q, double lo[3], double hi[3]) {
+    const int* s = v_to_st[0];
+    auto Q = [&](int i) { return q[s[i]]; };
+    const double s1 = Q(9) + Q(10), s2 = Q(11) + Q(12), d1 = Q(9) - Q(10), d2 = Q(11) - Q(12);
+    const double c[13] = {Q(0), Q(1) + Q(2), Q(3) + Q(4), Q(5) + Q(6), Q(7) + Q(8), s1 + s2, Q(1) - Q(2), Q(3) - Q(4),
+                          d1 + d2, Q(5) - Q(6), Q(7) - Q(8), s1 - s2, d1 - d2};
+    auto dot = [&](const double* z, const double* x, int n) {
+        double r = z[0] * x[0];
+        for (int i = 1; i < n; i++) r = fma(z[i], x[i], r);
+        return r;
+    };
+    const double *z = axis ? w.orbd.y0 : w.orbd.x0, *y = axis ? w.orbd.y1 : w.orbd.x1;
+    const double pp = dot(z, c, 6), mp = dot(z + 6, c + 6, 3), pm = dot(z + 9, c + 9, 3), mm = z[12] * c[12];
+    const double A = pp + pm, B = mp + mm, C = pp - pm, D = mp - mm;
+    const double p1 = dot(y, c, 6), m1 = dot(y + 6, c + (axis ? 9 : 6), 3);
+    lo[0] = A + B;
+    (axis ? lo[2] : hi[0]) = A - B;
+    (axis ? hi[0] : lo[2]) = C + D;
+    hi[2] = C - D;
+    lo[1] = p1 + m1;
+    hi[1] = p1 - m1;
+}
+int main() {
+    std::mt19937_64 r(1);
+    std::uniform_real_distribution<double> U(-1, 1);
+    for (double ell : {1.0, 3.0, 12.0, 50.0})
+        for (double aspect : {1.0, 0.25, 8.0}) {
+            GpWeights w;
+            double ie[3];
+            if (gpm_gp_presim(ell, 1.0, aspect, 64, 64, 5, 3, &w, ie) || !w.orb.ok) return 2;
+            for (int kind = 0; kind < 6; kind++) {
+                double ef = 0, ed = 0, mf = 0, md = 0;
+                for (int it = 0; it < 5000; it++) {
+                    double q[13], mx = 0;
+                    const double b = pow(10, 6 * U(r));
+                    for (int m = 0; m < 13; m++) {
+                        const double u = U(r);
+                        q[m] = kind == 0 ? b * (1 + 0.01 * u) : kind == 1 ? b * (1 + 0.9 * u)
+                             : kind == 2 ? b * (u > 0 ? 1e3 : 1) * (1 + 0.1 * U(r))
+                             : kind == 3 ? b * (u > 0 ? 1e10 : 1) * (1 + 0.1 * U(r)) : kind == 4 ? b * u
+                                         : b * u * pow(10, 8 * U(r));
+                        mx = fmax(mx, fabs(q[m]));
+                    }
+                    for (int axis = 0; axis < 2; axis++) {
+                        double f[2][3], d[2][3];
+                        fixed(w, axis, q, f[0], f[1]);
+                        fp64(w, axis, q, d[0], d[1]);
+                        for (int side = 0; side < 2; side++)
+                            for (int g = 0; g < 3; g++) {
+                                const int face = axis ? (side ? 1 : 3) : (side ? 2 : 0);
+                                f128 ex = 0;
+                                for (int m = 0; m < 13; m++) ex += (f128)w.zt[2][face][g][m] * q[m];
+                                const double a = (double)(f[side][g] - ex) / mx, c = (double)(d[side][g] - ex) / mx;
+                                ef += a * a;
+                                ed += c * c;
+                                mf = fmax(mf, fabs(a));
+                                md = fmax(md, fabs(c));
+                            }
+                    }
+                }
+                printf("%g %g %d %.3e %.3e %.3e %.3e\n", ell, aspect, kind, sqrt(ef), sqrt(ed), mf, md);
+            }
+        }
+    GpWeights w;
+    double ie[3], lo[3], hi[3], q[13];
+    if (gpm_gp_presim(12, 1, 1, 64, 64, 5, 3, &w, ie)) return 2;
+    for (int m = 0; m < 13; m++) q[m] = 0.7;
+    for (int axis = 0; axis < 2; axis++) {
+        for (double bad : {(double)INFINITY, -(double)INFINITY, (double)NAN, 1e308}) {
+            q[8] = bad;
+            fixed(w, axis, q, lo, hi);
+            for (int g = 0; g < 3; g++)
+                if (!isnan(lo[g]) || !isnan(hi[g])) return 4;
+            q[8] = 0.7;
+        }
+    }
+    for (double small : {0.0, -0.0, 1e-300, 5e-324}) {
+        for (int m = 0; m < 13; m++) q[m] = small;
+        fixed(w, 0, q, lo, hi);
+        for (int g = 0; g < 3; g++)
+            if (lo[g] != 0 || hi[g] != 0) return 5;
+    }
+    return 0;
+}
+"""
+
+
+def test_fixed_point_error_is_no_larger_than_fp64(tmp_path):
+    gxx = shutil.which("g++")
+    cuda = Path("/usr/local/cuda/include")
+    if not gxx or not cuda.exists():
+        pytest.skip("needs g++ and the CUDA headers")
+    src, exe = tmp_path / "fixed.cpp", tmp_path / "fixed"
+    src.write_text(SOURCE)
+    subprocess.run([gxx, "-O2", "-std=gnu++17", "-ffp-contract=off", f"-I{CSRC}", f"-I{cuda}", "-x", "c++", str(src),
+                    str(CSRC / "gp_weights.cpp"), "-o", str(exe), "-lm"], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert out.returncode == 0, (out.returncode, out.stdout[-400:])
+    rows = [[float(v) for v in line.split()] for line in out.stdout.splitlines()]
+    assert len(rows) == 4 * 3 * 6
+    for ell, aspect, kind, ef, ed, mf, md in rows:
+        # RMS error no larger; the largest one may be any of 60000 samples: within 1.1
+        assert ef <= ed, (ell, aspect, kind, ef, ed)
+        assert mf <= 1.1 * md, (ell, aspect, kind, mf, md)
