@@ -73,8 +73,15 @@ int main() {
             GpWeights w;
             double ie[3];
             if (gpm_gp_presim(ell, 1.0, aspect, 64, 64, 5, 3, &w, ie) || !w.orb.ok) return 2;
+            double sz = 0;  // largest sum of absolute weights of a state
+            for (int f = 0; f < 4; f++)
+                for (int g = 0; g < 3; g++) {
+                    double s = 0;
+                    for (int m = 0; m < 13; m++) s += fabs(w.zt[2][f][g][m]);
+                    sz = fmax(sz, s);
+                }
             for (int kind = 0; kind < 6; kind++) {
-                double ef = 0, ed = 0, mf = 0, md = 0;
+                double ef = 0, ed = 0, mf = 0;
                 for (int it = 0; it < 5000; it++) {
                     double q[13], mx = 0;
                     const double b = pow(10, 6 * U(r));
@@ -99,11 +106,10 @@ int main() {
                                 ef += a * a;
                                 ed += c * c;
                                 mf = fmax(mf, fabs(a));
-                                md = fmax(md, fabs(c));
                             }
                     }
                 }
-                printf("%g %g %d %.3e %.3e %.3e %.3e\n", ell, aspect, kind, sqrt(ef), sqrt(ed), mf, md);
+                printf("%g %g %d %.3e %.3e %.3e %.3e\n", ell, aspect, kind, sqrt(ef), sqrt(ed), mf, sz);
             }
         }
     GpWeights w;
@@ -143,7 +149,8 @@ def test_fixed_point_error_is_no_larger_than_fp64(tmp_path):
     assert out.returncode == 0, (out.returncode, out.stdout[-400:])
     rows = [[float(v) for v in line.split()] for line in out.stdout.splitlines()]
     assert len(rows) == 4 * 3 * 6
-    for ell, aspect, kind, ef, ed, mf, md in rows:
-        # RMS error no larger; the largest one may be any of 60000 samples: within 1.1
+    for ell, aspect, kind, ef, ed, mf, sz in rows:
         assert ef <= ed, (ell, aspect, kind, ef, ed)
-        assert mf <= 1.1 * md, (ell, aspect, kind, mf, md)
+        # a priori, of the stencil's largest value: symmetrised weights within 2 ulp of each face's own (both forms
+        # have them), one rounding of the result, 13 alignments and dropped products
+        assert mf <= sz * (2.0**-51 + 2.0**-53) + 13 * 2.0**-57, (ell, aspect, kind, mf)
