@@ -1,7 +1,6 @@
 """The fixed-point reconstruction of the fast first pass (csrc/fixed_recon.cuh,
 csrc/gp_weights.cpp) on the CPU: its error against binary128 sums of the same
-stencils and weights, beside the error of the FP64 symmetry sums it stands in
-for (GpOrbit), over smooth, rough, discontinuous and sign-changing stencils;
+stencils and weights, beside the error of the same sums in FP64 (GpOrbit), over smooth, rough, discontinuous and sign-changing stencils;
 and its special exponents."""
 from __future__ import annotations
 
@@ -42,22 +41,23 @@ static void fixed(const GpWeights& w, int axis, const double* q, double lo[3], d
         hi[g] = fix_exponent_ok(E) ? fix_value(h[g], E) : sp;
     }
 }
-// the FP64 form: components and fused multiply-adds in the order of the cell tile
-static void fp64(const GpWeights& w, int axis, const double* q, double lo[3], double hi[3]) {
+// the form in T: the components and sums of the cell tile, with the doubles the fixed-point weights come from
+template <class T, class Fma>
+static void sums(const GpWeights& w, int axis, const double* q, T lo[3], T hi[3], Fma fm) {
     const int* s = v_to_st[0];
-    auto Q = [&](int i) { return q[s[i]]; };
-    const double s1 = Q(9) + Q(10), s2 = Q(11) + Q(12), d1 = Q(9) - Q(10), d2 = Q(11) - Q(12);
-    const double c[13] = {Q(0), Q(1) + Q(2), Q(3) + Q(4), Q(5) + Q(6), Q(7) + Q(8), s1 + s2, Q(1) - Q(2), Q(3) - Q(4),
-                          d1 + d2, Q(5) - Q(6), Q(7) - Q(8), s1 - s2, d1 - d2};
-    auto dot = [&](const double* z, const double* x, int n) {
-        double r = z[0] * x[0];
-        for (int i = 1; i < n; i++) r = fma(z[i], x[i], r);
+    auto Q = [&](int i) { return (T)q[s[i]]; };
+    const T s1 = Q(9) + Q(10), s2 = Q(11) + Q(12), d1 = Q(9) - Q(10), d2 = Q(11) - Q(12);
+    const T c[13] = {Q(0), Q(1) + Q(2), Q(3) + Q(4), Q(5) + Q(6), Q(7) + Q(8), s1 + s2, Q(1) - Q(2), Q(3) - Q(4),
+                     d1 + d2, Q(5) - Q(6), Q(7) - Q(8), s1 - s2, d1 - d2};
+    auto dot = [&](const double* z, const T* x, int n) {
+        T r = (T)z[0] * x[0];
+        for (int i = 1; i < n; i++) r = fm((T)z[i], x[i], r);
         return r;
     };
     const double *z = axis ? w.orbd.y0 : w.orbd.x0, *y = axis ? w.orbd.y1 : w.orbd.x1;
-    const double pp = dot(z, c, 6), mp = dot(z + 6, c + 6, 3), pm = dot(z + 9, c + 9, 3), mm = z[12] * c[12];
-    const double A = pp + pm, B = mp + mm, C = pp - pm, D = mp - mm;
-    const double p1 = dot(y, c, 6), m1 = dot(y + 6, c + (axis ? 9 : 6), 3);
+    const T pp = dot(z, c, 6), mp = dot(z + 6, c + 6, 3), pm = dot(z + 9, c + 9, 3), mm = (T)z[12] * c[12];
+    const T A = pp + pm, B = mp + mm, C = pp - pm, D = mp - mm;
+    const T p1 = dot(y, c, 6), m1 = dot(y + 6, c + (axis ? 9 : 6), 3);
     lo[0] = A + B;
     (axis ? lo[2] : hi[0]) = A - B;
     (axis ? hi[0] : lo[2]) = C + D;
@@ -96,12 +96,12 @@ int main() {
                     for (int axis = 0; axis < 2; axis++) {
                         double f[2][3], d[2][3];
                         fixed(w, axis, q, f[0], f[1]);
-                        fp64(w, axis, q, d[0], d[1]);
+                        sums(w, axis, q, d[0], d[1], [](double a, double b, double c) { return fma(a, b, c); });
+                        f128 x[2][3];
+                        sums(w, axis, q, x[0], x[1], [](f128 a, f128 b, f128 c) { return a * b + c; });
                         for (int side = 0; side < 2; side++)
                             for (int g = 0; g < 3; g++) {
-                                const int face = axis ? (side ? 1 : 3) : (side ? 2 : 0);
-                                f128 ex = 0;
-                                for (int m = 0; m < 13; m++) ex += (f128)w.zt[2][face][g][m] * q[m];
+                                const f128 ex = x[side][g];
                                 const double a = (double)(f[side][g] - ex) / mx, c = (double)(d[side][g] - ex) / mx;
                                 ef += a * a;
                                 ed += c * c;
@@ -151,6 +151,6 @@ def test_fixed_point_error_is_no_larger_than_fp64(tmp_path):
     assert len(rows) == 4 * 3 * 6
     for ell, aspect, kind, ef, ed, mf, sz in rows:
         assert ef <= ed, (ell, aspect, kind, ef, ed)
-        # a priori, of the stencil's largest value: symmetrised weights within 2 ulp of each face's own (both forms
-        # have them), one rounding of the result, 13 alignments and dropped products
-        assert mf <= sz * (2.0**-51 + 2.0**-53) + 13 * 2.0**-57, (ell, aspect, kind, mf)
+        # a priori, of the stencil's largest value: one rounding of the result; 13 alignments, each weighted; 26
+        # roundings of weights and dropped products of a unit (2^-58)
+        assert mf <= sz * (2.0**-53 + 2.0**-57) + 26 * 2.0**-58, (ell, aspect, kind, mf)
