@@ -215,6 +215,8 @@ __device__ __forceinline__ double cell_dt(const Cell& u, double dx, double dy) {
 // components of its 13-point stencil (GpOrbit; 80 FP64 operations per variable
 // against 128 face by face), left and bottom states handed to the neighbours
 // through shared memory.
+constexpr int XS = 13;  // doubles per published state set (12 used, padded)
+
 struct XyOut {
     double lo[3][4];  // left (x) or bottom (y) face states
     double hi[3][4];  // right (x) or top (y) face states

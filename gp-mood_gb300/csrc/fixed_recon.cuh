@@ -1,14 +1,15 @@
 // fixed_recon.cuh -- the fast first pass's GP reconstruction in fixed point.
 //
-// A cell's 12 face states (left/right/bottom/top faces at 3 Gauss points) are
-// constant-weight sums over its 13-point stencil.  On this part an SM issues
+// A cell's face states (left/right/bottom/top faces at 2 or 3 Gauss points) are
+// constant-weight sums over its 13-point (order 5) or 5-point (order 3) stencil.  On this part an SM issues
 // an FP64 instruction every 16-19 cycles but two integer instructions per
 // cycle beside it (measured: eight 32x32+64-bit multiply-adds next to every
 // FP64 FMA cost nothing), and the first pass is bound by the FP64 pipe, so the
-// sums run on the integer pipe and FP64 is left to the Riemann solves.
+// sums run on the integer pipe and FP64 is left to the Riemann solves.  Radius 1
+// (order 3, 5 points) uses the same form.
 //
 // Per variable and stencil the values share one exponent E, the largest biased
-// exponent of the 13: a double M * 2^(e-1075) becomes Q = M << 5 >> (E - e), a
+// exponent of its cells: a double M * 2^(e-1075) becomes Q = M << 5 >> (E - e), a
 // 58-bit integer with 5 guard bits below the largest value's last place.  The
 // mirror-symmetry components (GpOrbit) are exact integer sums of up to four Q
 // (60 bits).  A weight is w * 2^58 rounded to an integer.  Both factors are
@@ -59,8 +60,9 @@ GPM_HD long long fix_shift(long long v, unsigned n) {
 GPM_HD long long fix_wide(int a, int b) { return (long long)a * b; }
 
 // Mirror-symmetry components (the order of FixOrbit) of the aligned stencil
-// values v at (n, t) = (0,0), (-1,0), (1,0), (-2,0), (2,0), (0,-1), (0,1),
-// (0,-2), (0,2), (-1,-1), (1,-1), (-1,1), (1,1); each split into signed halves.
+// values v, each split into signed halves.  Order 5: v at (n, t) = (0,0),
+// (-1,0), (1,0), (0,-1), (0,1), (-2,0), (2,0), (0,-2), (0,2), (-1,-1), (1,-1),
+// (-1,1), (1,1); order 3: the first five.
 struct FixHalves {
     int h, l;
 };
@@ -70,18 +72,27 @@ GPM_HD FixHalves fix_split(long long q) {
     s.l = (int)((unsigned)q - ((unsigned)s.h << 30));
     return s;
 }
+template <int ORD>
 GPM_HD void fix_components(const long long* v, FixHalves* c) {
+    if (ORD == 3) {
+        c[0] = fix_split(v[0]);
+        c[1] = fix_split(v[1] + v[2]);
+        c[2] = fix_split(v[3] + v[4]);
+        c[3] = fix_split(v[1] - v[2]);
+        c[4] = fix_split(v[3] - v[4]);
+        return;
+    }
     const long long s1 = v[9] + v[10], s2 = v[11] + v[12], d1 = v[9] - v[10], d2 = v[11] - v[12];
     c[0] = fix_split(v[0]);
     c[1] = fix_split(v[1] + v[2]);
-    c[2] = fix_split(v[3] + v[4]);
-    c[3] = fix_split(v[5] + v[6]);
+    c[2] = fix_split(v[5] + v[6]);
+    c[3] = fix_split(v[3] + v[4]);
     c[4] = fix_split(v[7] + v[8]);
     c[5] = fix_split(s1 + s2);
     c[6] = fix_split(v[1] - v[2]);
-    c[7] = fix_split(v[3] - v[4]);
+    c[7] = fix_split(v[5] - v[6]);
     c[8] = fix_split(d1 + d2);
-    c[9] = fix_split(v[5] - v[6]);
+    c[9] = fix_split(v[3] - v[4]);
     c[10] = fix_split(v[7] - v[8]);
     c[11] = fix_split(s1 - s2);
     c[12] = fix_split(d1 - d2);
@@ -102,19 +113,23 @@ GPM_HD long long fix_dot(const FixWeight* w, const FixHalves* c) {
     return (long long)((unsigned long long)hh << 2) + (hl >> 28);
 }
 
-// The six states of an axis's two faces (lo: left or bottom, hi: right or top)
-// at Gauss points 0, 1, 2 from the components in that axis's frame.
+// The states of an axis's two faces (lo: left or bottom, hi: right or top) at
+// its NGP Gauss points from the components in that axis's frame.
+template <int ORD, int NGP>
 GPM_HD void fix_family(const FixWeight* w0, const FixWeight* w1, const FixHalves* c, long long* lo, long long* hi) {
-    const long long pp = fix_dot<6>(w0, c), mp = fix_dot<3>(w0 + 6, c + 6), pm = fix_dot<3>(w0 + 9, c + 9),
-                    mm = fix_dot<1>(w0 + 12, c + 12);
+    constexpr int P = ORD == 5 ? 6 : 3, M = ORD == 5 ? 3 : 1;  // sizes of the first group, of the next two
+    const long long pp = fix_dot<P>(w0, c), mp = fix_dot<M>(w0 + P, c + P), pm = fix_dot<M>(w0 + P + M, c + P + M);
+    const long long mm = ORD == 5 ? fix_dot<1>(w0 + 12, c + 12) : 0;
     const long long A = pp + pm, B = mp + mm, C = pp - pm, D = mp - mm;
     lo[0] = A + B;
     hi[0] = A - B;
-    lo[2] = C + D;
-    hi[2] = C - D;
-    const long long p1 = fix_dot<6>(w1, c), m1 = fix_dot<3>(w1 + 6, c + 6);
-    lo[1] = p1 + m1;
-    hi[1] = p1 - m1;
+    lo[NGP - 1] = C + D;
+    hi[NGP - 1] = C - D;
+    if (NGP == 3) {
+        const long long p1 = fix_dot<P>(w1, c), m1 = fix_dot<M>(w1 + P, c + P);
+        lo[1] = p1 + m1;
+        hi[1] = p1 - m1;
+    }
 }
 
 // Whether exponent E has normal results (see the head of the file).

@@ -150,6 +150,65 @@ extern "C" void gpm_pol_weights(GpWeights* w) {
         }
 }
 
+// The fixed-point orbit weights (FixOrbit) of orders 3 and 5 for 2 or 3 Gauss
+// points.  The far faces and the last Gauss point are taken from the near
+// face's first point by mirroring, so the weights must have that symmetry.
+extern "C" void gpm_fix_orbits(GpWeights* w, int ngp) {
+    memset(w->orb, 0, sizeof w->orb);
+    if (ngp != 2 && ngp != 3) return;
+    static const int mx[13] = {0, 3, 2, 1, 4, 8, 7, 6, 5, 9, 12, 11, 10};   // stencil index under x -> -x
+    static const int my[13] = {0, 1, 4, 3, 2, 6, 5, 8, 7, 11, 10, 9, 12};   // y -> -y
+    static const int tr[13] = {0, 4, 3, 2, 1, 5, 8, 7, 6, 10, 9, 12, 11};   // x <-> y
+    for (int o = 1; o <= 2; o++) {
+        FixOrbit& orb = w->orb[o - 1];
+        const int np = o == 1 ? 5 : 13;
+        bool ok = true;
+        for (int axis = 0; axis < 2; axis++) {
+            const int near = axis == 0 ? 0 : 3, far = axis == 0 ? 2 : 1;
+            const int *mn = axis == 0 ? mx : my, *mt = axis == 0 ? my : mx;
+            for (int g = 0; g < ngp; g++)
+                for (int m = 0; m < np; m++) {
+                    const double z = w->zt[o][near][g][m];
+                    ok = ok && fabs(w->zt[o][far][g][mn[m]] - z) <= 1e-14 &&
+                         fabs(w->zt[o][near][ngp - 1 - g][mt[m]] - z) <= 1e-14;
+                }
+            for (int mid = 0; mid < (ngp == 3 ? 2 : 1); mid++) {
+                double z[13] = {0.0}, c[13];
+                for (int m = 0; m < np; m++) z[axis == 0 ? m : tr[m]] = w->zt[o][near][mid][m];  // (n, t) frame
+                // 0 (0,0), 1 (-1,0), 2 (0,1), 3 (1,0), 4 (0,-1), 5 (-1,-1), 6 (-1,1), 7 (1,1), 8 (1,-1), 9 (0,-2),
+                // 10 (-2,0), 11 (0,2), 12 (2,0)
+                c[0] = z[0];
+                c[1] = 0.5 * (z[1] + z[3]);
+                c[2] = 0.5 * (z[10] + z[12]);
+                c[3] = 0.5 * (z[4] + z[2]);
+                c[4] = 0.5 * (z[9] + z[11]);
+                c[5] = 0.25 * (z[5] + z[8] + z[6] + z[7]);
+                c[6] = 0.5 * (z[1] - z[3]);
+                c[7] = 0.5 * (z[10] - z[12]);
+                c[8] = 0.25 * (z[5] - z[8] + z[6] - z[7]);
+                c[9] = 0.5 * (z[4] - z[2]);
+                c[10] = 0.5 * (z[9] - z[11]);
+                c[11] = 0.25 * (z[5] + z[8] - z[6] - z[7]);
+                c[12] = 0.25 * (z[5] - z[8] - z[6] + z[7]);
+                static const int nc[13] = {1, 2, 2, 2, 2, 4, 2, 2, 4, 2, 2, 4, 4};  // cells in each component
+                static const int all[13] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12}, five[5] = {0, 1, 3, 6, 9};
+                const int n = o == 2 ? (mid ? 9 : 13) : (mid ? 4 : 5);
+                FixWeight* fw = mid ? orb.w1[axis] : orb.w0[axis];
+                double sum = 0.0;
+                for (int i = 0; i < n; i++) {
+                    const int k = o == 2 ? all[i] : five[i];
+                    sum += fabs(c[k]) * nc[k];
+                    const long long v = llrint(ldexp(c[k], 58));
+                    fw[i].h = (int)((v + (1LL << 29)) >> 30);
+                    fw[i].l = (int)(v - ((long long)fw[i].h << 30));
+                }
+                ok = ok && sum <= 4.0;
+            }
+        }
+        orb.ok = ok;
+    }
+}
+
 extern "C" int gpm_gp_presim(double ell_o_dx, double lx, double ly, int lf, int nf, int mord, int ngp,
                              GpWeights* out, double inv_err[3]) {
     if (!(mord == 1 || mord == 3 || mord == 5) || ngp < 1 || ngp > GPM_MAXGP || lf < 1 || nf < 1)
@@ -279,30 +338,7 @@ extern "C" int gpm_gp_presim(double ell_o_dx, double lx, double ly, int lf, int 
         split(out->zt[2][3][1], c);
         for (int k = 0; k < 6; k++) d.y1[k] = c[k];  // x-symmetric: groups 2, 4 vanish
         for (int k = 0; k < 3; k++) d.y1[6 + k] = c[9 + k];
-        // w * 2^58, split in two signed halves; nc: stencil cells in each component
-        static const int nc[13] = {1, 2, 2, 2, 2, 4, 2, 2, 4, 2, 2, 4, 4};
-        static const int id[13] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12};
-        static const int swap[13] = {0, 3, 4, 1, 2, 5, 9, 10, 11, 6, 7, 8, 12};  // y faces: n is y, t is x
-        static const int swap9[9] = {0, 3, 4, 1, 2, 5, 6, 7, 8};
-        FixOrbit& orb = out->orb;
-        orb.ok = 1;
-        auto store = [&](const double* w, const int* order, int n, FixWeight* fw) {
-            double sum = 0.0;
-            for (int i = 0; i < n; i++) sum += fabs(w[order[i]]) * nc[i];
-            if (!(sum <= 4.0)) {
-                orb.ok = 0;
-                return;
-            }
-            for (int i = 0; i < n; i++) {
-                const long long v = llrint(ldexp(w[order[i]], 58));
-                fw[i].h = (int)((v + (1LL << 29)) >> 30);
-                fw[i].l = (int)(v - ((long long)fw[i].h << 30));
-            }
-        };
-        store(d.x0, id, 13, orb.w0[0]);
-        store(d.x1, id, 9, orb.w1[0]);
-        store(d.y0, swap, 13, orb.w0[1]);
-        store(d.y1, swap9, 9, orb.w1[1]);
     }
+    gpm_fix_orbits(out, ngp);
     return 0;
 }

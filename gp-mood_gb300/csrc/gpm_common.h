@@ -62,17 +62,19 @@ __host__ __device__ constexpr int gpm_sym_pair(int dir, int k, int side) {
 struct GpOrbit {
     double x0[13], x1[9], y0[13], y1[9];
 };
-// The same weights in 58-bit fixed point, split for 32-bit multiplies:
-// w = (h * 2^30 + l) * 2^-58, |l| <= 2^29 (fixed_recon.cuh).  [axis 0: x faces,
-// 1: y faces]; components in the axis's own frame (n: along it, t: across it):
-// [Q0 Q1p Q2p Q3p Q4p Q5pp | Q1m Q2m Q5mp | Q3m Q4m Q5pm | Q5mm] with Q1, Q2 the
-// pairs along n and Q3, Q4 along t.
+// Orbit weights in 58-bit fixed point, split for 32-bit multiplies:
+// w = (h * 2^30 + l) * 2^-58, |l| <= 2^29 (fixed_recon.cuh), for order 3 and 5
+// and 2 or 3 Gauss points.  [axis 0: x faces, 1: y faces]; components in the
+// axis's own frame (n: along it, t: across it), order 5: [Q0 Q1p Q2p Q3p Q4p
+// Q5pp | Q1m Q2m Q5mp | Q3m Q4m Q5pm | Q5mm] with Q1, Q2 the pairs along n and
+// Q3, Q4 along t; order 3: [Q0 Q1p Q3p | Q1m | Q3m].  w0 is the first Gauss
+// point's, w1 (3 points) the middle one's, whose last two groups vanish.
 struct FixWeight {
     int h, l;
 };
 struct FixOrbit {
     FixWeight w0[2][13], w1[2][9];
-    int ok;  // the weights are in the fixed-point form's range; 0: the fast first pass runs per face instead
+    int ok;  // mirror symmetric and in the fixed-point form's range; 0: the first pass runs face by face instead
     int pad;
 };
 
@@ -88,8 +90,8 @@ struct GpWeights {
     double gw[GPM_MAXGP];            // gauss_weight(ngp, :)
     double d2x[5], d2y[5];           // GP_d2x_sp(3,:), GP_d2y_sp(3,:)
     GpSym sym[3][4];                 // ngp = 3 split of zt (fast mode); zero otherwise
-    FixOrbit orb;                    // ngp = 3 order-5 cell-wise split (fast mode); zero otherwise
-    GpOrbit orbd;                    // ... in doubles (batched form)
+    FixOrbit orb[2];                 // orders 3 and 5, ngp 2 or 3: cell-wise split (fast mode; gpm_fix_orbits)
+    GpOrbit orbd;                    // ngp = 3, order 5, in doubles (batched form)
 };
 
 struct GridGeom {
@@ -193,6 +195,9 @@ void gpm_set_thread_error(const char* msg);
 
 // real(L_16/n, PR): the cell size rounded once from binary128 (global_variables.f90:86-88).
 double gpm_cell_size(double length, int n);
+
+// Fill w->orb from w->zt (ngp Gauss points), after zt is final.
+extern "C" void gpm_fix_orbits(GpWeights* w, int ngp);
 
 // Host GP precompute (gp_weights.cpp).  Returns 0 or -1 on bad knobs.
 extern "C" int gpm_gp_presim(double ell_o_dx, double lx, double ly, int lf, int nf, int mord, int ngp,

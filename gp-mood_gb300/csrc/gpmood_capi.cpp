@@ -518,7 +518,10 @@ int gpmood_create(const gpmood_params* p, gpmood_ctx** out) {
         delete c;
         return fail(nullptr, GPMOOD_E_ARG, "GP precompute rejected the knobs");
     }
-    if (pol) gpm_pol_weights(&c->w);
+    if (pol) {
+        gpm_pol_weights(&c->w);
+        gpm_fix_orbits(&c->w, p->ngp);
+    }
     int ndev = 0;
     cudaError_t e = cudaGetDeviceCount(&ndev);
     if (e != cudaSuccess || ndev < 1) {

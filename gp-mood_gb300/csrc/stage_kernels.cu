@@ -313,80 +313,85 @@ __device__ __forceinline__ void face_global(const GridGeom& g, const GpWeights& 
 
 #if !GPM_EXACT
 // ---------------------------------------------------------------------------
-// Fast first pass at uniform order 5 with ngp = 3: both face directions of a
-// tile of cells in one CTA.  A cell's six states on an axis's two faces come
-// from the mirror-symmetry components of its 13-point stencil (FixOrbit) in
-// fixed point, on the integer pipe (fixed_recon.cuh), so the FP64 pipe, which
-// bounds this kernel, runs only the Riemann solves: 192 FP64 instructions per
-// face instead of 350 with FP64 sums.  After staging, a CTA turns its tile
-// into signed mantissas (in place) and 16-bit exponents once.  Then, for x and
-// for y: every cell's states go to shared memory, its far-face (right, top)
-// states in its own slot and its near-face (left, bottom) states in the slot
-// of the neighbour that shares the face, and every thread solves the face of
-// which its cell is the low side.  Both axes and all four variables run the
-// same code (an axis's frame is a pair of strides): unrolled, the kernel
-// outgrew the instruction cache.  128-thread CTAs of 32 x 4 cells, five on an
-// SM, keep some CTAs in the FP64 phase while others are in the integer phase.
-// Tiles own the interior cells (l0..l0+XT-1, n0..n0+FY-1), l0, n0 >= 1; the
-// near-face states of the next column and row are computed by one warp in a
-// second turn.  The faces whose low cell is a ghost -- x faces (0,n), y faces
-// (l,0) -- are 32-face edge items computed face by face (edge_faces).
+// Fast first pass at a uniform order 3 or 5 with 2 or 3 Gauss points: both
+// face directions of a tile of cells in one CTA.  A cell's states on an axis's
+// two faces come from the mirror-symmetry components of its stencil (FixOrbit)
+// in fixed point, on the integer pipe (fixed_recon.cuh), so the FP64 pipe,
+// which bounds this kernel, runs only the Riemann solves: at order 5 with 3
+// points 192 FP64 instructions per face instead of 350 with FP64 sums.  After
+// staging, a CTA turns its tile into signed mantissas (in place) and 16-bit
+// exponents once.  Then, for x and for y: every cell's states go to shared
+// memory, its far-face (right, top) states in its own slot and its near-face
+// (left, bottom) states in the slot of the neighbour that shares the face, and
+// every thread solves the face of which its cell is the low side.  Both axes
+// and all four variables run the same code (an axis's frame is a pair of
+// strides): unrolled, the kernel outgrew the instruction cache.  Tiles own the
+// interior cells (l0..l0+XT-1, n0..n0+R-1), l0, n0 >= 1; the near-face states of
+// the next column and row are computed by one warp in a second turn, and a
+// tile on the domain's low edge runs a short second part of an axis for the
+// faces whose low cell is a ghost (x faces (0,n), y faces (l,0)).
+//
+// R = 4 rows, 128 threads, five CTAs an SM keep some CTAs in the FP64 phase
+// while others are in the integer phase (2048^2 Sedov step at order 5: 11.3 ms;
+// four CTAs 12.6, 32 x 8 tiles two to an SM 13.5).
 constexpr int XT = 32, XY = 8;  // cells per tile of the batched form; XT is also the width here
-constexpr int FY = 4;           // rows of the single-problem tile
-constexpr int FCTAS = 5;        // CTAs per SM (40 KB of shared memory and 102 registers a thread)
-constexpr int XS = 13;          // doubles per published state set (12 used, padded)
-constexpr int TW = XT + 5;      // tile width with halo
+constexpr int TW = XT + 6;      // tile width with halo: 3 cells below, 3 above
 
+template <int NGP, int R>
 struct XySmem {
-    Cell tile[FY + 5][TW];       // staged doubles, then their signed mantissas (fix_decode)
-    ushort4 ex[FY + 5][TW];      // biased exponents of the four variables
-    double far[FY][XT][XS];      // each cell's right (top) face states
-    double near[FY][XT][XS];     // the left (bottom) face states of its right (upper) neighbour
+    static constexpr int XS = 4 * NGP + 1;  // doubles per state set, padded to an odd stride
+    Cell tile[R + 6][TW];                   // staged doubles, then their signed mantissas (fix_decode)
+    ushort4 ex[R + 6][TW];                  // biased exponents of the four variables
+    double far[R][XT][XS];                  // each cell's right (top) face states
+    double near[R][XT][XS];                 // the left (bottom) face states of its right (upper) neighbour
 };
 
 // Variable k's states on the two faces of one axis of the cell at tile
 // position `at`; sn, st: strides in cells along and across the axis.
-__device__ __forceinline__ void recon_axis(const XySmem& sm, const FixWeight* w0, const FixWeight* w1, int at, int sn,
-                                           int st, int k, double* lo, double* hi) {
-    const int off[13] = {0, -sn, sn, -2 * sn, 2 * sn, -st, st, -2 * st, 2 * st, -sn - st, sn - st, st - sn, sn + st};
+template <int ORD, int NGP, class S>
+__device__ __forceinline__ void recon_axis(const S& sm, const FixWeight* w0, const FixWeight* w1, int at, int sn, int st,
+                                           int k, double* lo, double* hi) {
+    constexpr int NP = np_of(ORD);
+    const int off[13] = {0, -sn, sn, -st, st, -2 * sn, 2 * sn, -2 * st, 2 * st, -sn - st, sn - st, st - sn, sn + st};
     const unsigned short* ex = reinterpret_cast<const unsigned short*>(&sm.ex[0][0] + at) + k;
     const long long* q = reinterpret_cast<const long long*>(&sm.tile[0][0] + at) + k;
-    int e[13], E = 0;
+    int e[NP], E = 0;
 #pragma unroll
-    for (int i = 0; i < 13; i++) {
+    for (int i = 0; i < NP; i++) {
         e[i] = ex[4 * off[i]];
         E = max(E, e[i]);
     }
-    long long v[13];
+    long long v[NP];
 #pragma unroll
-    for (int i = 0; i < 13; i++) v[i] = fix_shift(q[4 * off[i]], (unsigned)(E - e[i]));
-    FixHalves c[13];
-    fix_components(v, c);
-    long long l[3], h[3];
-    fix_family(w0, w1, c, l, h);
+    for (int i = 0; i < NP; i++) v[i] = fix_shift(q[4 * off[i]], (unsigned)(E - e[i]));
+    FixHalves c[NP];
+    fix_components<ORD>(v, c);
+    long long l[NGP], h[NGP];
+    fix_family<ORD, NGP>(w0, w1, c, l, h);
     const bool ok = fix_exponent_ok(E);
     const double special = __longlong_as_double(fix_special_bits(E));
 #pragma unroll
-    for (int g = 0; g < 3; g++) {
+    for (int g = 0; g < NGP; g++) {
         lo[g] = ok ? fix_value(l[g], E) : special;
         hi[g] = ok ? fix_value(h[g], E) : special;
     }
 }
 
 // staged: the halo tile is already in sm.tile (TMA); otherwise load it here.
+template <int ORD, int NGP, int R>
 __device__ __forceinline__ void xy_tile(const GridGeom& g, const FixOrbit& o, const double* gw,
                                         const double* __restrict__ uin, double* __restrict__ fx,
-                                        double* __restrict__ fy, int l0, int n0, XySmem& sm, bool staged) {
+                                        double* __restrict__ fy, int l0, int n0, XySmem<NGP, R>& sm, bool staged) {
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * XT + tx;
     if (!staged)
-        for (int i = tid; i < TW * (FY + 5); i += XT * FY) {
+        for (int i = tid; i < TW * (R + 6); i += XT * R) {
             const int cy = i / TW, cx = i - cy * TW;
-            const int l = l0 - 2 + cx, n = n0 - 2 + cy;
+            const int l = l0 - 3 + cx, n = n0 - 3 + cy;
             if (l >= -3 && l <= g.lf + 4 && n >= -3 && n <= g.nf + 4)
                 sm.tile[cy][cx] = ld_cell(uin + 4 * cidx(g, l, n));
         }
     __syncthreads();
-    for (int i = tid; i < TW * (FY + 5); i += XT * FY) {
+    for (int i = tid; i < TW * (R + 6); i += XT * R) {
         long long* c = reinterpret_cast<long long*>(&sm.tile[0][0] + i);
         int e[4];
 #pragma unroll
@@ -394,44 +399,55 @@ __device__ __forceinline__ void xy_tile(const GridGeom& g, const FixOrbit& o, co
         (&sm.ex[0][0])[i] = make_ushort4((unsigned short)e[0], (unsigned short)e[1], (unsigned short)e[2],
                                          (unsigned short)e[3]);
     }
-    const int l = l0 + tx, n = n0 + ty;
 #pragma unroll 1
-    for (int axis = 0; axis < 2; axis++) {
-        __syncthreads();  // the tile is decoded; the previous axis is done with the states
+    for (int ap = 0; ap < 4; ap++) {
+        const int axis = ap >> 1, edge = ap & 1;  // edge: the faces below the tile's first column or row
+        if (edge && (axis == 0 ? l0 : n0) != 1) continue;
+        __syncthreads();  // the tile is decoded; the states are free
         const int sn = axis == 0 ? 1 : TW, st = axis == 0 ? TW : 1;
-        // turn 0: every cell of the tile; turn 1: the next column (axis 0) or row (axis 1).
+        const int across = axis == 0 ? R : XT;  // cells of a tile's column (x) or row (y)
+        // Turn 0: every cell of the tile; turn 1: the next column or row.  On the edge: the ghost column or row
+        // (warp 0, far states) and the first one (warp 1, near states), face j in the slot of the tile's j-th cell.
         // A cell up to (lf+1, nf+1) provides states: its stencil stays inside the padded grid.
         int cx = tx, cy = ty;
-        bool live = l <= g.lf + 1 && n <= g.nf + 1;
+        if (edge) {
+            const int c = (tid >> 5) - 1;  // -1: ghost, 0: first
+            cx = axis == 0 ? c : tx;
+            cy = axis == 0 ? tx : c;
+        }
 #pragma unroll 1
-        for (int turn = 0; turn < 2; turn++) {
-            if (live) {
-                const int px = cx - (axis == 0), py = cy - (axis != 0);  // the low neighbour's slot
-                const bool give = px >= 0 && py >= 0, keep = turn == 0;
+        for (int turn = 0; turn < 2 - edge; turn++) {
+            const bool mine = edge ? tid < 64 && tx < across : turn == 0 || tid < across;
+            if (mine && l0 + cx <= g.lf + 1 && n0 + cy <= g.nf + 1) {
+                const int px = edge ? (axis == 0 ? 0 : tx) : cx - (axis == 0);  // slot of the near states
+                const int py = edge ? (axis == 0 ? tx : 0) : cy - (axis != 0);
+                const bool give = edge ? tid >= 32 : px >= 0 && py >= 0, keep = edge ? tid < 32 : turn == 0;
+                const int fx_ = edge ? px : cx, fy_ = edge ? py : cy;           // slot of the far states
 #pragma unroll 1
                 for (int k = 0; k < 4; k++) {
-                    double lo[3], hi[3];
-                    recon_axis(sm, o.w0[axis], o.w1[axis], (cy + 2) * TW + cx + 2, sn, st, k, lo, hi);
+                    double lo[NGP], hi[NGP];
+                    recon_axis<ORD, NGP>(sm, o.w0[axis], o.w1[axis], (cy + 3) * TW + cx + 3, sn, st, k, lo, hi);
 #pragma unroll
-                    for (int gp = 0; gp < 3; gp++) {
+                    for (int gp = 0; gp < NGP; gp++) {
                         if (give) sm.near[py][px][4 * gp + k] = lo[gp];
-                        if (keep) sm.far[cy][cx][4 * gp + k] = hi[gp];
+                        if (keep) sm.far[fy_][fx_][4 * gp + k] = hi[gp];
                     }
                 }
             }
             cx = axis == 0 ? XT : tid;
-            cy = axis == 0 ? tid : FY;
-            live = tid < (axis == 0 ? FY : XT) && l0 + cx <= g.lf + 1 && n0 + cy <= g.nf + 1;
+            cy = axis == 0 ? tid : R;
         }
         __syncthreads();
-        if (l <= g.lf && n <= g.nf) {  // the face between (l,n) and its upper neighbour on the axis
-            const double* uL = sm.far[ty][tx];
-            const double* uR = sm.near[ty][tx];
+        // the face of low cell (l, n): the thread's own cell, or the ghost before the j-th cell of the edge
+        const int sx = edge ? (axis == 0 ? 0 : tx) : tx, sy = edge ? (axis == 0 ? tx : 0) : ty;
+        const int l = l0 + sx - (edge && axis == 0), n = n0 + sy - (edge && axis != 0);
+        if ((!edge || tid < across) && l <= g.lf && n <= g.nf) {
+            const double *uL = sm.far[sy][sx], *uR = sm.near[sy][sx];
             const int kn = 1 + axis, kt = 2 - axis;  // normal and tangential momentum
             NormalFlux acc{0., 0., 0., 0.};
             bool adm = true;
 #pragma unroll
-            for (int gp = 0; gp < 3; gp++) {
+            for (int gp = 0; gp < NGP; gp++) {
                 NormalFlux f;
                 const double *a = uL + 4 * gp, *b = uR + 4 * gp;
                 adm = hllc_normal(a[0], a[kn], a[kt], a[3], b[0], b[kn], b[kt], b[3], f) && adm;
@@ -464,26 +480,27 @@ __device__ __forceinline__ void edge_faces(const GridGeom& g, const GpWeights& w
     }
 }
 
+// CTAs an SM should hold: 20 warps at 102 registers a thread.
+constexpr int xy_ctas(int R) { return 20 / R; }
+
 // One cell tile per block (x fastest).
-__global__ void __launch_bounds__(XT * FY, FCTAS) k_flux_xy(StageArgs a, const __grid_constant__ GpWeights w, int tiles_x) {
+template <int ORD, int NGP, int R>
+__global__ void __launch_bounds__(XT * R, xy_ctas(R)) k_flux_xy(StageArgs a, const __grid_constant__ GpWeights w,
+                                                                int tiles_x) {
     extern __shared__ __align__(16) unsigned char xy_raw[];
-    XySmem& sm = *reinterpret_cast<XySmem*>(xy_raw);
+    XySmem<NGP, R>& sm = *reinterpret_cast<XySmem<NGP, R>*>(xy_raw);
     const int by = blockIdx.x / tiles_x, bx = blockIdx.x - by * tiles_x;
-    xy_tile(a.g, w.orb, w.gw, a.uin, a.fx, a.fy, 1 + bx * XT, 1 + by * FY, sm, false);
+    xy_tile<ORD, NGP, R>(a.g, w.orb[ORD / 2 - 1], w.gw, a.uin, a.fx, a.fy, 1 + bx * XT, 1 + by * R, sm, false);
 }
 
 // ---- the same kernel with the halo tile staged by the Tensor Memory Accelerator
 // The padded state is a 2-D tensor of ny rows by 4*nx doubles; one
-// cp.async.bulk.tensor copies the tile's (FY+5) rows of 4*(XT+5) doubles --
+// cp.async.bulk.tensor copies the tile's (R+6) rows of 4*(XT+6) doubles --
 // exactly the row-major layout of XySmem::tile -- into this CTA's own shared
 // memory and completes on an mbarrier.  The innermost start coordinate is
-// 4*(l0+1) doubles, a multiple of 32 bytes; boxes that reach past the padded
+// 4*l0 doubles, a multiple of 32 bytes; boxes that reach past the padded
 // grid on the right or top are zero-filled, and those cells feed no live
 // cell's stencil.
-constexpr unsigned XY_TILE_BYTES = (unsigned)sizeof(Cell) * (XT + 5) * (FY + 5);
-static_assert(sizeof(XySmem::tile) == XY_TILE_BYTES, "TMA box = staged tile");
-static_assert(sizeof(XySmem) % 8 == 0, "mbarrier after the tile data");
-
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // Bounded wait for phase `parity` of an mbarrier (~1 s at most).
@@ -500,25 +517,29 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, uint32_t pari
     return false;
 }
 
-__global__ void __launch_bounds__(XT * FY, FCTAS) k_flux_xy_tma(StageArgs a, const __grid_constant__ GpWeights w,
-                                                         const __grid_constant__ CUtensorMap tm, int tiles_x) {
+template <int ORD, int NGP, int R>
+__global__ void __launch_bounds__(XT * R, xy_ctas(R)) k_flux_xy_tma(StageArgs a, const __grid_constant__ GpWeights w,
+                                                                    const __grid_constant__ CUtensorMap tm,
+                                                                    int tiles_x) {
     extern __shared__ __align__(1024) unsigned char xy_raw[];
-    XySmem& sm = *reinterpret_cast<XySmem*>(xy_raw);
-    unsigned long long* bar = reinterpret_cast<unsigned long long*>(xy_raw + sizeof(XySmem));
+    using Smem = XySmem<NGP, R>;
+    static_assert(sizeof(Smem) % 8 == 0, "mbarrier after the tile data");
+    Smem& sm = *reinterpret_cast<Smem*>(xy_raw);
+    unsigned long long* bar = reinterpret_cast<unsigned long long*>(xy_raw + sizeof(Smem));
     const int by = blockIdx.x / tiles_x, bx = blockIdx.x - by * tiles_x;
-    const int l0 = 1 + bx * XT, n0 = 1 + by * FY;
+    const int l0 = 1 + bx * XT, n0 = 1 + by * R;
     if (threadIdx.x == 0 && threadIdx.y == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
-                     "r"(XY_TILE_BYTES)
+                     "r"((unsigned)sizeof(Smem::tile))
                      : "memory");
-        // padded cell (l0-2, n0-2) is column l0+1, row n0+1 of the padded grid
+        // padded cell (l0-3, n0-3) is column l0, row n0 of the padded grid
         asm volatile(
             "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
             "[%4];" ::"r"(smem_addr(&sm.tile[0][0])),
-            "l"(reinterpret_cast<uint64_t>(&tm)), "r"(4 * (l0 + 1)), "r"(n0 + 1), "r"(smem_addr(bar))
+            "l"(reinterpret_cast<uint64_t>(&tm)), "r"(4 * l0), "r"(n0), "r"(smem_addr(bar))
             : "memory");
     }
     __syncthreads();  // the barrier is initialised before anyone waits on it
@@ -530,7 +551,7 @@ __global__ void __launch_bounds__(XT * FY, FCTAS) k_flux_xy_tma(StageArgs a, con
         }
         return;
     }
-    xy_tile(a.g, w.orb, w.gw, a.uin, a.fx, a.fy, l0, n0, sm, true);
+    xy_tile<ORD, NGP, R>(a.g, w.orb[ORD / 2 - 1], w.gw, a.uin, a.fx, a.fy, l0, n0, sm, true);
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no -lcuda).
@@ -548,44 +569,42 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
-// The tile map of a padded state: ny rows of 4*nx doubles, boxes of FY+5 rows
-// by 4*(XT+5) doubles.  False if the CUDA driver refuses it or the state is not
+// The tile map of a padded state: ny rows of 4*nx doubles, boxes of R+6 rows
+// by 4*(XT+6) doubles.  False if the CUDA driver refuses it or the state is not
 // 16-byte aligned (TMA's rule for the global address).
-static bool encode_tile_map(CUtensorMap* m, const double* u, const GridGeom& g) {
+static bool encode_tile_map(CUtensorMap* m, const double* u, const GridGeom& g, int R) {
     PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
     if (!enc || (reinterpret_cast<uintptr_t>(u) & 15)) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)4 * g.nx, (cuuint64_t)g.ny};
     const cuuint64_t strides[1] = {(cuuint64_t)4 * g.nx * sizeof(double)};
-    const cuuint32_t box[2] = {4 * (XT + 5), FY + 5};
+    const cuuint32_t box[2] = {4 * TW, (cuuint32_t)R + 6};
     const cuuint32_t estr[2] = {1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<double*>(u), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// The faces whose low cell is a ghost, EDGE_T per block.
-__global__ void __launch_bounds__(EDGE_T) k_flux_edge(StageArgs a, const __grid_constant__ GpWeights w) {
-    edge_faces<FaceMath>(a.g, w, a.uin, a.fx, a.fy, blockIdx.x * EDGE_T);
-}
-
-bool launch_flux_xy(const StageArgs& a, const GpWeights& w, cudaStream_t s) {
+template <int ORD, int NGP, int R>
+static void launch_flux_xy_t(const StageArgs& a, const GpWeights& w, cudaStream_t s) {
     static std::atomic<bool> attr[GPM_MAX_DEVICES];
     const int dev = gpm_device();
-    constexpr int tma_smem = (int)sizeof(XySmem) + 8;  // + the mbarrier
+    constexpr int smem = (int)sizeof(XySmem<NGP, R>), tma_smem = smem + 8;  // + the mbarrier
     if (!attr[dev].load(std::memory_order_relaxed)) {
-        cudaFuncSetAttribute(k_flux_xy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(XySmem));
-        cudaFuncSetAttribute(k_flux_xy_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, tma_smem);
+        cudaFuncSetAttribute(k_flux_xy<ORD, NGP, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaFuncSetAttribute(k_flux_xy_tma<ORD, NGP, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, tma_smem);
         attr[dev].store(true, std::memory_order_relaxed);
     }
-    const int tx = (a.g.lf + XT - 1) / XT, ty = (a.g.nf + FY - 1) / FY;
-    const int edges = (a.g.lf + a.g.nf + EDGE_T - 1) / EDGE_T;
+    const int tx = (a.g.lf + XT - 1) / XT, ty = (a.g.nf + R - 1) / R;
     CUtensorMap tm;
-    if (a.g.flux_tma && encode_tile_map(&tm, a.uin, a.g))
-        k_flux_xy_tma<<<tx * ty, dim3(XT, FY), tma_smem, s>>>(a, w, tm, tx);
+    if (a.g.flux_tma && encode_tile_map(&tm, a.uin, a.g, R))
+        k_flux_xy_tma<ORD, NGP, R><<<tx * ty, dim3(XT, R), tma_smem, s>>>(a, w, tm, tx);
     else
-        k_flux_xy<<<tx * ty, dim3(XT, FY), sizeof(XySmem), s>>>(a, w, tx);
-    k_flux_edge<<<edges, EDGE_T, 0, s>>>(a, w);
-    return true;
+        k_flux_xy<ORD, NGP, R><<<tx * ty, dim3(XT, R), smem, s>>>(a, w, tx);
+}
+
+template <int ORD, int NGP>
+static void launch_flux_xy(const StageArgs& a, const GpWeights& w, cudaStream_t s) {
+    launch_flux_xy_t<ORD, NGP, 4>(a, w, s);
 }
 #endif
 
@@ -608,8 +627,14 @@ void launch_flux_ngp(const StageArgs& a, const GpWeights& w, cudaStream_t s) {
 
 int launch_flux_all(const StageArgs& a, const GpWeights& w, cudaStream_t s) {
 #if !GPM_EXACT
-    if (a.uniform_order && a.g.mord == 5 && a.g.ngp == 3 && a.g.num_flux == 100 && w.orb.ok && launch_flux_xy(a, w, s))
-        return 2;
+    if (a.uniform_order && a.g.num_flux == 100 && a.g.mord >= 3 && (a.g.ngp == 2 || a.g.ngp == 3) &&
+        w.orb[a.g.mord / 2 - 1].ok) {
+        if (a.g.mord == 5 && a.g.ngp == 3) launch_flux_xy<5, 3>(a, w, s);
+        else if (a.g.mord == 5) launch_flux_xy<5, 2>(a, w, s);
+        else if (a.g.ngp == 3) launch_flux_xy<3, 3>(a, w, s);
+        else launch_flux_xy<3, 2>(a, w, s);
+        return 1;
+    }
 #endif
     switch (a.g.ngp) {
     case 1: launch_flux_ngp<1>(a, w, s); break;

@@ -1,6 +1,6 @@
 """The fixed-point reconstruction of the fast first pass (csrc/fixed_recon.cuh,
 csrc/gp_weights.cpp) on the CPU: its error against binary128 sums of the same
-stencils and weights, beside the error of the same sums in FP64 (GpOrbit), over smooth, rough, discontinuous and sign-changing stencils;
+stencils and weights, beside the error of the same sums in FP64, for orders 3 and 5, over smooth, rough, discontinuous and sign-changing stencils;
 and its special exponents."""
 from __future__ import annotations
 
@@ -19,20 +19,24 @@ SOURCE = r"""
 #include <random>
 #include "fixed_recon.cuh"
 typedef __float128 f128;
-static const int v_to_st[2][13] = {{0, 1, 3, 10, 12, 4, 2, 9, 11, 5, 8, 6, 7}, {0, 4, 2, 9, 11, 1, 3, 10, 12, 5, 6, 8, 7}};
+// stencil index of v's entries in the axis's (n, t) frame
+static const int v_to_st[2][13] = {{0, 1, 3, 4, 2, 10, 12, 9, 11, 5, 8, 6, 7}, {0, 4, 2, 1, 3, 9, 11, 10, 12, 5, 6, 8, 7}};
+template <int ORD>
 static void fixed(const GpWeights& w, int axis, const double* q, double lo[3], double hi[3]) {
+    constexpr int NP = ORD == 5 ? 13 : 5;
     long long m[13], v[13], l[3], h[3];
     int e[13], E = 0;
-    for (int i = 0; i < 13; i++) {
+    for (int i = 0; i < NP; i++) {
         long long b;
         memcpy(&b, &q[v_to_st[axis][i]], 8);
         m[i] = fix_decode(b, &e[i]);
         E = e[i] > E ? e[i] : E;
     }
-    for (int i = 0; i < 13; i++) v[i] = fix_shift(m[i], E - e[i]);
+    for (int i = 0; i < NP; i++) v[i] = fix_shift(m[i], E - e[i]);
     FixHalves c[13];
-    fix_components(v, c);
-    fix_family(w.orb.w0[axis], w.orb.w1[axis], c, l, h);
+    const FixOrbit& o = w.orb[ORD / 2 - 1];
+    fix_components<ORD>(v, c);
+    fix_family<ORD, 3>(o.w0[axis], o.w1[axis], c, l, h);
     for (int g = 0; g < 3; g++) {
         double sp;
         long long b = fix_special_bits(E);
@@ -41,26 +45,39 @@ static void fixed(const GpWeights& w, int axis, const double* q, double lo[3], d
         hi[g] = fix_exponent_ok(E) ? fix_value(h[g], E) : sp;
     }
 }
-// the form in T: the components and sums of the cell tile, with the doubles the fixed-point weights come from
+// the same sums in T with the symmetrised double weights
 template <class T, class Fma>
-static void sums(const GpWeights& w, int axis, const double* q, T lo[3], T hi[3], Fma fm) {
-    const int* s = v_to_st[0];
-    auto Q = [&](int i) { return (T)q[s[i]]; };
+static void sums(const GpWeights& w, int o, int axis, const double* q, T lo[3], T hi[3], Fma fm) {
+    const int* s = v_to_st[axis];
+    const int np = o == 2 ? 13 : 5;
+    auto Q = [&](int i) { return i < np ? (T)q[s[i]] : (T)0; };
     const T s1 = Q(9) + Q(10), s2 = Q(11) + Q(12), d1 = Q(9) - Q(10), d2 = Q(11) - Q(12);
-    const T c[13] = {Q(0), Q(1) + Q(2), Q(3) + Q(4), Q(5) + Q(6), Q(7) + Q(8), s1 + s2, Q(1) - Q(2), Q(3) - Q(4),
-                     d1 + d2, Q(5) - Q(6), Q(7) - Q(8), s1 - s2, d1 - d2};
-    auto dot = [&](const double* z, const T* x, int n) {
-        T r = (T)z[0] * x[0];
-        for (int i = 1; i < n; i++) r = fm((T)z[i], x[i], r);
+    const T c[13] = {Q(0), Q(1) + Q(2), Q(5) + Q(6), Q(3) + Q(4), Q(7) + Q(8), s1 + s2, Q(1) - Q(2), Q(5) - Q(6),
+                     d1 + d2, Q(3) - Q(4), Q(7) - Q(8), s1 - s2, d1 - d2};
+    auto weights = [&](int g, double* c13) {
+        const double* zt = w.zt[o][axis ? 3 : 0][g];
+        double z[13];
+        for (int i = 0; i < 13; i++) z[i] = i < np ? zt[s[i]] : 0.0;
+        const double k[13] = {z[0], 0.5 * (z[1] + z[2]), 0.5 * (z[5] + z[6]), 0.5 * (z[3] + z[4]), 0.5 * (z[7] + z[8]),
+                              0.25 * (z[9] + z[10] + z[11] + z[12]), 0.5 * (z[1] - z[2]), 0.5 * (z[5] - z[6]),
+                              0.25 * (z[9] - z[10] + z[11] - z[12]), 0.5 * (z[3] - z[4]), 0.5 * (z[7] - z[8]),
+                              0.25 * (z[9] + z[10] - z[11] - z[12]), 0.25 * (z[9] - z[10] - z[11] + z[12])};
+        memcpy(c13, k, sizeof k);
+    };
+    double z[13], y[13];
+    weights(0, z);
+    weights(1, y);
+    auto dot = [&](const double* a, const T* x, int n) {
+        T r = (T)a[0] * x[0];
+        for (int i = 1; i < n; i++) r = fm((T)a[i], x[i], r);
         return r;
     };
-    const double *z = axis ? w.orbd.y0 : w.orbd.x0, *y = axis ? w.orbd.y1 : w.orbd.x1;
     const T pp = dot(z, c, 6), mp = dot(z + 6, c + 6, 3), pm = dot(z + 9, c + 9, 3), mm = (T)z[12] * c[12];
     const T A = pp + pm, B = mp + mm, C = pp - pm, D = mp - mm;
-    const T p1 = dot(y, c, 6), m1 = dot(y + 6, c + (axis ? 9 : 6), 3);
+    const T p1 = dot(y, c, 6), m1 = dot(y + 6, c + 6, 3);
     lo[0] = A + B;
-    (axis ? lo[2] : hi[0]) = A - B;
-    (axis ? hi[0] : lo[2]) = C + D;
+    hi[0] = A - B;
+    lo[2] = C + D;
     hi[2] = C - D;
     lo[1] = p1 + m1;
     hi[1] = p1 - m1;
@@ -72,17 +89,19 @@ int main() {
         for (double aspect : {1.0, 0.25, 8.0}) {
             GpWeights w;
             double ie[3];
-            if (gpm_gp_presim(ell, 1.0, aspect, 64, 64, 5, 3, &w, ie) || !w.orb.ok) return 2;
+            if (gpm_gp_presim(ell, 1.0, aspect, 64, 64, 5, 3, &w, ie) || !w.orb[0].ok || !w.orb[1].ok) return 2;
+            for (int o = 1; o <= 2; o++) {
             double sz = 0;  // largest sum of absolute weights of a state
             for (int f = 0; f < 4; f++)
                 for (int g = 0; g < 3; g++) {
                     double s = 0;
-                    for (int m = 0; m < 13; m++) s += fabs(w.zt[2][f][g][m]);
+                    for (int m = 0; m < 13; m++) s += fabs(w.zt[o][f][g][m]);
                     sz = fmax(sz, s);
                 }
+            const int np = o == 2 ? 13 : 5;
             for (int kind = 0; kind < 6; kind++) {
                 double ef = 0, ed = 0, mf = 0;
-                for (int it = 0; it < 5000; it++) {
+                for (int it = 0; it < 3000; it++) {
                     double q[13], mx = 0;
                     const double b = pow(10, 6 * U(r));
                     for (int m = 0; m < 13; m++) {
@@ -91,14 +110,14 @@ int main() {
                              : kind == 2 ? b * (u > 0 ? 1e3 : 1) * (1 + 0.1 * U(r))
                              : kind == 3 ? b * (u > 0 ? 1e10 : 1) * (1 + 0.1 * U(r)) : kind == 4 ? b * u
                                          : b * u * pow(10, 8 * U(r));
-                        mx = fmax(mx, fabs(q[m]));
+                        if (m < np) mx = fmax(mx, fabs(q[m]));
                     }
                     for (int axis = 0; axis < 2; axis++) {
                         double f[2][3], d[2][3];
-                        fixed(w, axis, q, f[0], f[1]);
-                        sums(w, axis, q, d[0], d[1], [](double a, double b, double c) { return fma(a, b, c); });
+                        o == 2 ? fixed<5>(w, axis, q, f[0], f[1]) : fixed<3>(w, axis, q, f[0], f[1]);
+                        sums(w, o, axis, q, d[0], d[1], [](double a, double b, double c) { return fma(a, b, c); });
                         f128 x[2][3];
-                        sums(w, axis, q, x[0], x[1], [](f128 a, f128 b, f128 c) { return a * b + c; });
+                        sums(w, o, axis, q, x[0], x[1], [](f128 a, f128 b, f128 c) { return a * b + c; });
                         for (int side = 0; side < 2; side++)
                             for (int g = 0; g < 3; g++) {
                                 const f128 ex = x[side][g];
@@ -111,6 +130,7 @@ int main() {
                 }
                 printf("%g %g %d %.3e %.3e %.3e %.3e\n", ell, aspect, kind, sqrt(ef), sqrt(ed), mf, sz);
             }
+            }
         }
     GpWeights w;
     double ie[3], lo[3], hi[3], q[13];
@@ -119,7 +139,7 @@ int main() {
     for (int axis = 0; axis < 2; axis++) {
         for (double bad : {(double)INFINITY, -(double)INFINITY, (double)NAN, 1e308}) {
             q[8] = bad;
-            fixed(w, axis, q, lo, hi);
+            fixed<5>(w, axis, q, lo, hi);
             for (int g = 0; g < 3; g++)
                 if (!isnan(lo[g]) || !isnan(hi[g])) return 4;
             q[8] = 0.7;
@@ -127,7 +147,7 @@ int main() {
     }
     for (double small : {0.0, -0.0, 1e-300, 5e-324}) {
         for (int m = 0; m < 13; m++) q[m] = small;
-        fixed(w, 0, q, lo, hi);
+        fixed<5>(w, 0, q, lo, hi);
         for (int g = 0; g < 3; g++)
             if (lo[g] != 0 || hi[g] != 0) return 5;
     }
@@ -148,7 +168,7 @@ def test_fixed_point_error_is_no_larger_than_fp64(tmp_path):
     out = subprocess.run([str(exe)], capture_output=True, text=True)
     assert out.returncode == 0, (out.returncode, out.stdout[-400:])
     rows = [[float(v) for v in line.split()] for line in out.stdout.splitlines()]
-    assert len(rows) == 4 * 3 * 6
+    assert len(rows) == 4 * 3 * 2 * 6
     for ell, aspect, kind, ef, ed, mf, sz in rows:
         assert ef <= ed, (ell, aspect, kind, ef, ed)
         # a priori, of the stencil's largest value: one rounding of the result; 13 alignments, each weighted; 26

@@ -20,8 +20,9 @@ def _state(lf, nf, decades):
     return np.ascontiguousarray(np.stack([r, r * u, r * v, p / 0.4 + 0.5 * r * (u * u + v * v)], axis=-1))
 
 
-def _step(pkg, U, fp):
-    with pkg.Solver(lf=U.shape[1] - 8, nf=U.shape[0] - 8, bc_type=17, method=pkg.GP_SE, fp_mode=fp) as s:
+def _step(pkg, U, fp, mord=5, ngp=3):
+    with pkg.Solver(lf=U.shape[1] - 8, nf=U.shape[0] - 8, bc_type=17, method=pkg.GP_SE, fp_mode=fp, mord=mord,
+                    ngp=ngp) as s:
         V, out = U.copy(), np.empty_like(U)
         s.Boundary_C(V)
         s.time_stepping(V, out, 0.0, 1e-4)
@@ -30,9 +31,10 @@ def _step(pkg, U, fp):
 
 @pytest.mark.parametrize("lf,nf", [(4, 4), (31, 5), (32, 4), (33, 9), (64, 7), (65, 33), (5, 70)])
 @pytest.mark.parametrize("decades", [0.0, 0.15])
-def test_tile_edges_equal_exact(pkg, lf, nf, decades):
+@pytest.mark.parametrize("mord,ngp", [(5, 3), (5, 2), (3, 3), (3, 2)])
+def test_tile_edges_equal_exact(pkg, lf, nf, decades, mord, ngp):
     U = _state(lf, nf, decades)
-    a, b = _step(pkg, U, pkg.FP_EXACT), _step(pkg, U, pkg.FP_FAST)
+    a, b = _step(pkg, U, pkg.FP_EXACT, mord, ngp), _step(pkg, U, pkg.FP_FAST, mord, ngp)
     # ~40 rounded operations on values of the cell's own density or energy (x10 for its neighbours'): 1e-13 of them
     assert np.isfinite(a).all()
     size = np.maximum(a[..., :1], a[..., 3:])
