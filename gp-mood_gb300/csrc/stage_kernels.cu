@@ -327,9 +327,11 @@ __device__ __forceinline__ void face_global(const GridGeom& g, const GpWeights& 
 // and all four variables run the same code (an axis's frame is a pair of
 // strides): unrolled, the kernel outgrew the instruction cache.  Tiles own the
 // interior cells (l0..l0+XT-1, n0..n0+R-1), l0, n0 >= 1; the near-face states of
-// the next column and row are computed by one warp in a second turn, and a
-// tile on the domain's low edge runs a short second part of an axis for the
-// faces whose low cell is a ghost (x faces (0,n), y faces (l,0)).
+// the next column and row are computed by one warp in a second turn.  The
+// faces whose low cell is a ghost (x faces (0,n), y faces (l,0)) have blocks of
+// their own at the front of the grid, which stage the same tiles and solve only
+// those faces (done by the low-edge tiles themselves, or by a launch of their
+// own, they were 20 us of dependent FP64 at the end of a 256^2 first pass).
 //
 // R = 4 rows, 128 threads, five CTAs an SM keep some CTAs in the FP64 phase
 // while others are in the integer phase (2048^2 Sedov step at order 5: 11.3 ms;
@@ -378,10 +380,12 @@ __device__ __forceinline__ void recon_axis(const S& sm, const FixWeight* w0, con
 }
 
 // staged: the halo tile is already in sm.tile (TMA); otherwise load it here.
+// edge_axis: -1, or the axis whose low-edge faces this block solves.
 template <int ORD, int NGP, int R>
 __device__ __forceinline__ void xy_tile(const GridGeom& g, const FixOrbit& o, const double* gw,
                                         const double* __restrict__ uin, double* __restrict__ fx,
-                                        double* __restrict__ fy, int l0, int n0, XySmem<NGP, R>& sm, bool staged) {
+                                        double* __restrict__ fy, int l0, int n0, int edge_axis, XySmem<NGP, R>& sm,
+                                        bool staged) {
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * XT + tx;
     if (!staged)
         for (int i = tid; i < TW * (R + 6); i += XT * R) {
@@ -400,9 +404,9 @@ __device__ __forceinline__ void xy_tile(const GridGeom& g, const FixOrbit& o, co
                                          (unsigned short)e[3]);
     }
 #pragma unroll 1
-    for (int ap = 0; ap < 4; ap++) {
-        const int axis = ap >> 1, edge = ap & 1;  // edge: the faces below the tile's first column or row
-        if (edge && (axis == 0 ? l0 : n0) != 1) continue;
+    for (int axis = 0; axis < 2; axis++) {
+        const int edge = edge_axis >= 0;  // an edge block: the faces below the tile's first column or row
+        if (edge && axis != edge_axis) continue;
         __syncthreads();  // the tile is decoded; the states are free
         const int sn = axis == 0 ? 1 : TW, st = axis == 0 ? TW : 1;
         const int across = axis == 0 ? R : XT;  // cells of a tile's column (x) or row (y)
@@ -483,14 +487,26 @@ __device__ __forceinline__ void edge_faces(const GridGeom& g, const GpWeights& w
 // CTAs an SM should hold: 20 warps at 102 registers a thread.
 constexpr int xy_ctas(int R) { return 20 / R; }
 
-// One cell tile per block (x fastest).
+// The tile of a block: the edge blocks come first (one per row of tiles for
+// the x faces, one per column for the y faces), then one per tile, x fastest.
+template <int R>
+__device__ __forceinline__ void xy_block(int tiles_x, int tiles_y, int* l0, int* n0, int* edge) {
+    const int b = (int)blockIdx.x, t = b - (tiles_x + tiles_y);
+    const int by = t >= 0 ? t / tiles_x : b < tiles_y ? b : 0;
+    const int bx = t >= 0 ? t - by * tiles_x : b < tiles_y ? 0 : b - tiles_y;
+    *edge = t >= 0 ? -1 : b < tiles_y ? 0 : 1;
+    *l0 = 1 + bx * XT;
+    *n0 = 1 + by * R;
+}
+
 template <int ORD, int NGP, int R>
 __global__ void __launch_bounds__(XT * R, xy_ctas(R)) k_flux_xy(StageArgs a, const __grid_constant__ GpWeights w,
-                                                                int tiles_x) {
+                                                                int tiles_x, int tiles_y) {
     extern __shared__ __align__(16) unsigned char xy_raw[];
     XySmem<NGP, R>& sm = *reinterpret_cast<XySmem<NGP, R>*>(xy_raw);
-    const int by = blockIdx.x / tiles_x, bx = blockIdx.x - by * tiles_x;
-    xy_tile<ORD, NGP, R>(a.g, w.orb[ORD / 2 - 1], w.gw, a.uin, a.fx, a.fy, 1 + bx * XT, 1 + by * R, sm, false);
+    int l0, n0, edge;
+    xy_block<R>(tiles_x, tiles_y, &l0, &n0, &edge);
+    xy_tile<ORD, NGP, R>(a.g, w.orb[ORD / 2 - 1], w.gw, a.uin, a.fx, a.fy, l0, n0, edge, sm, false);
 }
 
 // ---- the same kernel with the halo tile staged by the Tensor Memory Accelerator
@@ -520,14 +536,14 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, uint32_t pari
 template <int ORD, int NGP, int R>
 __global__ void __launch_bounds__(XT * R, xy_ctas(R)) k_flux_xy_tma(StageArgs a, const __grid_constant__ GpWeights w,
                                                                     const __grid_constant__ CUtensorMap tm,
-                                                                    int tiles_x) {
+                                                                    int tiles_x, int tiles_y) {
     extern __shared__ __align__(1024) unsigned char xy_raw[];
     using Smem = XySmem<NGP, R>;
     static_assert(sizeof(Smem) % 8 == 0, "mbarrier after the tile data");
     Smem& sm = *reinterpret_cast<Smem*>(xy_raw);
     unsigned long long* bar = reinterpret_cast<unsigned long long*>(xy_raw + sizeof(Smem));
-    const int by = blockIdx.x / tiles_x, bx = blockIdx.x - by * tiles_x;
-    const int l0 = 1 + bx * XT, n0 = 1 + by * R;
+    int l0, n0, edge;
+    xy_block<R>(tiles_x, tiles_y, &l0, &n0, &edge);
     if (threadIdx.x == 0 && threadIdx.y == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -551,7 +567,7 @@ __global__ void __launch_bounds__(XT * R, xy_ctas(R)) k_flux_xy_tma(StageArgs a,
         }
         return;
     }
-    xy_tile<ORD, NGP, R>(a.g, w.orb[ORD / 2 - 1], w.gw, a.uin, a.fx, a.fy, l0, n0, sm, true);
+    xy_tile<ORD, NGP, R>(a.g, w.orb[ORD / 2 - 1], w.gw, a.uin, a.fx, a.fy, l0, n0, edge, sm, true);
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no -lcuda).
@@ -597,9 +613,9 @@ static void launch_flux_xy_t(const StageArgs& a, const GpWeights& w, cudaStream_
     const int tx = (a.g.lf + XT - 1) / XT, ty = (a.g.nf + R - 1) / R;
     CUtensorMap tm;
     if (a.g.flux_tma && encode_tile_map(&tm, a.uin, a.g, R))
-        k_flux_xy_tma<ORD, NGP, R><<<tx * ty, dim3(XT, R), tma_smem, s>>>(a, w, tm, tx);
+        k_flux_xy_tma<ORD, NGP, R><<<tx * ty + tx + ty, dim3(XT, R), tma_smem, s>>>(a, w, tm, tx, ty);
     else
-        k_flux_xy<ORD, NGP, R><<<tx * ty, dim3(XT, R), smem, s>>>(a, w, tx);
+        k_flux_xy<ORD, NGP, R><<<tx * ty + tx + ty, dim3(XT, R), smem, s>>>(a, w, tx, ty);
 }
 
 template <int ORD, int NGP>
