@@ -124,14 +124,15 @@ int gpm_solo_split_default();
 // Scalars that stay on the device across a step.
 struct DevScalars {
     double t, dt, qx, qy;             // time, step, dt/dx, dt/dy
-    double tmax, cfl;
-    unsigned long long dtmin_bits;    // Setdt reduction slot (bits of a positive double)
-    int ntrb[2];                      // troubled-cell counts, double-buffered lists
-    int status;                       // GPMOOD status bits
-    int passes_stage[GPM_MAXST];      // MOOD passes of each RK stage of the last step (device loop)
-    unsigned stamp_epoch;             // first unused pass stamp of the device MOOD loop
     unsigned long long detected_step; // count_detected_cell of the current step
     unsigned long long apriori_step;
+    int status;                       // GPMOOD status bits
+    int pad;                          // the fields so far are a step's own: one upload sets them (set_time)
+    double tmax, cfl;
+    unsigned long long dtmin_bits;    // Setdt reduction slot (bits of a positive double)
+    int ntrb[2];                      // troubled-cell counts, double-buffered lists; the MOOD loop leaves them 0
+    int passes_stage[GPM_MAXST];      // MOOD passes of each RK stage of the last step (device loop)
+    unsigned stamp_epoch;             // first unused pass stamp of the device MOOD loop
     double bcd[4][4];                 // Dirichlet BC (19): the right ghost columns' states, from the host
 };
 
@@ -173,9 +174,13 @@ struct KernelTable {
     void (*mood_faces)(const StageArgs& a, const GpWeights& w, int cur, int max_trb, cudaStream_t s);
     void (*combine)(const GridGeom& g, const double* x, double* y, double a, double b, int with_cfl,
                     DevScalars* sc, cudaStream_t s);
+    // out = a*x + b*y with the ghosts of y taken as Boundary_C(y) at RK stage `stage`; out is neither x nor y
+    void (*combine_bc)(const GridGeom& g, const double* x, const double* y, double* out, double a, double b,
+                       int with_cfl, DevScalars* sc, int stage, cudaStream_t s);
     void (*cfl)(const GridGeom& g, const double* u, DevScalars* sc, cudaStream_t s);
     void (*dt_finalize)(const GridGeom& g, DevScalars* sc, double dtfinal, cudaStream_t s);
-    void (*advance_t)(DevScalars* sc, cudaStream_t s);
+    // a device-resident step's start at time t: dt from Setdt, counters cleared
+    void (*step_begin)(const GridGeom& g, DevScalars* sc, double t, cudaStream_t s);
     // MOOD passes 2, 3, ... of RK stage `stage` in one cooperative launch; the
     // pass count goes to sc->passes_stage[stage]; returns -1 if the launch failed
     int (*mood_loop)(const StageArgs& a, const GpWeights& w, GridBar* bar, int max_pass, int stage,

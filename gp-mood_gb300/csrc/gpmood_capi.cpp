@@ -12,6 +12,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <stddef.h>
+
 #include <new>
 
 #include "../../include/gpmood.h"
@@ -33,13 +35,15 @@ struct gpmood_ctx {
     int* dList[2];
     DevScalars* dSc;
     DevScalars* hSc;              // pinned mirror
-    GridBar* dBar;                // barrier of the cooperative MOOD loop
-    GridBar* hBar;                // pinned mirror
+    GridBar* dBar;                // barrier of the cooperative MOOD loop, directly behind dSc
+    GridBar* hBar;                // pinned mirror, directly behind hSc
     int* hCount;                  // pinned troubled count
     double t;                     // host mirror of the time
     int niter;
     bool have_state;
     bool dt_pending;              // dSc->dtmin_bits holds Setdt of dU
+    bool ghosts_done;             // dU's ghosts are Boundary_C's already (the last step's combination)
+    const int8_t* ordLast;        // CellGPO that gpmood_get_orders returns
     gpmood_counters ctr;
     NnGate* nn;                   // a-priori gate and training kernels
     NnRef* nnref;                 // the reference's own network (nn_reference = 1)
@@ -142,11 +146,20 @@ StageArgs stage_args(gpmood_ctx* c, const double* uin, double* uout, int stage, 
     return a;
 }
 
+// Boundary types whose ghosts are copies of interior cells (up to a sign): the
+// same bits come out whether Boundary_C or a combination of arrays that have
+// had it fills them, at any t_rk.
+bool bc_copies(int bc) {
+    return bc == GPMOOD_NEUMANN || bc == GPMOOD_PERIODIC || bc == GPMOOD_REFLECTIVE || bc == GPMOOD_KH;
+}
+
 // One Forward_Euler stage (mod_FE.f90:20-190) from uin (device) into uout;
 // `stage` counts the Forward_Euler calls of the step, bc_stage selects t_rk
-// for time-dependent boundaries (0: t, 1: t+dt, 2: t+dt/2).  Nothing here
-// waits for the GPU: pass counts and status come back once per step.
-int run_stage(gpmood_ctx* c, double* uin, double* uout, int stage, int bc_stage) {
+// for time-dependent boundaries (0: t, 1: t+dt, 2: t+dt/2).  bc_in: uin's ghosts
+// may not be Boundary_C's yet; bc_out: fill uout's (otherwise the caller's
+// combination does).  Nothing here waits for the GPU: pass counts and status
+// come back once per step.
+int run_stage(gpmood_ctx* c, double* uin, double* uout, int stage, int bc_stage, bool bc_in, bool bc_out) {
     static const char* const kName[GPM_MAXST] = {"Forward_Euler 1", "Forward_Euler 2", "Forward_Euler 3",
                                                  "Forward_Euler 4", "Forward_Euler 5"};
     NvtxRange range(kName[stage < GPM_MAXST ? stage : GPM_MAXST - 1]);
@@ -154,23 +167,26 @@ int run_stage(gpmood_ctx* c, double* uin, double* uout, int stage, int bc_stage)
     const KernelTable& kt = *c->kt;
     cudaEvent_t* ev = c->ev[stage];
     bool uniform = true, fixup = false, nnref = false;
-    CU(cudaMemsetAsync(c->dOrder, c->p.mord, c->ncell, s));  // CellGPO = mord, :48
-    CU(cudaMemsetAsync(c->dSc->ntrb, 0, sizeof(c->dSc->ntrb), s));
+    int8_t* const order = c->dStageOrd + (size_t)stage * c->ncell;  // the stage's own CellGPO
+    c->ordLast = order;
     const bool nn_on = c->p.method == GPMOOD_NN_GP_MOOD && c->niter + 1 > c->p.nsteps_with_no_nn;  // :51
+    if (nn_on) CU(cudaMemsetAsync(order, c->p.mord, c->ncell, s));  // CellGPO = mord, :48 (else the update's)
     if (nn_on && c->p.nn_reference) {
         // the reference's network sets every CellGPO to 1 or 3; it reads Uin
         // before Boundary_C, as mod_FE.f90:51-56 come before :64
-        const int rc = nn_ref_orders(c->nnref, c->g, uin, c->dOrder, &c->dSc->apriori_step, nullptr,
+        const int rc = nn_ref_orders(c->nnref, c->g, uin, order, &c->dSc->apriori_step, nullptr,
                                      c->cc ? c->dCcw : nullptr, s);
         if (rc < 0) return fail(c, GPMOOD_E_CUDA, "NN gate: %s", cudaGetErrorString(cudaGetLastError()));
         c->ctr.kernel_launches += rc;
         nnref = true;
         uniform = false;
     }
-    c->kt->bc(c->g, uin, c->dSc, bc_stage, s);  // Boundary_C(Uin), :64
-    c->ctr.kernel_launches += 2;
+    if (bc_in || !bc_copies(c->p.bc_type)) {
+        c->kt->bc(c->g, uin, c->dSc, bc_stage, s);  // Boundary_C(Uin), :64
+        c->ctr.kernel_launches += 1;
+    }
     if (nn_on && !c->p.nn_reference) {  // gated cells start at mord-2 and are listed in tlist[1]
-        const int rc = nn_gate_orders(c->nn, c->g, uin, c->dOrder, &c->dSc->apriori_step, c->dList[1],
+        const int rc = nn_gate_orders(c->nn, c->g, uin, order, &c->dSc->apriori_step, c->dList[1],
                                       &c->dSc->ntrb[1], nullptr, &c->dSc->status, s);
         if (rc < 0) return fail(c, GPMOOD_E_CUDA, "NN gate: %s", cudaGetErrorString(cudaGetLastError()));
         c->ctr.kernel_launches += rc;
@@ -178,6 +194,7 @@ int run_stage(gpmood_ctx* c, double* uin, double* uout, int stage, int bc_stage)
         uniform = false;
     }
     StageArgs a = stage_args(c, uin, uout, stage, uniform);
+    a.order = order;
     if (nnref) a.g.dmp = 0;  // NN_DETECTION: NaN and positivity only (mod_subroutine_NN_MOOD.f90:22-35)
     if (nnref && c->cc) {    // NN_GP_MOOD_CC_ reconstruction (mod_Reconstruction.f90:26-31)
         a.ccw = c->dCcw;
@@ -215,15 +232,16 @@ int run_stage(gpmood_ctx* c, double* uin, double* uout, int stage, int bc_stage)
         c->ctr.kernel_launches += 1;
     }
     if (c->timing) cudaEventRecord(ev[3], s);
-    CU(cudaMemcpyAsync(c->dStageOrd + (size_t)stage * c->ncell, c->dOrder, c->ncell, cudaMemcpyDeviceToDevice, s));
     if (stage == 0 && c->hvX) {  // training samples of stage 1 (mod_FE.f90:176-181)
-        if (nn_harvest(c->g, uin, c->dOrder, c->hvX, c->hvY, c->hvCap, c->hvCount, c->hvKeep,
+        if (nn_harvest(c->g, uin, order, c->hvX, c->hvY, c->hvCap, c->hvCount, c->hvKeep,
                        c->hvSeed * 2654435761u + (unsigned)c->ctr.steps, s))
             return fail(c, GPMOOD_E_CUDA, "NN harvest: %s", cudaGetErrorString(cudaGetLastError()));
         c->ctr.kernel_launches += 1;
     }
-    kt.bc(c->g, uout, c->dSc, bc_stage, s);  // the last DETECTION's Boundary_C(Uout)
-    c->ctr.kernel_launches += 2;
+    if (bc_out) {
+        kt.bc(c->g, uout, c->dSc, bc_stage, s);  // the last DETECTION's Boundary_C(Uout)
+        c->ctr.kernel_launches += 1;
+    }
     if (c->p.integrator == GPMOOD_SSP_RK4) {  // SSP_RK4_ takes the increment, mod_FE.f90:188
         const double* x[2] = {uout, uin};
         const double k[2] = {1.0, -1.0};
@@ -234,7 +252,7 @@ int run_stage(gpmood_ctx* c, double* uin, double* uout, int stage, int bc_stage)
 }
 
 // SSP_RK4_, mod_SSP_RK4.f90:12-38, with the constants of constants.f90:46-51.
-int run_rk4(gpmood_ctx* c, double* u, double* ur, bool with_cfl) {
+int run_rk4(gpmood_ctx* c, double* u, double* ur, bool with_cfl, bool bc_in) {
     const KernelTable& kt = *c->kt;
     cudaStream_t s = c->stream;
     const double c1 = 0.391752226571890, a20 = 0.444370493651235, a21 = 0.555629506348765,
@@ -245,31 +263,31 @@ int run_rk4(gpmood_ctx* c, double* u, double* ur, bool with_cfl) {
     double *U1 = c->dU1, *U2 = c->dU2, *U3 = c->dRk4[0], *U4 = c->dRk4[1], *FU3 = c->dRk4[2], *FU4 = c->dRk4[3],
            *Fl = c->dRk4[4];
     int rc;
-    if ((rc = run_stage(c, u, Fl, 0, 0))) return rc;
+    if ((rc = run_stage(c, u, Fl, 0, 0, bc_in, true))) return rc;
     {
         const double* x[2] = {u, Fl};
         const double k[2] = {1.0, c1};
         kt.lincomb(c->g, U1, 2, x, k, 0, c->dSc, s);
     }
-    if ((rc = run_stage(c, U1, Fl, 1, 0))) return rc;
+    if ((rc = run_stage(c, U1, Fl, 1, 0, false, true))) return rc;
     {
         const double* x[3] = {u, U1, Fl};
         const double k[3] = {a20, a21, c2};
         kt.lincomb(c->g, U2, 3, x, k, 0, c->dSc, s);
     }
-    if ((rc = run_stage(c, U2, Fl, 2, 0))) return rc;
+    if ((rc = run_stage(c, U2, Fl, 2, 0, false, true))) return rc;
     {
         const double* x[3] = {u, U2, Fl};
         const double k[3] = {a30, a32, c3};
         kt.lincomb(c->g, U3, 3, x, k, 0, c->dSc, s);
     }
-    if ((rc = run_stage(c, U3, FU3, 3, 0))) return rc;
+    if ((rc = run_stage(c, U3, FU3, 3, 0, false, true))) return rc;
     {
         const double* x[3] = {u, U3, FU3};
         const double k[3] = {a40, a43, c4};
         kt.lincomb(c->g, U4, 3, x, k, 0, c->dSc, s);
     }
-    if ((rc = run_stage(c, U4, FU4, 4, 0))) return rc;
+    if ((rc = run_stage(c, U4, FU4, 4, 0, false, true))) return rc;
     {
         const double* x[5] = {U2, U3, FU3, U4, FU4};
         const double k[5] = {f2, f3, ff3, f4, ff4};
@@ -283,35 +301,34 @@ int run_rk4(gpmood_ctx* c, double* u, double* ur, bool with_cfl) {
 // configured integrator; t, dt, qx, qy already on the device.  with_cfl fuses
 // the next step's Setdt into the final combination.  One host
 // synchronisation per step, at its end.
-int run_step(gpmood_ctx* c, double* u, double* ur, bool with_cfl) {
+// bc_in: u's ghosts may not be Boundary_C's.
+int run_step(gpmood_ctx* c, double* u, double* ur, bool with_cfl, bool bc_in) {
     NvtxRange range("time_stepping");
     cudaStream_t s = c->stream;
-    CU(cudaMemsetAsync(&c->dSc->detected_step, 0, 2 * sizeof(unsigned long long), s));
-    CU(cudaMemsetAsync(&c->dSc->status, 0, sizeof(int), s));  // this step's flags (counters keep them all)
     int rc = 0;
     if (c->p.integrator == GPMOOD_SSP_RK3) {  // SSP_RK3_, mod_SSP_RK3.f90:12-39
-        rc = run_stage(c, u, c->dU1, 0, 0);
+        rc = run_stage(c, u, c->dU1, 0, 0, bc_in, true);
         if (rc) return rc;
-        rc = run_stage(c, c->dU1, c->dU2, 1, 1);
+        rc = run_stage(c, c->dU1, c->dU2, 1, 1, false, false);
         if (rc) return rc;
-        c->kt->combine(c->g, u, c->dU2, 0.75, 0.25, 0, c->dSc, s);  // U2 = 0.75 Uin + 0.25 U2
+        c->kt->combine_bc(c->g, u, c->dU2, c->dU1, 0.75, 0.25, 0, c->dSc, 1, s);  // U2 = 0.75 Uin + 0.25 U2
         c->ctr.kernel_launches += 2;
-        rc = run_stage(c, c->dU2, ur, 2, 2);
+        rc = run_stage(c, c->dU1, c->dU2, 2, 2, false, false);
         if (rc) return rc;
-        c->kt->combine(c->g, u, ur, 1. / 3, 2. / 3, with_cfl ? 1 : 0, c->dSc, s);  // Uout = Uin/3 + 2 Uout/3
+        c->kt->combine_bc(c->g, u, c->dU2, ur, 1. / 3, 2. / 3, with_cfl ? 1 : 0, c->dSc, 2, s);  // Uin/3 + 2 Uout/3
     } else if (c->p.integrator == GPMOOD_SSP_RK2) {  // SSP_RK2_, mod_SSP_RK2.f90:12-24 (t_rk = t)
-        rc = run_stage(c, u, c->dU1, 0, 0);
+        rc = run_stage(c, u, c->dU1, 0, 0, bc_in, true);
         if (rc) return rc;
-        rc = run_stage(c, c->dU1, ur, 1, 0);
+        rc = run_stage(c, c->dU1, c->dU2, 1, 0, false, false);
         if (rc) return rc;
         // 0.5*(Uin+Uout): both halvings are exact, so 0.5*Uin + 0.5*Uout rounds the same
-        c->kt->combine(c->g, u, ur, 0.5, 0.5, with_cfl ? 1 : 0, c->dSc, s);
+        c->kt->combine_bc(c->g, u, c->dU2, ur, 0.5, 0.5, with_cfl ? 1 : 0, c->dSc, 0, s);
         c->ctr.kernel_launches += 1;
     } else if (c->p.integrator == GPMOOD_SSP_RK4) {
-        rc = run_rk4(c, u, ur, with_cfl);
+        rc = run_rk4(c, u, ur, with_cfl, bc_in);
         if (rc) return rc;
     } else {  // FE: one Forward_Euler (time_stepper.f90:18)
-        rc = run_stage(c, u, ur, 0, 0);
+        rc = run_stage(c, u, ur, 0, 0, bc_in, true);
         if (rc) return rc;
         if (with_cfl) {
             c->kt->cfl(c->g, ur, c->dSc, s);
@@ -320,8 +337,7 @@ int run_step(gpmood_ctx* c, double* u, double* ur, bool with_cfl) {
     }
     rc = check_launch(c, "combine");
     if (rc) return rc;
-    CU(cudaMemcpyAsync(c->hSc, c->dSc, sizeof(DevScalars), cudaMemcpyDeviceToHost, s));
-    CU(cudaMemcpyAsync(c->hBar, c->dBar, sizeof(GridBar), cudaMemcpyDeviceToHost, s));
+    CU(cudaMemcpyAsync(c->hSc, c->dSc, sizeof(DevScalars) + sizeof(GridBar), cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
     const bool mood = c->p.method == GPMOOD_GP_MOOD || c->p.method == GPMOOD_NN_GP_MOOD;
     long long passes = 0;
@@ -358,6 +374,7 @@ int run_step(gpmood_ctx* c, double* u, double* ur, bool with_cfl) {
         if (c->wait_limit) cudaMemcpyAsync(&c->dBar->limit, &c->wait_limit, sizeof(int), cudaMemcpyHostToDevice, s);
         cudaMemsetAsync(c->dStamp, 0, c->ncell * sizeof(unsigned), s);
         cudaMemsetAsync(&c->dSc->stamp_epoch, 0, sizeof(unsigned), s);
+        cudaMemsetAsync(c->dSc->ntrb, 0, sizeof(c->dSc->ntrb), s);
         cudaStreamSynchronize(s);
         return fail(c, GPMOOD_E_CUDA, "MOOD loop: grid barrier timed out");
     }
@@ -370,13 +387,16 @@ int run_step(gpmood_ctx* c, double* u, double* ur, bool with_cfl) {
     return 0;
 }
 
-// Put t, dt and dt/dx, dt/dy computed on the host (IEEE, same bits) on the device.
+// Put t, dt and dt/dx, dt/dy computed on the host (IEEE, same bits) on the
+// device and clear the step's counters and flags.
 int set_time(gpmood_ctx* c, double t, double dt) {
     c->hSc->t = t;
     c->hSc->dt = dt;
     c->hSc->qx = dt / c->g.dx;
     c->hSc->qy = dt / c->g.dy;
-    CU(cudaMemcpyAsync(c->dSc, c->hSc, 4 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    c->hSc->detected_step = c->hSc->apriori_step = 0;
+    c->hSc->status = 0;
+    CU(cudaMemcpyAsync(c->dSc, c->hSc, offsetof(DevScalars, tmax), cudaMemcpyHostToDevice, c->stream));
     return 0;
 }
 
@@ -418,9 +438,8 @@ void free_all(gpmood_ctx* c) {
     if (!c) return;
     cudaFree(c->dU); cudaFree(c->dUr); cudaFree(c->dU1); cudaFree(c->dU2);
     cudaFree(c->dFx); cudaFree(c->dFy); cudaFree(c->dOrder); cudaFree(c->dStamp);
-    cudaFree(c->dList[0]); cudaFree(c->dList[1]); cudaFree(c->dSc); cudaFree(c->dStageOrd); cudaFree(c->dBar);
+    cudaFree(c->dList[0]); cudaFree(c->dList[1]); cudaFree(c->dSc); cudaFree(c->dStageOrd);
     for (int i = 0; i < 5; i++) cudaFree(c->dRk4[i]);
-    if (c->hBar) cudaFreeHost(c->hBar);
     if (c->hSc) cudaFreeHost(c->hSc);
     if (c->hCount) cudaFreeHost(c->hCount);
     if (c->nn) nn_gate_destroy(c->nn);
@@ -549,15 +568,14 @@ int gpmood_create(const gpmood_params* p, gpmood_ctx** out) {
     ALLOC(c->dStamp, c->ncell * sizeof(unsigned));
     ALLOC(c->dList[0], c->ncell * sizeof(int));
     ALLOC(c->dList[1], c->ncell * sizeof(int));
-    ALLOC(c->dSc, sizeof(DevScalars));
+    ALLOC(c->dSc, sizeof(DevScalars) + sizeof(GridBar));
     ALLOC(c->dStageOrd, GPM_MAXST * c->ncell);
     if (p->integrator == GPMOOD_SSP_RK4)
         for (int i = 0; i < 5; i++) ALLOC(c->dRk4[i], sb);
-    ALLOC(c->dBar, sizeof(GridBar));
+    c->dBar = reinterpret_cast<GridBar*>(c->dSc + 1);
 #undef ALLOC
-    if (cudaMallocHost((void**)&c->hSc, sizeof(DevScalars)) != cudaSuccess ||
+    if (cudaMallocHost((void**)&c->hSc, sizeof(DevScalars) + sizeof(GridBar)) != cudaSuccess ||
         cudaMallocHost((void**)&c->hCount, sizeof(int)) != cudaSuccess ||
-        cudaMallocHost((void**)&c->hBar, sizeof(GridBar)) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
         fail(c, GPMOOD_E_CUDA, "pinned memory / stream creation failed");
         free_all(c);
@@ -572,7 +590,9 @@ int gpmood_create(const gpmood_params* p, gpmood_ctx** out) {
             return GPMOOD_E_CUDA;
         }
     }
-    memset(c->hSc, 0, sizeof(DevScalars));
+    c->hBar = reinterpret_cast<GridBar*>(c->hSc + 1);
+    memset(c->hSc, 0, sizeof(DevScalars) + sizeof(GridBar));
+    c->ordLast = c->dStageOrd;
     c->hSc->tmax = p->tmax;
     c->hSc->cfl = p->cfl;
     if (p->bc_type == GPMOOD_DIRICHLET)  // BC.f90:68: sin() on the host, as the CPU restatement does
@@ -705,7 +725,7 @@ int gpmood_time_stepping(gpmood_ctx* c, const double* uin_host, double* uout_hos
     CU(cudaMemcpyAsync(c->dU, uin_host, state_bytes(c), cudaMemcpyHostToDevice, c->stream));
     int rc = set_time(c, t, dt);
     if (rc) return rc;
-    rc = run_step(c, c->dU, c->dUr, false);
+    rc = run_step(c, c->dU, c->dUr, false, true);
     if (rc) return rc;
     CU(cudaMemcpyAsync(uout_host, c->dUr, state_bytes(c), cudaMemcpyDeviceToHost, c->stream));
     CU(cudaStreamSynchronize(c->stream));
@@ -732,7 +752,7 @@ int gpmood_setdt_time_stepping(gpmood_ctx* c, const double* uin_host, double* uo
         return fail(c, GPMOOD_E_DT, "Setdt produced dt = %g", dt);
     rc = set_time(c, t, dt);
     if (rc) return rc;
-    rc = run_step(c, c->dU, c->dUr, false);
+    rc = run_step(c, c->dU, c->dUr, false, true);
     if (rc) return rc;
     CU(cudaMemcpyAsync(uout_host, c->dUr, state_bytes(c), cudaMemcpyDeviceToHost, c->stream));
     CU(cudaStreamSynchronize(c->stream));
@@ -744,7 +764,7 @@ int gpmood_time_stepping_dev(gpmood_ctx* c, double* d_uin, double* d_uout, doubl
     if (!(dt > 0) || !isfinite(dt)) return fail(c, GPMOOD_E_DT, "dt = %g", dt);
     int rc = set_time(c, t, dt);
     if (rc) return rc;
-    return run_step(c, d_uin, d_uout, false);
+    return run_step(c, d_uin, d_uout, false, true);
 }
 
 int gpmood_set_state(gpmood_ctx* c, const double* u_host, double t) {
@@ -757,6 +777,7 @@ int gpmood_set_state(gpmood_ctx* c, const double* u_host, double t) {
     c->niter = 0;
     c->have_state = true;
     c->dt_pending = false;
+    c->ghosts_done = false;
     return 0;
 }
 
@@ -782,6 +803,7 @@ int gpmood_set_state_dev(gpmood_ctx* c, const double* d_u, double t) {
     c->niter = 0;
     c->have_state = true;
     c->dt_pending = false;
+    c->ghosts_done = false;
     return 0;
 }
 
@@ -796,7 +818,7 @@ int gpmood_get_state_dev(gpmood_ctx* c, double* d_u) {
 int gpmood_get_orders(gpmood_ctx* c, signed char* orders) {
     if (!c || !orders) return fail(c, GPMOOD_E_ARG, "NULL argument");
     // CellGPO(1:lf, 1:nf): interior rows of the padded order array.
-    CU(cudaMemcpy2DAsync(orders, (size_t)c->p.lf, c->dOrder + (size_t)(GPM_NGC) * c->g.nx + GPM_NGC,
+    CU(cudaMemcpy2DAsync(orders, (size_t)c->p.lf, c->ordLast + (size_t)(GPM_NGC) * c->g.nx + GPM_NGC,
                          (size_t)c->g.nx, (size_t)c->p.lf, (size_t)c->p.nf, cudaMemcpyDeviceToHost, c->stream));
     CU(cudaStreamSynchronize(c->stream));
     return 0;
@@ -814,17 +836,18 @@ int gpmood_advance(gpmood_ctx* c, int nsteps, int* steps_done) {
             c->kt->cfl(c->g, c->dU, c->dSc, c->stream);
             c->ctr.kernel_launches += 1;
         }
-        c->kt->dt_finalize(c->g, c->dSc, -1.0, c->stream);
+        c->kt->step_begin(c->g, c->dSc, c->t, c->stream);
         c->ctr.kernel_launches += 1;
-        int rc = run_step(c, c->dU, c->dUr, true);
+        const bool bc_in = !c->ghosts_done;
+        c->ghosts_done = false;
+        int rc = run_step(c, c->dU, c->dUr, true, bc_in);
         if (rc) return rc;
         if (c->hSc->status & GPM_STATUS_DT) return fail(c, GPMOOD_E_DT, "Setdt produced dt = %g", c->hSc->dt);
-        c->kt->advance_t(c->dSc, c->stream);  // t = t + dt
-        c->ctr.kernel_launches += 1;
+        c->ghosts_done = true;
         double* tmp = c->dU;                   // U = Ur
         c->dU = c->dUr;
         c->dUr = tmp;
-        c->t = c->hSc->t + c->hSc->dt;
+        c->t = c->hSc->t + c->hSc->dt;         // t = t + dt (main.f90:160)
         c->niter++;
         if (c->trace)
             fprintf(stderr, "[gpmood] step %d t=%.9e dt=%.9e detected=%lld passes=%lld status=%d\n", c->niter,
@@ -906,6 +929,7 @@ int gpmood_nn_ref_logits(gpmood_ctx* c, float* d_logits) {
     if (!c || !d_logits) return fail(c, GPMOOD_E_ARG, "NULL argument");
     if (!c->have_state) return fail(c, GPMOOD_E_STATE, "no device-resident state (call gpmood_set_state)");
     if (!c->p.nn_reference || !nn_ref_loaded(c->nnref)) return fail(c, GPMOOD_E_STATE, "no reference network loaded");
+    c->ordLast = c->dOrder;
     CU(cudaMemsetAsync(&c->dSc->apriori_step, 0, sizeof(unsigned long long), c->stream));
     if (nn_ref_orders(c->nnref, c->g, c->dU, c->dOrder, &c->dSc->apriori_step, d_logits, c->cc ? c->dCcw : nullptr,
                       c->stream) < 0)
@@ -918,6 +942,7 @@ int gpmood_nn_gate_logits(gpmood_ctx* c, float* d_logits) {
     if (!c || !d_logits) return fail(c, GPMOOD_E_ARG, "NULL argument");
     if (!c->have_state) return fail(c, GPMOOD_E_STATE, "no device-resident state (call gpmood_set_state)");
     if (c->p.nn_reference || !nn_gate_loaded(c->nn)) return fail(c, GPMOOD_E_STATE, "no gate parameters loaded");
+    c->ordLast = c->dOrder;
     CU(cudaMemsetAsync(c->dOrder, c->p.mord, c->ncell, c->stream));
     CU(cudaMemsetAsync(&c->dSc->apriori_step, 0, sizeof(unsigned long long), c->stream));
     CU(cudaMemsetAsync(c->dSc->ntrb, 0, sizeof(c->dSc->ntrb), c->stream));
@@ -959,6 +984,7 @@ int gpmood_nn_predict(gpmood_ctx* c, signed char* gated, long long* n_gated) {
     const bool ref = c->p.nn_reference != 0;
     if (ref ? !nn_ref_loaded(c->nnref) : !nn_gate_loaded(c->nn))
         return fail(c, GPMOOD_E_STATE, "no network parameters (gpmood_set_nn)");
+    c->ordLast = c->dOrder;
     CU(cudaMemsetAsync(c->dOrder, c->p.mord, c->ncell, c->stream));
     CU(cudaMemsetAsync(&c->dSc->apriori_step, 0, sizeof(unsigned long long), c->stream));
     CU(cudaMemsetAsync(c->dSc->ntrb, 0, sizeof(c->dSc->ntrb), c->stream));

@@ -6,7 +6,7 @@
 //   -DGPM_EXACT=0 --fmad=true   -> namespace gpm_fast
 //
 // One stage (Forward_Euler, gp-mood-code/mod_FE.f90:20-190) runs as:
-//   k_bc_x / k_bc_y       Boundary_C(Uin)                      BC.f90:10-421
+//   k_bc                  Boundary_C(Uin)                      BC.f90:10-421
 //   k_flux_xy_tma         every face: GP recon + HLLC + quadrature, stored
 //   (k_flux_tile<x|y>)    (the first MOOD pass, mod_FE.f90:73-145); fast mode
 //                         both directions per tile, exact mode one per launch
@@ -18,9 +18,10 @@
 //                         recompute the 4 faces of each troubled cell, then
 //                         Uout of its 5-point cross with DETECTION there ->
 //                         next list
-//   k_bc_x / k_bc_y       Boundary_C(Uout)
-//   k_combine             SSP-RK3 combination (mod_SSP_RK3.f90:28,33), with
-//                         the next step's Setdt reduction fused into the last
+//   k_bc                  Boundary_C(Uout)
+//   k_combine_bc          SSP-RK3 combination (mod_SSP_RK3.f90:28,33) with
+//                         Boundary_C(Uout) of the stage before it and, in the
+//                         last, the next step's Setdt reduction
 //
 // Why the list-based loop equals the reference's full-grid loop: after a
 // DETECTION pass the reference flags exactly the faces of troubled cells and
@@ -57,7 +58,8 @@ __device__ __forceinline__ size_t cidx(const GridGeom& g, int l, int n) {
 // ---------------------------------------------------------------------------
 // Boundary_C, BC.f90:10-421.  Pass 1 fills the ghost columns of interior rows,
 // pass 2 the ghost rows of every column (so corners come from pass 1 values,
-// as in the reference's loop nest).
+// as in the reference's loop nest).  Each of the two passes as a launch cost
+// ~3.4 us, twelve times a step.
 
 __device__ __forceinline__ void p2c(double r, double u, double v, double p, double* out) {
     out[0] = r;
@@ -73,114 +75,121 @@ __device__ __forceinline__ void f_dmr(double x, double y, double* r) {  // IC.f9
     else p2c(1.4, 0.0, 0.0, 1.0, r);
 }
 
-__global__ void k_bc_x(GridGeom g, double* __restrict__ u, const DevScalars* __restrict__ sc, int stage) {
-    const int n = 1 + blockIdx.x * blockDim.y + threadIdx.y;   // interior row
-    const int k = threadIdx.x;                                  // 0..7: 4 left + 4 right ghosts
-    if (n > g.nf || k >= 2 * GPM_NGC) return;
-    const bool right = k >= GPM_NGC;
-    const int j = right ? k - GPM_NGC : k;                      // 0..3
-    const int l = right ? g.lf + 1 + j : -j;                    // right: lf+1..lf+4, left: 0..-3
-    double* dst = u + 4 * cidx(g, l, n);
-    if (g.bc_type == 17) {  // Neumann
-        const double* src = u + 4 * cidx(g, right ? g.lf : 1, n);
-        for (int v = 0; v < 4; v++) dst[v] = src[v];
-    } else if (g.bc_type == 18) {  // Periodic
-        const int ls = right ? 1 + j : g.lf - j;
-        const double* src = u + 4 * cidx(g, ls, n);
-        for (int v = 0; v < 4; v++) dst[v] = src[v];
-    } else if (g.bc_type == 20) {  // Reflective: mirror, flip normal momentum
-        const int ls = right ? g.lf - j : 1 + j;
-        const double* src = u + 4 * cidx(g, ls, n);
-        dst[0] = src[0]; dst[1] = -src[1]; dst[2] = src[2]; dst[3] = src[3];
-    } else if (g.bc_type == 35) {  // DMR: exact pre/post-shock states
-        f_dmr(l * g.dx - g.dx / 2, n * g.dy - g.dy / 2, dst);
-    } else if (g.bc_type == 19) {  // Dirichlet: the right states come from the host (sin), BC.f90:61-75
-        if (right) {
-            for (int v = 0; v < 4; v++) dst[v] = sc->bcd[j][v];
-        } else {
-            p2c(3.857143, 2.629369, 0., 10.33333, dst);
-        }
-    } else if (g.bc_type == 201 || g.bc_type == 301) {  // Mach800 jets: outflow in x, BC.f90:137-152
-        const double* src = u + 4 * cidx(g, right ? g.lf : 1, n);
-        for (int v = 0; v < 4; v++) dst[v] = src[v];
-    } else if (g.bc_type == 401) {  // RMI: inflow left, outflow right, BC.f90:243-256
-        if (right) {
-            const double* src = u + 4 * cidx(g, g.lf, n);
-            for (int v = 0; v < 4; v++) dst[v] = src[v];
-        } else {
-            p2c(2.666666666666667, 2. * sqrt(1.4), 0., 4.5, dst);
-        }
-    } else if (g.bc_type == 402) {  // RT: reflective in x, BC.f90:344-362
-        const int ls = right ? g.lf - j : 1 + j;
-        const double* src = u + 4 * cidx(g, ls, n);
-        dst[0] = src[0]; dst[1] = -src[1]; dst[2] = src[2]; dst[3] = src[3];
-    } else if (g.bc_type == 403) {  // KH: periodic in x, BC.f90:394-400
-        const int ls = right ? 1 + j : g.lf - j;
-        const double* src = u + 4 * cidx(g, ls, n);
-        for (int v = 0; v < 4; v++) dst[v] = src[v];
+// The value that pass 1 gives the ghost column l <= 0 or l > lf of interior
+// row n, from the interior of u.
+__device__ __forceinline__ Cell bc_x_cell(const GridGeom& g, const double* __restrict__ u,
+                                          const DevScalars* __restrict__ sc, int l, int n) {
+    const bool right = l > g.lf;
+    const int j = right ? l - g.lf - 1 : -l;  // 0..3
+    auto at = [&](int ls) { return ld_cell_cg(u + 4 * cidx(g, ls, n)); };
+    double w[4];
+    switch (g.bc_type) {
+    case 18:  // Periodic
+    case 403:  // KH: periodic in x, BC.f90:394-400
+        return at(right ? 1 + j : g.lf - j);
+    case 20:     // Reflective: mirror, flip normal momentum
+    case 402: {  // RT: reflective in x, BC.f90:344-362
+        Cell c = at(right ? g.lf - j : 1 + j);
+        c.mx = -c.mx;
+        return c;
     }
+    case 35:  // DMR: exact pre/post-shock states
+        f_dmr(l * g.dx - g.dx / 2, n * g.dy - g.dy / 2, w);
+        break;
+    case 19:  // Dirichlet: the right states come from the host (sin), BC.f90:61-75
+        if (right) return Cell{sc->bcd[j][0], sc->bcd[j][1], sc->bcd[j][2], sc->bcd[j][3]};
+        p2c(3.857143, 2.629369, 0., 10.33333, w);
+        break;
+    case 401:  // RMI: inflow left, outflow right, BC.f90:243-256
+        if (right) return at(g.lf);
+        p2c(2.666666666666667, 2. * sqrt(1.4), 0., 4.5, w);
+        break;
+    default:  // 17 Neumann; 201, 301 Mach800 jets: outflow in x, BC.f90:137-152
+        return at(right ? g.lf : 1);
+    }
+    return Cell{w[0], w[1], w[2], w[3]};
 }
 
-__global__ void k_bc_y(GridGeom g, double* __restrict__ u, const DevScalars* __restrict__ sc, int stage) {
-    const int l = (int)(blockIdx.x * blockDim.y + threadIdx.y) - 3;  // every column incl. ghosts
-    const int k = threadIdx.x;
-    if (l > g.lf + GPM_NGC || k >= 2 * GPM_NGC) return;
-    const bool top = k >= GPM_NGC;
-    const int j = top ? k - GPM_NGC : k;
-    const int n = top ? g.nf + 1 + j : -j;
-    double* dst = u + 4 * cidx(g, l, n);
-    if (g.bc_type == 17) {
-        const double* src = u + 4 * cidx(g, l, top ? g.nf : 1);
-        for (int v = 0; v < 4; v++) dst[v] = src[v];
-    } else if (g.bc_type == 18) {
-        const int ns = top ? 1 + j : g.nf - j;
-        const double* src = u + 4 * cidx(g, l, ns);
-        for (int v = 0; v < 4; v++) dst[v] = src[v];
-    } else if (g.bc_type == 20) {
-        const int ns = top ? g.nf - j : 1 + j;
-        const double* src = u + 4 * cidx(g, l, ns);
-        dst[0] = src[0]; dst[1] = src[1]; dst[2] = -src[2]; dst[3] = src[3];
-    } else if (g.bc_type == 35) {
+// Boundary_C's value of ghost cell (l, n): pass 1's in interior rows, else
+// pass 2's, whose source columns outside the interior are pass 1's values.
+// Only interior cells are read, so both passes are one kernel.
+__device__ __forceinline__ Cell bc_cell(const GridGeom& g, const double* __restrict__ u,
+                                        const DevScalars* __restrict__ sc, int stage, int l, int n) {
+    if (n >= 1 && n <= g.nf) return bc_x_cell(g, u, sc, l, n);
+    const bool top = n > g.nf;
+    const int j = top ? n - g.nf - 1 : -n;
+    const bool inner = l >= 1 && l <= g.lf;
+    auto at = [&](int ns) { return inner ? ld_cell_cg(u + 4 * cidx(g, l, ns)) : bc_x_cell(g, u, sc, l, ns); };
+    double w[4];
+    switch (g.bc_type) {
+    case 18:
+        return at(top ? 1 + j : g.nf - j);
+    case 20:
+    case 401: {  // RMI: reflective in y, BC.f90:258-280
+        Cell c = at(top ? g.nf - j : 1 + j);
+        c.my = -c.my;
+        return c;
+    }
+    case 35: {
         const double x = l * g.dx - g.dx / 2;
         if (top) {
             // t_rk of the stage (mod_SSP_RK3.f90:22,26,29)
             const double t_rk = stage == 0 ? sc->t : (stage == 1 ? sc->t + sc->dt : sc->t + 0.5 * sc->dt);
             const double xmin = 1. / 6 + 10. * t_rk / (0.5 * sqrt(3.)) + 1. / sqrt(3.);
-            if (x < xmin) p2c(8., 7.1447096, -4.125, 116.5, dst);
-            else p2c(1.4, 0.0, 0.0, 1.0, dst);
+            if (x < xmin) p2c(8., 7.1447096, -4.125, 116.5, w);
+            else p2c(1.4, 0.0, 0.0, 1.0, w);
         } else if (x > 1. / 6) {
-            const double* src = u + 4 * cidx(g, l, 1 + j);
-            dst[0] = src[0]; dst[1] = src[1]; dst[2] = -src[2]; dst[3] = src[3];
+            Cell c = at(1 + j);
+            c.my = -c.my;
+            return c;
         } else {
-            p2c(8., 7.1447096, -4.125, 116.5, dst);
+            p2c(8., 7.1447096, -4.125, 116.5, w);
         }
-    } else if (g.bc_type == 19 || g.bc_type == 403) {  // Neumann in y (BC.f90:77-87, :402-413)
-        const double* src = u + 4 * cidx(g, l, top ? g.nf : 1);
-        for (int v = 0; v < 4; v++) dst[v] = src[v];
-    } else if (g.bc_type == 201 || g.bc_type == 301) {  // outflow, then the jets (BC.f90:154-178, :199-236)
-        const double* src = u + 4 * cidx(g, l, top ? g.nf : 1);
-        for (int v = 0; v < 4; v++) dst[v] = src[v];
-        if (fabs((l * g.dx - g.dx / 2) - 0.75) <= 0.05) {
-            if (!top) p2c(1.4, 0.0, 800.0, 1.0, dst);
-            else if (g.bc_type == 301) p2c(1.4, 0.0, -800.0, 1.0, dst);
+        break;
+    }
+    case 201:
+    case 301:  // outflow, then the jets (BC.f90:154-178, :199-236)
+        if (fabs((l * g.dx - g.dx / 2) - 0.75) <= 0.05 && (!top || g.bc_type == 301)) {
+            p2c(1.4, 0.0, top ? -800.0 : 800.0, 1.0, w);
+            break;
         }
-    } else if (g.bc_type == 401) {  // RMI: reflective in y, BC.f90:258-280
-        const int ns = top ? g.nf - j : 1 + j;
-        const double* src = u + 4 * cidx(g, l, ns);
-        dst[0] = src[0]; dst[1] = src[1]; dst[2] = -src[2]; dst[3] = src[3];
-    } else if (g.bc_type == 402) {  // RT: hydrostatic ghosts, g = real(0.1, 4), BC.f90:364-389
-        const double* q = u + 4 * cidx(g, l, top ? g.nf - j : 1 + j);
+        return at(top ? g.nf : 1);
+    case 402: {  // RT: hydrostatic ghosts, g = real(0.1, 4), BC.f90:364-389
+        const Cell c = at(top ? g.nf - j : 1 + j);
+        const double q[4] = {c.r, c.mx, c.my, c.e};
         const double grav = (double)0.1f;
         const double pr = (GPM_GAMMA - 1.) * (q[3] - (0.5 * (q[1] * q[1] + q[2] * q[2]) / q[0]));
         const double dp = 2 * j * g.dy * grav * q[0];
-        p2c(q[0], q[1] / q[0], -(q[2] / q[0]), top ? pr - dp : pr + dp, dst);
+        p2c(q[0], q[1] / q[0], -(q[2] / q[0]), top ? pr - dp : pr + dp, w);
+        break;
     }
+    default:  // 17; 19, 403: Neumann in y (BC.f90:77-87, :402-413)
+        return at(top ? g.nf : 1);
+    }
+    return Cell{w[0], w[1], w[2], w[3]};
+}
+
+// One thread per ghost cell: the 8 ghost columns of the interior rows, then
+// the 8 ghost rows.
+__global__ void __launch_bounds__(256) k_bc(GridGeom g, double* __restrict__ u, const DevScalars* __restrict__ sc,
+                                            int stage) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x, l, n;
+    if (i < 8 * g.nf) {
+        const int k = i & 7;
+        n = 1 + (i >> 3);
+        l = k < 4 ? -k : g.lf + k - 3;
+    } else {
+        i -= 8 * g.nf;
+        if (i >= 8 * g.nx) return;
+        const int k = i / g.nx;
+        l = i - k * g.nx - 3;
+        n = k < 4 ? -k : g.nf + k - 3;
+    }
+    st_cell(u + 4 * cidx(g, l, n), bc_cell(g, u, sc, stage, l, n));
 }
 
 void launch_bc(const GridGeom& g, double* u, const DevScalars* sc, int stage, cudaStream_t s) {
-    const dim3 blk(8, 32);
-    k_bc_x<<<(g.nf + 31) / 32, blk, 0, s>>>(g, u, sc, stage);
-    k_bc_y<<<(g.nx + 31) / 32, blk, 0, s>>>(g, u, sc, stage);
+    k_bc<<<(8 * (g.nf + g.nx) + 255) / 256, 256, 0, s>>>(g, u, sc, stage);
 }
 
 // ---------------------------------------------------------------------------
@@ -739,7 +748,8 @@ __global__ void __launch_bounds__(256) k_update_detect(StageArgs a, const __grid
         if (o > 1) trb = mood_troubled(uo, a.uin + 4 * c, g.nx, g, w.d2x, w.d2y);
         else if (inadmissible(uo)) atomicOr(&a.sc->status, GPM_STATUS_NAN);
     }
-    if (trb) cascade_order(&a.order[c]);
+    if (a.uniform_order) a.order[c] = (int8_t)(!trb ? g.mord : g.mord == 3 ? 1 : 3);  // CellGPO = mord, :48, lowered
+    else if (trb) cascade_order(&a.order[c]);
     list_append(trb, a.tlist[cur], &a.sc->ntrb[cur], (int)c);
 }
 
@@ -1211,7 +1221,7 @@ __global__ void __launch_bounds__(MOOD_THREADS, 1) k_mood_loop(StageArgs a, cons
     if (gtid == 0) {  // every CTA read the epoch before the first barrier
         a.sc->passes_stage[stage] = pass;
         a.sc->stamp_epoch = epoch + (unsigned)pass + 1u;
-        if (shared_lists) a.sc->ntrb[cur] = solo_ls.count[cur];
+        a.sc->ntrb[0] = a.sc->ntrb[1] = 0;  // for the next stage; CTAs that still poll leave on 0 as on the end
     }
 }
 
@@ -1367,6 +1377,30 @@ __global__ void __launch_bounds__(256) k_combine(GridGeom g, const double* __res
     if (with_cfl) dt_reduce(v, sc);
 }
 
+// The same combination out = a*x + b*y of a stage's y before Boundary_C(y):
+// a ghost cell of y is Boundary_C's value (bc_cell; stage selects t_rk), so the
+// stage needs no Boundary_C launch of its own.  out is neither x nor y.
+__global__ void __launch_bounds__(256) k_combine_bc(GridGeom g, const double* __restrict__ x,
+                                                    const double* __restrict__ y, double* __restrict__ out, double ca,
+                                                    double cb, int with_cfl, DevScalars* sc, int stage) {
+    const unsigned ncell = (unsigned)g.nx * (unsigned)g.ny;
+    double v = 1.0e30;
+    for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += gridDim.x * blockDim.x) {
+        const int n = (int)(c / (unsigned)g.nx) - 3, l = (int)(c - (unsigned)(n + 3) * g.nx) - 3;
+        const Cell a = ld_cell(x + 4 * (size_t)c);
+        const bool inner = l >= 1 && l <= g.lf && n >= 1 && n <= g.nf;
+        const Cell b = inner ? ld_cell(y + 4 * (size_t)c) : bc_cell(g, y, sc, stage, l, n);
+        Cell o;
+        o.r = ca * a.r + cb * b.r;
+        o.mx = ca * a.mx + cb * b.mx;
+        o.my = ca * a.my + cb * b.my;
+        o.e = ca * a.e + cb * b.e;
+        st_cell(out + 4 * (size_t)c, o);
+        if (with_cfl) v = fmin(v, cell_dt(o, g.dx, g.dy));
+    }
+    if (with_cfl) dt_reduce(v, sc);
+}
+
 // y = c[0]*x[0] + c[1]*x[1] + ... (n terms, summed left to right as the
 // reference's whole-array expressions of mod_SSP_RK4.f90:25-36 and
 // mod_FE.f90:188), over every cell; y may be one of the x.
@@ -1411,6 +1445,11 @@ void launch_combine(const GridGeom& g, const double* x, double* y, double a, dou
     k_combine<<<list_grid(g.nx * g.ny, 256), 256, 0, s>>>(g, x, y, a, b, with_cfl, sc);
 }
 
+void launch_combine_bc(const GridGeom& g, const double* x, const double* y, double* out, double a, double b,
+                       int with_cfl, DevScalars* sc, int stage, cudaStream_t s) {
+    k_combine_bc<<<list_grid(g.nx * g.ny, 256), 256, 0, s>>>(g, x, y, out, a, b, with_cfl, sc, stage);
+}
+
 // dt = CFL * min, clipped to dtfinal (physics.f90:292-296); qx = dt/dx.
 // dtfinal < 0 selects tmax - t (main.f90:149).
 __global__ void k_dt_finalize(GridGeom g, DevScalars* sc, double dtfinal_in) {
@@ -1430,12 +1469,30 @@ void launch_dt_finalize(const GridGeom& g, DevScalars* sc, double dtfinal, cudaS
     k_dt_finalize<<<1, 1, 0, s>>>(g, sc, dtfinal);
 }
 
-__global__ void k_advance_t(DevScalars* sc) { sc->t = sc->t + sc->dt; }  // main.f90:160
-void launch_advance_t(DevScalars* sc, cudaStream_t s) { k_advance_t<<<1, 1, 0, s>>>(sc); }
+// The start of a step of the device-resident loop (main.f90:149-160) at time
+// t: Setdt's dt, and the step's counters.
+__global__ void k_step_begin(GridGeom g, DevScalars* sc, double t) {
+    sc->t = t;
+    double dt = __longlong_as_double((long long)sc->dtmin_bits);
+    dt = dt * sc->cfl;
+    const double dtfinal = sc->tmax - t;
+    if (dt > dtfinal) dt = dtfinal;
+    sc->dt = dt;
+    sc->qx = dt / g.dx;
+    sc->qy = dt / g.dy;
+    sc->dtmin_bits = (unsigned long long)__double_as_longlong(1.0e30);
+    sc->detected_step = 0;
+    sc->apriori_step = 0;
+    sc->status = 0;
+}
 
-const KernelTable table = {launch_bc,          launch_flux_all,  launch_update_detect, launch_mood_faces,
-                           launch_combine,     launch_cfl,       launch_dt_finalize,   launch_advance_t,
-                           launch_mood_loop,   launch_lincomb,   launch_gate_repair};
+void launch_step_begin(const GridGeom& g, DevScalars* sc, double t, cudaStream_t s) {
+    k_step_begin<<<1, 1, 0, s>>>(g, sc, t);
+}
+
+const KernelTable table = {launch_bc,       launch_flux_all, launch_update_detect, launch_mood_faces,
+                           launch_combine,  launch_combine_bc, launch_cfl,         launch_dt_finalize,
+                           launch_step_begin, launch_mood_loop, launch_lincomb,    launch_gate_repair};
 
 }  // namespace GPM_NS
 
