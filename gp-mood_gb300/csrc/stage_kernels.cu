@@ -734,22 +734,80 @@ __device__ __forceinline__ void cascade_order(int8_t* o) {
     *o = (int8_t)(v == 3 ? 1 : (v > 3 ? 3 : v));
 }
 
+// Uout of every cell and DETECTION on it (mood_troubled's decision).  The
+// cells whose new density breaks the DMP bound (mood_uout_part 2) need up to
+// ~150 more FP64 instructions; run by the threads that found them they cost
+// their whole warp that much (34.6 us of a 256^2 2DRP3 stage), so a CTA lists
+// them in shared memory and runs the remaining tests on full warps: both
+// halves of the shock detector at once on different warps, then both U2 tests
+// of the cells that it left.
+struct DetectSmem {
+    int n[2];               // cells in each list
+    short list[2][256];     // candidates; those left by the shock detector
+    bool hit[2][256];       // shock_flow, shock_grad; U2 smooth in x, in y
+    bool troubled[256];
+};
+
 __global__ void __launch_bounds__(256) k_update_detect(StageArgs a, const __grid_constant__ GpWeights w, int cur) {
+    __shared__ DetectSmem sm;
     const GridGeom& g = a.g;
+    const int tid = threadIdx.y * 32 + threadIdx.x;
     const int l = 1 + blockIdx.x * 32 + threadIdx.x, n = 1 + blockIdx.y * 8 + threadIdx.y;
-    if (l > g.lf || n > g.nf) return;
+    const bool in = l <= g.lf && n <= g.nf;
+    const bool mood = g.method == 2 || g.method == 203;
     const size_t c = cidx(g, l, n);
-    const double qx = a.sc->qx, qy = a.sc->qy;
-    const Cell uo = cell_update(g, a.uin, a.fx, a.fy, c, qx, qy);
-    st_cell(a.uout + 4 * c, uo);
-    bool trb = false;
-    if (g.method == 2 || g.method == 203) {
-        const int o = a.uniform_order ? g.mord : (int)a.order[c];
-        if (o > 1) trb = mood_troubled(uo, a.uin + 4 * c, g.nx, g, w.d2x, w.d2y);
-        else if (inadmissible(uo)) atomicOr(&a.sc->status, GPM_STATUS_NAN);
+    if (tid < 2) sm.n[tid] = 0;
+    int part = 0;
+    if (in) {
+        const Cell uo = cell_update(g, a.uin, a.fx, a.fy, c, a.sc->qx, a.sc->qy);
+        st_cell(a.uout + 4 * c, uo);
+        if (mood) {
+            const int o = a.uniform_order ? g.mord : (int)a.order[c];
+            if (o > 1) part = mood_uout_part(uo, a.uin + 4 * c, g.nx, g);
+            else if (inadmissible(uo)) atomicOr(&a.sc->status, GPM_STATUS_NAN);
+        }
     }
-    if (a.uniform_order) a.order[c] = (int8_t)(!trb ? g.mord : g.mord == 3 ? 1 : 3);  // CellGPO = mord, :48, lowered
-    else if (trb) cascade_order(&a.order[c]);
+    bool trb = part == 1;
+    if (mood && __syncthreads_or(part == 2)) {  // most CTAs have none and leave with this one barrier
+        sm.troubled[tid] = false;
+        if (part == 2) sm.list[0][atomicAdd(&sm.n[0], 1)] = (short)tid;
+        __syncthreads();
+        // two tests at a time on the listed cells, one per warp: test t of chunk i is warp task 2*i + t
+        const int warp = tid >> 5, lane = tid & 31;
+#pragma unroll 1
+        for (int round = 0; round < 2; round++) {
+            const int m = sm.n[round];
+            for (int task = warp; task < 2 * ((m + 31) / 32); task += 8) {
+                const int t = task & 1, j = (task >> 1) * 32 + lane;
+                if (j < m) {
+                    const int i = sm.list[round][j];
+                    const double* u = a.uin + 4 * cidx(g, 1 + blockIdx.x * 32 + (i & 31), 1 + blockIdx.y * 8 + (i >> 5));
+                    if (round == 0)
+                        sm.hit[t][j] = t == 0 ? mood_shock_flow_part(u, g.nx, g) : mood_shock_grad_part(u, g.nx, g);
+                    else
+                        sm.hit[t][j] = t == 0 ? mood_u2_smooth<0>(u, g.nx, g, w.d2x) : mood_u2_smooth<1>(u, g.nx, g, w.d2y);
+                }
+            }
+            __syncthreads();
+            if (tid < m) {
+                const int i = sm.list[round][tid];
+                if (round == 0) {
+                    if (sm.hit[0][tid] && sm.hit[1][tid]) {
+                        if (g.u2) sm.list[1][atomicAdd(&sm.n[1], 1)] = (short)i;
+                        else sm.troubled[i] = true;
+                    }
+                } else {
+                    sm.troubled[i] = !(sm.hit[0][tid] || sm.hit[1][tid]);
+                }
+            }
+            __syncthreads();
+        }
+        trb = trb || sm.troubled[tid];
+    }
+    if (in) {
+        if (a.uniform_order) a.order[c] = (int8_t)(!trb ? g.mord : g.mord == 3 ? 1 : 3);  // CellGPO = mord, :48, lowered
+        else if (trb) cascade_order(&a.order[c]);
+    }
     list_append(trb, a.tlist[cur], &a.sc->ntrb[cur], (int)c);
 }
 
