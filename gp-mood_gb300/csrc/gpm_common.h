@@ -102,15 +102,18 @@ struct GridGeom {
     int u2_fd;           // POL_MOOD: the U2 test's second derivatives are the 3-point differences
                          // D2O2/dx^2 (mod_subroutine_MOOD.f90:81-84) instead of the GP weights
     int num_flux;        // 100 HLLC, 101 LLF, 102 HLL, 103 unsplit
-    int mood_solo;       // device MOOD loop: lists of at most this many cells run in one CTA
+    int mood_solo;       // device MOOD loop: lists of at most this many cells run on one cluster
     int flux_tma;        // fast first pass: halo tiles staged by a TMA bulk tensor copy (1) or loads (0)
-    int solo_split;      // one-CTA MOOD passes: DETECTION split over warp roles (1) or per cell (0)
+    int solo_split;      // one-cluster MOOD passes: DETECTION split over warps (1) or on one thread per cell (0)
     int cc_col;          // NN_GP_MOOD_CC: the column l whose order-3 states are blended (-1: none)
 };
 
-// Default of GridGeom::mood_solo; the environment variable GPMOOD_MOOD_SOLO
-// overrides it (tuning only: results do not depend on it).
-int gpm_mood_solo_default();
+// Longest troubled lists that one cluster (k_mood_loop) and one CTA (batched
+// loop) take over from all SMs; the environment variable
+// GPMOOD_MOOD_SOLO overrides both (tuning only: results do not depend on it).
+#define GPM_MOOD_TEAM_MAX 100
+#define GPM_MOOD_CTA_MAX 12
+int gpm_mood_solo_default(int otherwise);
 
 // Default of GridGeom::flux_tma (1); the environment variable GPMOOD_FLUX_TMA=0
 // selects the plain-load staging (A/B timing only: the staged tile, and so

@@ -73,12 +73,12 @@ extern "C" void gpm_pol_weights(GpWeights* w);
 int gpm_fast_rcp_dev(const double* x, double* y, int n);
 int gpm_fast_sqrt_dev(const double* x, double* y, int n);
 
-int gpm_mood_solo_default() {
+int gpm_mood_solo_default(int otherwise) {
     static const int v = [] {
         const char* e = getenv("GPMOOD_MOOD_SOLO");
-        return e && *e ? atoi(e) : 12;
+        return e && *e ? atoi(e) : -1;
     }();
-    return v;
+    return v >= 0 ? v : otherwise;
 }
 
 int gpm_flux_tma_default() {
@@ -518,7 +518,7 @@ int gpmood_create(const gpmood_params* p, gpmood_ctx** out) {
     c->g.mord = c->p.mord;
     c->g.method = c->p.method;
     c->g.num_flux = p->num_flux;
-    c->g.mood_solo = gpm_mood_solo_default();
+    c->g.mood_solo = gpm_mood_solo_default(GPM_MOOD_TEAM_MAX);
     c->g.flux_tma = gpm_flux_tma_default();
     c->g.solo_split = gpm_solo_split_default();
     c->g.cc_col = -1;

@@ -269,7 +269,7 @@ extern "C" int gpmood_time_stepping_noalloc(const gpmood_params* p, double* d_ui
     g.dmp = p->dmp;
     g.u2 = p->u2;
     g.u2_tol = p->u2_tol;
-    g.mood_solo = gpm_mood_solo_default();
+    g.mood_solo = gpm_mood_solo_default(GPM_MOOD_TEAM_MAX);
     g.flux_tma = gpm_flux_tma_default();
     g.solo_split = gpm_solo_split_default();
     g.cc_col = -1;

@@ -38,6 +38,8 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <cooperative_groups.h>
+
 #include <mutex>
 
 #if GPM_EXACT
@@ -1064,13 +1066,11 @@ __device__ __forceinline__ bool grid_sync(GridBar* b) {
     return *(volatile int*)&b->err == 0;
 }
 
-// Passes whose troubled list holds at most GridGeom::mood_solo cells run in CTA 0
-// alone, with CTA barriers: such a pass is a few dependent chains of FP64
-// work, and two grid barriers cost more than its work.  Every CTA reads the
-// same count after a grid barrier, so all take the switch at the same pass;
-// the others leave and CTA 0 runs the loop to its end (a list that grows
-// again is still done, by one CTA's threads).  Runs whose cascade crawls
-// cell by cell need hundreds of such passes per stage.
+// One-CTA passes of the batched loop: a pass with at most BatchArgs::mood_solo
+// cells runs in CTA 0 alone with CTA barriers.  Every CTA reads the same count
+// after a grid barrier, so all take the switch at the same pass; the others
+// leave and CTA 0 runs the loop to its end (a list that grows again is still
+// done, by one CTA's threads).
 __device__ __forceinline__ bool mood_sync(GridBar* b, bool solo) {
     if (solo) {
         __syncthreads();
@@ -1079,201 +1079,321 @@ __device__ __forceinline__ bool mood_sync(GridBar* b, bool solo) {
     return grid_sync(b);
 }
 
-// The cross phase of a pass run by one CTA (solo).  A lone warp pays ~64
-// cycles for every FP64 instruction, so one cross cell's DETECTION chain
-// (update, positivity, DMP bounds, shock detector, U2 in x and in y) is what
-// a short pass waits on.  Its parts are split over five warp roles that run
-// at once on every cross cell of a chunk: role 0 updates Uout and runs the
-// Uout tests (mood_uout_part), roles 1-4 the Uin-only tests -- the shock
-// detector's flow half, the two U2 tests and the shock detector's
-// pressure-jump half; after a CTA barrier role 0 combines them, lowers the
-// order of a troubled cell and lists it.  The decision is mood_troubled's.
-// Warp w takes role w % 5; 16 warps give every role at least 3 warps.
-constexpr int SOLO_ROLES = 5;
-constexpr int SOLO_CHUNK = (MOOD_THREADS / 32 / SOLO_ROLES) * 32;  // cross cells per chunk (96)
-// One-CTA passes keep the troubled lists in shared memory (every entry is also
-// written to the global list, which a list longer than this is read from):
-// reading a list entry and appending one then costs the SM's shared-memory
-// latency instead of an L2 round trip or a global atomic.
-constexpr int SOLO_LIST_CAP = 2048;
+// Short passes on one thread-block cluster (the "team").  A pass with at most
+// GridGeom::mood_solo cells is a few chains of dependent FP64 instructions, each
+// ~64 cycles for a lone warp however few of its lanes are active; the grid
+// barrier of the all-SM passes (~3.5 us, twice) costs more than the work, and
+// one SM's four partitions make more than ~4 warps of it queue.  The first
+// cluster's TEAM CTAs run such passes: a cluster barrier is ~470 cycles, and 8
+// SMs take 32 warps side by side.  The chains are cut over the lanes:
+//  * a face's Gauss point takes two lanes, one per side: each reconstructs its
+//    side's state and its primitive quantities; they swap them by shuffles,
+//    both run the Riemann join, and the face's lanes sum the quadrature, one
+//    variable a lane (~70 instructions in a row for ~112 on one lane);
+//  * the tests of the crosses that read only Uin (the shock detector's halves,
+//    U2 in x and in y) run beside the faces on warps of their own, so that
+//    after the barrier only the update, positivity and the density bounds are
+//    left for CTA 0, one lane a cross cell.
+// CTA 0 keeps the troubled lists in shared memory (every entry is also written
+// to the global list, which a longer one is read from); the others read them,
+// and write the tests' results, through distributed shared memory.
+// DMR 512x128, 30 steps: 12.6 -> 7 us a pass of this kind.
+constexpr int TEAM = 8;                  // CTAs of the cluster
+constexpr int TEAM_CROSS = 512;          // cross cells whose tests run beside the faces (one per thread of CTA 0)
+constexpr int TEAM_LIST_CAP = 2048;
 
-struct SoloCross {
-    int cell[SOLO_CHUNK];
-    int8_t part[SOLO_CHUNK];      // mood_uout_part; -1: ghost cell or already updated in this pass
-    int8_t ord[SOLO_CHUNK];       // the cell's order when it was checked
-    bool flag[4][SOLO_CHUNK];     // shock flow half, U2 smooth in x, U2 smooth in y, shock pressure-jump half
-};
-
-struct SoloLists {
-    int list[2][SOLO_LIST_CAP];
+struct TeamSmem {
+    int list[2][TEAM_LIST_CAP];
     int count[2];
+    bool flag[4][TEAM_CROSS];            // shock flow half, pressure-jump half, U2 smooth in x, in y
+    double z3[4][GPM_MAXGP][5];          // order-3 weights, read by lanes of mixed faces and Gauss points
+    double z1[4][GPM_MAXGP];             // order 1
 };
 
-// lst: the current troubled list (shared or global), nt entries.  A cross
-// cell that several listed cells share is updated once: in a pass that fits
-// one chunk by the first listed cell whose cross holds it (a scan of the
-// shared list), otherwise by whoever stamps it first (global atomics).
-__device__ __forceinline__ void solo_cross(const StageArgs& a, const GpWeights& w, int cur, int nt, unsigned pid,
-                                           const int* lst, SoloCross& sm, SoloLists& sl) {
+__device__ __forceinline__ void team_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Warp task `task` of the 4*nt faces of the listed cells.
+template <int NGP>
+__device__ __forceinline__ void team_faces(const StageArgs& a, const GpWeights& w, const TeamSmem& sm, const int* lst,
+                                           int nt, int task) {
+    constexpr int LPF = 2 * NGP, FPW = 32 / LPF;  // lanes per face, faces per warp
     const GridGeom& g = a.g;
-    const double qx = a.sc->qx, qy = a.sc->qy;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int role = warp % SOLO_ROLES, j = (warp / SOLO_ROLES) * 32 + lane;  // item of the chunk
-    const bool slot = j < SOLO_CHUNK;  // a role's fourth warp (warp 15) has no items
-    const int nxt = cur ^ 1, total = 5 * nt;
-    const bool scan = total <= SOLO_CHUNK && nt <= SOLO_LIST_CAP;  // one chunk, list in shared memory
-    const int nx = g.nx;
-    for (int base = 0; base < total; base += SOLO_CHUNK) {
-        const int i = base + j;
-        if (slot && i < total) {
-            const int q = i / 5;
-            const size_t t = (size_t)lst[q];
-            const int k = i % 5;
-            const size_t c = k == 0 ? t - nx : k == 1 ? t - 1 : k == 2 ? t : k == 3 ? t + 1 : t + nx;
-            const int l = (int)(c % (size_t)nx) - 3, n = (int)(c / (size_t)nx) - 3;
-            const bool interior = l >= 1 && l <= g.lf && n >= 1 && n <= g.nf;
-            const double* uin = a.uin + 4 * c;
-            if (role == 0) {
-                bool own = interior;
-                if (own && scan) {
-                    for (int q2 = 0; q2 < q; q2++) {
-                        const long long d = (long long)c - (long long)lst[q2];
-                        if (d == 0 || d == 1 || d == -1 || d == nx || d == -nx) own = false;
-                    }
-                } else if (own) {
-                    own = atomicExch(&a.stamp[c], pid) != pid;
-                }
-                int r = -1, o = 0;
-                if (own) {
-                    const Cell uo = cell_update(g, a.uin, a.fx, a.fy, c, qx, qy);
-                    st_cell(a.uout + 4 * c, uo);
-                    o = a.order[c];
-                    if (o > 1) {
-                        r = mood_uout_part(uo, uin, nx, g);
-                    } else {
-                        if (inadmissible(uo)) atomicOr(&a.sc->status, GPM_STATUS_NAN);
-                        r = 0;
-                    }
-                }
-                sm.cell[j] = (int)c;
-                sm.part[j] = (int8_t)r;
-                sm.ord[j] = (int8_t)o;
-            } else if (interior) {
-                sm.flag[role - 1][j] = role == 1   ? mood_shock_flow_part(uin, nx, g)
-                                       : role == 2 ? mood_u2_smooth<0>(uin, nx, g, w.d2x)
-                                       : role == 3 ? mood_u2_smooth<1>(uin, nx, g, w.d2y)
-                                                   : mood_shock_grad_part(uin, nx, g);
-            }
+    const int lane = threadIdx.x & 31, fl = lane / LPF, j = lane - fl * LPF, gp = j >> 1, side = j & 1;
+    const int base = lane - j, i = task * FPW + fl;
+    const bool act = fl < FPW && i < 4 * nt;
+    int dir = 0, sd = 0, lcell = 0;
+    if (act) lcell = lst[face_item(i, nt, &dir, &sd)];
+    const size_t step = dir == 0 ? (size_t)1 : (size_t)g.nx;
+    const size_t c0 = act ? (size_t)lcell - (sd == 0 ? step : 0) : cidx(g, 1, 1);  // idle lanes: any valid face
+    const size_t cs = c0 + (side ? step : 0);                                     // this lane's cell
+    const int face = dir == 0 ? (side ? 0 : 2) : (side ? 3 : 1);
+    const int o = min((int)__ldcg(a.order + c0), (int)__ldcg(a.order + c0 + step));
+    const ptrdiff_t row = g.nx;
+    double u[4];
+    if (o >= 5) {  // not reached by listed cells; keeps the function total
+        Cell q[13];
+#pragma unroll
+        for (int m = 0; m < 13; m++) q[m] = ld_cell(a.uin + 4 * (cs + st_ox(m) + row * st_oy(m)));
+        gp_recon_at<13>(&w.zt[2][face][gp][0], q, u);
+    } else {
+        Cell q[5];
+#pragma unroll
+        for (int m = 0; m < 5; m++) q[m] = ld_cell(a.uin + 4 * (cs + st_ox(m) + row * st_oy(m)));
+        if (o >= 3) gp_recon_at<5>(&sm.z3[face][gp][0], q, u);
+        else gp_recon_at<1>(&sm.z1[face][gp], q, u);
+        if (a.ccw) {
+            double v1, v2;
+            cc_weights(g, a.ccw, (int)(cs % (size_t)g.nx) - 3, (int)(cs / (size_t)g.nx) - 3, &v1, &v2);
+            if (o >= 3) cc_blend<5>(v1, v2, q[0], u);
+            else cc_blend<1>(v1, v2, q[0], u);
         }
-        __syncthreads();
-        if (role == 0) {
-            bool trb = false;
-            int cval = 0;
-            if (slot && i < total && sm.part[j] >= 0) {
-                const int r = sm.part[j];
-                cval = sm.cell[j];
-                const bool shock = sm.flag[0][j] && sm.flag[3][j];
-                trb = r == 1 || (r == 2 && shock && !(g.u2 && (sm.flag[1][j] || sm.flag[2][j])));
-            }
-            if (trb) {  // the cascade of cascade_order, on the order read above
-                const int v = sm.ord[j];
-                a.order[cval] = (int8_t)(v == 3 ? 1 : (v > 3 ? 3 : v));
-            }
-            // warp-aggregated append to the next list, shared and global
-            const unsigned m = __ballot_sync(0xffffffffu, trb);
-            if (m) {
-                int b0 = 0;
-                if (lane == 0) b0 = atomicAdd(&sl.count[nxt], __popc(m));
-                b0 = __shfl_sync(0xffffffffu, b0, 0);
-                if (trb) {
-                    const int idx = b0 + __popc(m & ((1u << lane) - 1));
-                    a.tlist[nxt][idx] = cval;
-                    if (idx < SOLO_LIST_CAP) sl.list[nxt][idx] = cval;
-                }
-            }
-        }
-        __syncthreads();
     }
+    auto swap = [](double x) { return __shfl_xor_sync(0xffffffffu, x, 1); };  // the other side's lane
+    double F[4];
+    if (g.num_flux == 100) {
+#if GPM_EXACT
+        const Prim mine = c2p_dyn(u, dir);
+        Prim other;
+        other.vn = swap(mine.vn);
+        other.vt = swap(mine.vt);
+        other.p = swap(mine.p);
+        other.c = swap(mine.c);
+        other.vx = swap(mine.vx);
+        other.adm = __shfl_xor_sync(0xffffffffu, (int)mine.adm, 1) != 0;
+        double uo[4], ul[4], ur[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            uo[k] = swap(u[k]);
+            ul[k] = side ? uo[k] : u[k];
+            ur[k] = side ? u[k] : uo[k];
+        }
+        hllc_join(ul, ur, side ? other : mine, side ? mine : other, dir, F);
+#else
+        const Side mine = hllc_side(u[0], dir ? u[2] : u[1], dir ? u[1] : u[2], u[3]);
+        const Side other{swap(mine.r), swap(mine.n), swap(mine.t), swap(mine.e),
+                         swap(mine.v), swap(mine.w), swap(mine.p), swap(mine.c)};
+        NormalFlux f;
+        hllc_join(side ? other : mine, side ? mine : other, f);
+        F[0] = f.r;
+        F[1] = dir ? f.t : f.n;
+        F[2] = dir ? f.n : f.t;
+        F[3] = f.e;
+        nan_flux(!(side_ok(mine) && side_ok(other)), F);
+#endif
+    } else {
+        double ul[4], ur[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const double x = swap(u[k]);
+            ul[k] = side ? x : u[k];
+            ur[k] = side ? u[k] : x;
+        }
+        if (dir == 0) riemann<0>(g.num_flux, ul, ur, F);
+        else riemann<1>(g.num_flux, ul, ur, F);
+    }
+    // quadrature (quad_flux's expression): variable k on lane k of the face; two rounds of two with one Gauss point
+#pragma unroll
+    for (int k0 = 0; k0 < 4; k0 += (LPF < 4 ? LPF : 4)) {
+        double acc = 0.;
+#pragma unroll
+        for (int gg = 0; gg < NGP; gg++) {
+            double x = 0.;
+#pragma unroll
+            for (int k = 0; k < (LPF < 4 ? LPF : 4); k++) {
+                const double y = __shfl_sync(0xffffffffu, F[k0 + k], min(base + 2 * gg, 31));
+                if (j == k) x = y;
+            }
+            acc = gg == 0 ? x * w.gw[0] : acc + x * w.gw[gg];
+        }
+#if GPM_EXACT
+        acc = plus_zero(acc);
+#endif
+        if (act && j < (LPF < 4 ? LPF : 4)) __stcg((dir == 0 ? a.fx : a.fy) + 4 * c0 + k0 + j, acc);
+    }
+}
+
+// Cross cell k of listed cell t; false outside the interior.
+__device__ __forceinline__ bool cross_cell(const GridGeom& g, int t, int k, int* c) {
+    *c = k == 0 ? t - g.nx : k == 1 ? t - 1 : k == 2 ? t : k == 3 ? t + 1 : t + g.nx;
+    const int n = *c / g.nx - 3, l = *c - (n + 3) * g.nx - 3;
+    return l >= 1 && l <= g.lf && n >= 1 && n <= g.nf;
+}
+
+// The update and the decision on the crosses, by CTA 0: the last half of
+// mood_troubled.  A cross cell that several listed cells share is taken by the
+// first of them (a scan of a short list), or by whoever stamps it first.
+__device__ __forceinline__ void team_cells(const StageArgs& a, const GpWeights& w, TeamSmem& sm, const int* lst,
+                                           int cur, int nt, unsigned pid, double qx, double qy) {
+    const GridGeom& g = a.g;
+    const int nxt = cur ^ 1, total = 5 * nt, lane = threadIdx.x & 31, nx = g.nx;
+    for (int i0 = (int)threadIdx.x - lane; i0 < total; i0 += MOOD_THREADS) {
+        const int i = i0 + lane, q = i / 5;
+        bool trb = false;
+        int c = 0;
+        if (i < total && cross_cell(g, lst[q], i - 5 * q, &c)) {
+            bool own = true;
+            if (nt <= 24) {
+                for (int q2 = 0; q2 < q; q2++) {
+                    const int d = c - lst[q2];
+                    if (d == 0 || d == 1 || d == -1 || d == nx || d == -nx) own = false;
+                }
+            } else {
+                own = atomicExch(&a.stamp[c], pid) != pid;
+            }
+            if (own) {
+                const double* uin = a.uin + 4 * (size_t)c;
+                const Cell uo = cell_update(g, a.uin, a.fx, a.fy, (size_t)c, qx, qy);
+                st_cell(a.uout + 4 * (size_t)c, uo);
+                const int o = (int)__ldcg(a.order + c);
+                if (o > 1) {
+                    const int r = mood_uout_part(uo, uin, nx, g);
+                    trb = r == 1;
+                    if (r == 2) {
+                        if (g.solo_split && i < TEAM_CROSS) {
+                            trb = sm.flag[0][i] && sm.flag[1][i] && !(g.u2 && (sm.flag[2][i] || sm.flag[3][i]));
+                        } else {
+                            trb = mood_shock_part(uin, nx, g) && !(g.u2 && (mood_u2_smooth<0>(uin, nx, g, w.d2x) ||
+                                                                            mood_u2_smooth<1>(uin, nx, g, w.d2y)));
+                        }
+                    }
+                    if (trb) __stcg(a.order + c, (int8_t)(o == 3 ? 1 : 3));  // the cascade of cascade_order
+                } else if (inadmissible(uo)) {
+                    atomicOr(&a.sc->status, GPM_STATUS_NAN);
+                }
+            }
+        }
+        // warp-aggregated append to the next list, shared and global
+        const unsigned m = __ballot_sync(0xffffffffu, trb);
+        if (m) {
+            int b0 = 0;
+            if (lane == 0) b0 = atomicAdd(&sm.count[nxt], __popc(m));
+            b0 = __shfl_sync(0xffffffffu, b0, 0);
+            if (trb) {
+                const int idx = b0 + __popc(m & ((1u << lane) - 1));
+                __stcg(a.tlist[nxt] + idx, c);
+                if (idx < TEAM_LIST_CAP) sm.list[nxt][idx] = c;
+            }
+        }
+    }
+}
+
+// Passes pass+1, ... on the first cluster until the list is empty; returns the
+// pass count.  sm0: CTA 0's shared memory, seen from this CTA.
+template <int NGP>
+__device__ __forceinline__ int team_loop(const StageArgs& a, const GpWeights& w, TeamSmem& sm, TeamSmem* sm0, int cur,
+                                         int nt, int pass, int max_pass, unsigned epoch, double qx, double qy) {
+    const int rank = (int)blockIdx.x, tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    constexpr int FPW = 32 / (2 * NGP);
+    for (int i = tid; i < 4 * NGP * 5; i += MOOD_THREADS) {
+        const int f = i / (5 * NGP), gp = (i / 5) % NGP, m = i % 5;
+        sm.z3[f][gp][m] = w.zt[1][f][gp][m];
+        if (m == 0) sm.z1[f][gp] = w.zt[0][f][gp][0];
+    }
+    if (rank == 0) {
+        for (int i = tid; i < nt && i < TEAM_LIST_CAP; i += MOOD_THREADS) sm.list[cur][i] = __ldcg(a.tlist[cur] + i);
+        if (tid == 0) sm.count[cur] = nt;
+    }
+    team_sync();
+    for (;;) {
+        nt = *(volatile int*)&sm0->count[cur];
+        if (nt == 0) break;
+        if (pass >= max_pass) {
+            if (rank == 0 && tid == 0) a.sc->status |= GPM_STATUS_MOODCAP;
+            break;
+        }
+        pass++;
+        if (rank == 0 && tid == 0) {
+            sm.count[cur ^ 1] = 0;  // read last before the two barriers of the pass before
+            a.sc->detected_step += (unsigned long long)nt;
+        }
+        const int* lst = nt <= TEAM_LIST_CAP ? sm0->list[cur] : a.tlist[cur];
+        const int nface = (4 * nt + FPW - 1) / FPW, ncross = a.g.solo_split ? min(5 * nt, TEAM_CROSS) : 0;
+        const int chunks = (ncross + 31) / 32;
+        for (int task = warp * TEAM + rank; task < nface + 4 * chunks; task += (MOOD_THREADS / 32) * TEAM) {
+            if (task < nface) {
+                team_faces<NGP>(a, w, sm, lst, nt, task);
+            } else {
+                const int t = (task - nface) & 3, i = ((task - nface) >> 2) * 32 + lane;
+                int c;
+                if (i < ncross && cross_cell(a.g, lst[i / 5], i % 5, &c)) {
+                    const double* u = a.uin + 4 * (size_t)c;
+                    sm0->flag[t][i] = t == 0   ? mood_shock_flow_part(u, a.g.nx, a.g)
+                                      : t == 1 ? mood_shock_grad_part(u, a.g.nx, a.g)
+                                      : t == 2 ? mood_u2_smooth<0>(u, a.g.nx, a.g, w.d2x)
+                                               : mood_u2_smooth<1>(u, a.g.nx, a.g, w.d2y);
+                }
+            }
+        }
+        team_sync();
+        if (rank == 0) team_cells(a, w, sm, lst, cur, nt, epoch + (unsigned)pass, qx, qy);
+        team_sync();
+        cur ^= 1;
+    }
+    team_sync();  // CTA 0's shared memory stays until everyone has left it
+    return pass;
 }
 
 template <int NGP>
 __global__ void __launch_bounds__(MOOD_THREADS, 1) k_mood_loop(StageArgs a, const __grid_constant__ GpWeights w, GridBar* bar,
                                                       int max_pass, int stage) {
-    __shared__ SoloCross solo_sm;
-    __shared__ SoloLists solo_ls;
+    __shared__ TeamSmem team_sm;
     const GridGeom& g = a.g;
     const double qx = a.sc->qx, qy = a.sc->qy;
     const unsigned epoch = a.sc->stamp_epoch;  // stamps epoch+2, epoch+3, ... are new
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gstride = gridDim.x * blockDim.x;
-    int stid = pack_tid(), wstride = gstride;  // whole warps of work items, dealt over all SMs
-    bool solo = false, shared_lists = false;  // shared_lists: a one-CTA loop with role-split DETECTION
+    const int stid = pack_tid();  // whole warps of work items, dealt over all SMs
     int cur = 0, pass = 1;  // pass 1 (all faces) ran before this kernel
     for (;;) {
-        const int nt = shared_lists ? solo_ls.count[cur] : *(volatile int*)&a.sc->ntrb[cur];
+        const int nt = *(volatile int*)&a.sc->ntrb[cur];
         if (nt == 0) break;
+        if (nt <= g.mood_solo) {
+            if (blockIdx.x >= TEAM) return;
+            TeamSmem* sm0 = cooperative_groups::this_cluster().map_shared_rank(&team_sm, 0);
+            pass = team_loop<NGP>(a, w, team_sm, sm0, cur, nt, pass, max_pass, epoch, qx, qy);
+            break;
+        }
         if (pass >= max_pass) {
             if (gtid == 0) a.sc->status |= GPM_STATUS_MOODCAP;
             break;
-        }
-        if (!solo && nt <= g.mood_solo) {
-            if (blockIdx.x != 0) return;
-            solo = true;
-            stid = threadIdx.x;
-            wstride = blockDim.x;
-            if (g.solo_split) {  // from here on the lists also live in shared memory
-                shared_lists = true;
-                for (int i = threadIdx.x; i < nt && i < SOLO_LIST_CAP; i += blockDim.x)
-                    solo_ls.list[cur][i] = a.tlist[cur][i];
-                if (threadIdx.x == 0) solo_ls.count[cur] = nt;
-                __syncthreads();
-            }
         }
         pass++;
         // the listed cells' orders were lowered when they were listed
         if (gtid == 0) {
             a.sc->ntrb[cur ^ 1] = 0;  // nobody appends to it before the next barrier
             a.sc->detected_step += (unsigned long long)nt;
-            if (shared_lists) solo_ls.count[cur ^ 1] = 0;
         }
-        const int* lst = shared_lists && nt <= SOLO_LIST_CAP ? solo_ls.list[cur] : a.tlist[cur];
         // the four faces of every troubled cell at the new orders
         // x and y faces share warps (face_gp_dyn): 4*nt items packed densely
-        face_phase_gp<NGP>(4 * nt, 4 * nt, stid, wstride, [&](int i, int gp, FaceGp& f) {
+        face_phase_gp<NGP>(4 * nt, 4 * nt, stid, gstride, [&](int i, int gp, FaceGp& f) {
             int dir, side;
-            const size_t c = (size_t)lst[face_item(i, nt, &dir, &side)];
+            const size_t c = (size_t)a.tlist[cur][face_item(i, nt, &dir, &side)];
             face_gp_dyn(a, w, side == 0 ? (dir == 0 ? c - 1 : c - g.nx) : c, dir, gp, f);
         });
-        if (!mood_sync(bar, solo)) return;
+        if (!grid_sync(bar)) return;
         // the 5-point crosses: Uout from Uin and the current fluxes, DETECTION
         const unsigned pid = epoch + (unsigned)pass;
-        if (shared_lists) {
-            solo_cross(a, w, cur, nt, pid, lst, solo_sm, solo_ls);
-            cur ^= 1;
-            continue;
-        }
         const int nxt = cur ^ 1, total = 5 * nt;
-        const int lim = ((total + wstride - 1) / wstride) * wstride;
-        for (int base = 0; base < lim; base += wstride) {
+        const int lim = ((total + gstride - 1) / gstride) * gstride;
+        for (int base = 0; base < lim; base += gstride) {
             const int i = base + stid;
             bool trb = false;
             int cval = 0;
             if (i < total) {
-                const size_t t = (size_t)a.tlist[cur][i / 5];
-                const int k = i % 5;
-                const size_t c = k == 0 ? t - g.nx : k == 1 ? t - 1 : k == 2 ? t : k == 3 ? t + 1 : t + g.nx;
-                const int l = (int)(c % (size_t)g.nx) - 3, n = (int)(c / (size_t)g.nx) - 3;
-                if (l >= 1 && l <= g.lf && n >= 1 && n <= g.nf && atomicExch(&a.stamp[c], pid) != pid) {
-                    const Cell uo = cell_update(g, a.uin, a.fx, a.fy, c, qx, qy);
-                    st_cell(a.uout + 4 * c, uo);
-                    if (a.order[c] > 1) trb = mood_troubled(uo, a.uin + 4 * c, g.nx, g, w.d2x, w.d2y);
+                int c;
+                if (cross_cell(g, a.tlist[cur][i / 5], i % 5, &c) && atomicExch(&a.stamp[c], pid) != pid) {
+                    const Cell uo = cell_update(g, a.uin, a.fx, a.fy, (size_t)c, qx, qy);
+                    st_cell(a.uout + 4 * (size_t)c, uo);
+                    if (a.order[c] > 1) trb = mood_troubled(uo, a.uin + 4 * (size_t)c, g.nx, g, w.d2x, w.d2y);
                     else if (inadmissible(uo)) atomicOr(&a.sc->status, GPM_STATUS_NAN);
-                    cval = (int)c;
+                    cval = c;
                 }
             }
             if (trb) cascade_order(&a.order[cval]);
             list_append(trb, a.tlist[nxt], &a.sc->ntrb[nxt], cval);
         }
-        if (!mood_sync(bar, solo)) return;
+        if (!grid_sync(bar)) return;
         cur ^= 1;
     }
     if (gtid == 0) {  // every CTA read the epoch before the first barrier
@@ -1289,19 +1409,27 @@ static int launch_mood_loop_n(const StageArgs& a, const GpWeights& w, GridBar* b
     static std::atomic<int> grids[GPM_MAX_DEVICES];
     const int dev = gpm_device();
     int grid = grids[dev].load(std::memory_order_relaxed);
-    if (!grid) {
-        int sms = 0, occ = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_mood_loop<NGP>, MOOD_THREADS, 0);
-        grid = sms * (occ > 0 ? occ : 1);
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = TEAM;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeCooperative;
+    at[1].val.cooperative = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(MOOD_THREADS);
+    cfg.stream = s;
+    cfg.attrs = at;
+    if (!grid) {  // every cluster that fits at once: the grid barrier needs all CTAs resident
+        int clusters = 0;
+        cfg.gridDim = dim3(TEAM);
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&clusters, k_mood_loop<NGP>, &cfg) != cudaSuccess || clusters < 1) return -1;
+        grid = clusters * TEAM;
         grids[dev].store(grid, std::memory_order_relaxed);
     }
-    StageArgs aa = a;
-    GpWeights ww = w;
-    void* args[] = {&aa, &ww, &bar, &max_pass, &stage};
-    return cudaLaunchCooperativeKernel((const void*)k_mood_loop<NGP>, dim3(grid), dim3(MOOD_THREADS), args, 0, s) == cudaSuccess
-               ? 0
-               : -1;
+    cfg.gridDim = dim3(grid);
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, k_mood_loop<NGP>, a, w, bar, max_pass, stage) == cudaSuccess ? 0 : -1;
 }
 
 int launch_mood_loop(const StageArgs& a, const GpWeights& w, GridBar* bar, int max_pass, int stage,
