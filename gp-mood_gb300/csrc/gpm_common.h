@@ -145,7 +145,7 @@ enum { GPM_STATUS_NAN = 1, GPM_STATUS_MOODCAP = 2, GPM_STATUS_DT = 4, GPM_STATUS
 
 // Grid barrier state of the cooperative MOOD-loop kernel (zeroed device memory).
 struct GridBar {
-    unsigned count, gen;
+    unsigned long long count;  // arrivals so far, of all launches
     int err;
     int limit;  // polls a waiting CTA makes before it gives up; 0: the default, ~1 s (test hook)
 };
@@ -160,6 +160,7 @@ struct StageArgs {
     int8_t* order;         // CellGPO per padded cell
     unsigned* stamp;       // per-cell pass stamps (dedup of the dirty set)
     int* tlist[2];         // troubled-cell lists (padded linear indices)
+    unsigned char* tests;  // 4 bytes per padded cell: results of the Uin-only DETECTION tests in a MOOD pass
     DevScalars* sc;
     int uniform_order;     // 1: every cell starts at mord (plain GP-MOOD)
     int stage;             // 0, 1, 2 -> t_rk = t, t+dt, t+dt/2

@@ -33,6 +33,7 @@ struct gpmood_ctx {
     int8_t* dOrder;
     unsigned* dStamp;
     int* dList[2];
+    unsigned char* dTests;        // StageArgs::tests
     DevScalars* dSc;
     DevScalars* hSc;              // pinned mirror
     GridBar* dBar;                // barrier of the cooperative MOOD loop, directly behind dSc
@@ -139,6 +140,7 @@ StageArgs stage_args(gpmood_ctx* c, const double* uin, double* uout, int stage, 
     a.stamp = c->dStamp;
     a.tlist[0] = c->dList[0];
     a.tlist[1] = c->dList[1];
+    a.tests = c->dTests;
     a.sc = c->dSc;
     a.uniform_order = uniform ? 1 : 0;
     a.stage = stage;
@@ -438,7 +440,7 @@ void free_all(gpmood_ctx* c) {
     if (!c) return;
     cudaFree(c->dU); cudaFree(c->dUr); cudaFree(c->dU1); cudaFree(c->dU2);
     cudaFree(c->dFx); cudaFree(c->dFy); cudaFree(c->dOrder); cudaFree(c->dStamp);
-    cudaFree(c->dList[0]); cudaFree(c->dList[1]); cudaFree(c->dSc); cudaFree(c->dStageOrd);
+    cudaFree(c->dList[0]); cudaFree(c->dList[1]); cudaFree(c->dTests); cudaFree(c->dSc); cudaFree(c->dStageOrd);
     for (int i = 0; i < 5; i++) cudaFree(c->dRk4[i]);
     if (c->hSc) cudaFreeHost(c->hSc);
     if (c->hCount) cudaFreeHost(c->hCount);
@@ -568,6 +570,7 @@ int gpmood_create(const gpmood_params* p, gpmood_ctx** out) {
     ALLOC(c->dStamp, c->ncell * sizeof(unsigned));
     ALLOC(c->dList[0], c->ncell * sizeof(int));
     ALLOC(c->dList[1], c->ncell * sizeof(int));
+    ALLOC(c->dTests, c->ncell * 4);
     ALLOC(c->dSc, sizeof(DevScalars) + sizeof(GridBar));
     ALLOC(c->dStageOrd, GPM_MAXST * c->ncell);
     if (p->integrator == GPMOOD_SSP_RK4)

@@ -29,8 +29,8 @@
 #include "gpm_common.h"
 
 #define GPM_NOALLOC_MAX_CELLS (264 * 264)
-// Bytes per padded cell: U1, U2, Fx, Fy (4 doubles each), order (1), stamp (4), two lists (4 + 4).
-#define GPM_NOALLOC_CELL_BYTES (4 * 32 + 1 + 4 + 4 + 4)
+// Bytes per padded cell: U1, U2, Fx, Fy (4 doubles each), order (1), stamp (4), two lists (4 + 4), tests (4).
+#define GPM_NOALLOC_CELL_BYTES (4 * 32 + 1 + 4 + 4 + 4 + 4)
 #define GPM_NOALLOC_BYTES ((size_t)GPM_NOALLOC_MAX_CELLS * GPM_NOALLOC_CELL_BYTES + 16 * 256)
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[GPM_NOALLOC_BYTES];
@@ -166,6 +166,7 @@ struct Carve {
     int8_t* order;
     unsigned* stamp;
     int* list[2];
+    unsigned char* tests;
     DevScalars* sc;
     GridBar* bar;
 };
@@ -187,6 +188,7 @@ Carve carve(unsigned char* base, size_t ncell) {
     c.stamp = reinterpret_cast<unsigned*>(take(ncell * 4));
     c.list[0] = reinterpret_cast<int*>(take(ncell * 4));
     c.list[1] = reinterpret_cast<int*>(take(ncell * 4));
+    c.tests = reinterpret_cast<unsigned char*>(take(ncell * 4));
     c.order = reinterpret_cast<int8_t*>(take(ncell));
     return c;
 }
@@ -215,6 +217,7 @@ int stage_noalloc(const KernelTable& kt, const GridGeom& g, const GpWeights& w, 
     a.stamp = s.stamp;
     a.tlist[0] = s.list[0];
     a.tlist[1] = s.list[1];
+    a.tests = s.tests;
     a.sc = s.sc;
     a.uniform_order = 1;
     a.stage = stage;

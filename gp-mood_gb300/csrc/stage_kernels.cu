@@ -1038,30 +1038,42 @@ __global__ void __launch_bounds__(128) k_mood_faces(StageArgs a, const __grid_co
 // keeps the barrier's arrival count at the SM count.
 constexpr int MOOD_THREADS = 512;
 
-__device__ __forceinline__ bool grid_sync(GridBar* b) {
+// Arrivals are counted up and never reset: every launch adds a multiple of the
+// grid's size, and before its first barrier opens a CTA can see at most one
+// grid's worth of arrivals above that, so the count rounded down to a multiple
+// is where the launch began.  One release-add and polls of the same word: two
+// trips to L2 instead of the four of a count, a reset and a generation word
+// (4.8k cycles a barrier at best before).
+struct GridWait {
+    unsigned long long next;  // arrivals that open the next barrier
+};
+
+__device__ __forceinline__ GridWait grid_start(GridBar* b) {
+    unsigned long long c;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(c) : "l"(&b->count) : "memory");
+    return GridWait{(c / gridDim.x + 1) * gridDim.x};
+}
+
+__device__ __forceinline__ bool grid_sync(GridBar* b, GridWait& w) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        volatile unsigned* vgen = &b->gen;
-        const unsigned g = *vgen;
         const int lim = *(volatile int*)&b->limit;
-        const long long max_it = lim > 0 ? lim : (1LL << 24);  // ~1 s: far beyond any pass
+        const long long max_it = lim > 0 ? lim : (1LL << 22);  // ~1 s: far beyond any pass
         __threadfence();
-        if (atomicAdd(&b->count, 1u) == gridDim.x - 1) {
-            atomicExch(&b->count, 0u);
-            __threadfence();
-            atomicAdd(&b->gen, 1u);
-        } else {
-            long long it = 0;
-            while (*vgen == g) {
-                if (++it > max_it) {
-                    atomicExch(&b->err, 1);
-                    break;
-                }
-                __nanosleep(32);
+        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&b->count), "l"(1ull) : "memory");
+        long long it = 0;
+        for (;;) {
+            unsigned long long c;
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(c) : "l"(&b->count) : "memory");
+            if (c >= w.next) break;
+            if (++it > max_it) {
+                atomicExch(&b->err, 1);
+                break;
             }
         }
         __threadfence();
     }
+    w.next += gridDim.x;
     __syncthreads();
     return *(volatile int*)&b->err == 0;
 }
@@ -1071,21 +1083,17 @@ __device__ __forceinline__ bool grid_sync(GridBar* b) {
 // after a grid barrier, so all take the switch at the same pass; the others
 // leave and CTA 0 runs the loop to its end (a list that grows again is still
 // done, by one CTA's threads).
-__device__ __forceinline__ bool mood_sync(GridBar* b, bool solo) {
+__device__ __forceinline__ bool mood_sync(GridBar* b, GridWait& w, bool solo) {
     if (solo) {
         __syncthreads();
         return true;
     }
-    return grid_sync(b);
+    return grid_sync(b, w);
 }
 
-// Short passes on one thread-block cluster (the "team").  A pass with at most
-// GridGeom::mood_solo cells is a few chains of dependent FP64 instructions, each
-// ~64 cycles for a lone warp however few of its lanes are active; the grid
-// barrier of the all-SM passes (~3.5 us, twice) costs more than the work, and
-// one SM's four partitions make more than ~4 warps of it queue.  The first
-// cluster's TEAM CTAs run such passes: a cluster barrier is ~470 cycles, and 8
-// SMs take 32 warps side by side.  The chains are cut over the lanes:
+// A pass of the MOOD loop.  It is a few chains of dependent FP64 instructions,
+// each ~64 cycles for a lone warp however few of its lanes are active, and
+// trips to L2 of ~1k cycles, so the chains are cut over lanes and warps:
 //  * a face's Gauss point takes two lanes, one per side: each reconstructs its
 //    side's state and its primitive quantities; they swap them by shuffles,
 //    both run the Riemann join, and the face's lanes sum the quadrature, one
@@ -1093,18 +1101,21 @@ __device__ __forceinline__ bool mood_sync(GridBar* b, bool solo) {
 //  * the tests of the crosses that read only Uin (the shock detector's halves,
 //    U2 in x and in y) run beside the faces on warps of their own, so that
 //    after the barrier only the update, positivity and the density bounds are
-//    left for CTA 0, one lane a cross cell.
-// CTA 0 keeps the troubled lists in shared memory (every entry is also written
-// to the global list, which a longer one is read from); the others read them,
-// and write the tests' results, through distributed shared memory.
-// DMR 512x128, 30 steps: 12.6 -> 7 us a pass of this kind.
+//    left, one lane a cross cell.
+// Passes over more than GridGeom::mood_solo cells run on all SMs with grid
+// barriers.  Shorter ones run on the first thread-block cluster (the "team")
+// with cluster barriers (~1k cycles with what they wait for, against ~4k):
+// 8 SMs take 32 warps side by side, and CTA 0 runs the cells.  The team's lists
+// live in every member's shared memory (and in the global list, which a longer
+// one is read from), the tests' results in CTA 0's, through distributed shared
+// memory.
 constexpr int TEAM = 8;                  // CTAs of the cluster
 constexpr int TEAM_CROSS = 512;          // cross cells whose tests run beside the faces (one per thread of CTA 0)
-constexpr int TEAM_LIST_CAP = 2048;
+constexpr int TEAM_LIST_CAP = 1024;
 
 struct TeamSmem {
     int list[2][TEAM_LIST_CAP];
-    int count[2];
+    int count[2];                        // the team's count: appended to in CTA 0, then copied to every member
     bool flag[4][TEAM_CROSS];            // shock flow half, pressure-jump half, U2 smooth in x, in y
     double z3[4][GPM_MAXGP][5];          // order-3 weights, read by lanes of mixed faces and Gauss points
     double z1[4][GPM_MAXGP];             // order 1
@@ -1112,6 +1123,14 @@ struct TeamSmem {
 
 __device__ __forceinline__ void team_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The Uin-only test t of a cross cell.
+__device__ __forceinline__ bool cross_test(const GridGeom& g, const GpWeights& w, const double* u, int t) {
+    return t == 0   ? mood_shock_flow_part(u, g.nx, g)
+           : t == 1 ? mood_shock_grad_part(u, g.nx, g)
+           : t == 2 ? mood_u2_smooth<0>(u, g.nx, g, w.d2x)
+                    : mood_u2_smooth<1>(u, g.nx, g, w.d2y);
 }
 
 // Warp task `task` of the 4*nt faces of the listed cells.
@@ -1124,23 +1143,23 @@ __device__ __forceinline__ void team_faces(const StageArgs& a, const GpWeights& 
     const int base = lane - j, i = task * FPW + fl;
     const bool act = fl < FPW && i < 4 * nt;
     int dir = 0, sd = 0, lcell = 0;
-    if (act) lcell = lst[face_item(i, nt, &dir, &sd)];
+    if (act) lcell = *(volatile const int*)(lst + face_item(i, nt, &dir, &sd));
     const size_t step = dir == 0 ? (size_t)1 : (size_t)g.nx;
     const size_t c0 = act ? (size_t)lcell - (sd == 0 ? step : 0) : cidx(g, 1, 1);  // idle lanes: any valid face
     const size_t cs = c0 + (side ? step : 0);                                     // this lane's cell
     const int face = dir == 0 ? (side ? 0 : 2) : (side ? 3 : 1);
-    const int o = min((int)__ldcg(a.order + c0), (int)__ldcg(a.order + c0 + step));
     const ptrdiff_t row = g.nx;
+    Cell q[5];  // in flight with the orders: listed cells' faces are at order 3 or 1
+#pragma unroll
+    for (int m = 0; m < 5; m++) q[m] = ld_cell(a.uin + 4 * (cs + st_ox(m) + row * st_oy(m)));
+    const int o = min((int)__ldcg(a.order + c0), (int)__ldcg(a.order + c0 + step));
     double u[4];
     if (o >= 5) {  // not reached by listed cells; keeps the function total
-        Cell q[13];
+        Cell q5[13];
 #pragma unroll
-        for (int m = 0; m < 13; m++) q[m] = ld_cell(a.uin + 4 * (cs + st_ox(m) + row * st_oy(m)));
-        gp_recon_at<13>(&w.zt[2][face][gp][0], q, u);
+        for (int m = 0; m < 13; m++) q5[m] = ld_cell(a.uin + 4 * (cs + st_ox(m) + row * st_oy(m)));
+        gp_recon_at<13>(&w.zt[2][face][gp][0], q5, u);
     } else {
-        Cell q[5];
-#pragma unroll
-        for (int m = 0; m < 5; m++) q[m] = ld_cell(a.uin + 4 * (cs + st_ox(m) + row * st_oy(m)));
         if (o >= 3) gp_recon_at<5>(&sm.z3[face][gp][0], q, u);
         else gp_recon_at<1>(&sm.z1[face][gp], q, u);
         if (a.ccw) {
@@ -1221,9 +1240,34 @@ __device__ __forceinline__ bool cross_cell(const GridGeom& g, int t, int k, int*
     return l >= 1 && l <= g.lf && n >= 1 && n <= g.nf;
 }
 
-// The update and the decision on the crosses, by CTA 0: the last half of
-// mood_troubled.  A cross cell that several listed cells share is taken by the
-// first of them (a scan of a short list), or by whoever stamps it first.
+// The update of one cross cell and the decision on it: the last half of
+// mood_troubled.  flags: the Uin-only tests' results as bits, or -1 to run them
+// here.  Returns whether the cell is troubled (its order is lowered then).
+__device__ __forceinline__ bool cross_update(const StageArgs& a, const GpWeights& w, int c, int flags, double qx,
+                                             double qy) {
+    const GridGeom& g = a.g;
+    const double* uin = a.uin + 4 * (size_t)c;
+    const int o = (int)__ldcg(a.order + c);
+    const Cell uo = cell_update(g, a.uin, a.fx, a.fy, (size_t)c, qx, qy);
+    st_cell(a.uout + 4 * (size_t)c, uo);
+    if (o <= 1) {
+        if (inadmissible(uo)) atomicOr(&a.sc->status, GPM_STATUS_NAN);
+        return false;
+    }
+    const int r = mood_uout_part(uo, uin, g.nx, g);
+    bool trb = r == 1;
+    if (r == 2) {
+        if (flags >= 0) trb = (flags & 3) == 3 && !(g.u2 && (flags & 12));
+        else trb = mood_shock_part(uin, g.nx, g) && !(g.u2 && (mood_u2_smooth<0>(uin, g.nx, g, w.d2x) ||
+                                                               mood_u2_smooth<1>(uin, g.nx, g, w.d2y)));
+    }
+    if (trb) __stcg(a.order + c, (int8_t)(o == 3 ? 1 : 3));  // the cascade of cascade_order
+    return trb;
+}
+
+// The crosses of a team pass, by CTA 0.  A cross cell that several listed cells
+// share is taken by the first of them (a scan of a short list), or by whoever
+// stamps it first.
 __device__ __forceinline__ void team_cells(const StageArgs& a, const GpWeights& w, TeamSmem& sm, const int* lst,
                                            int cur, int nt, unsigned pid, double qx, double qy) {
     const GridGeom& g = a.g;
@@ -1242,29 +1286,12 @@ __device__ __forceinline__ void team_cells(const StageArgs& a, const GpWeights& 
             } else {
                 own = atomicExch(&a.stamp[c], pid) != pid;
             }
-            if (own) {
-                const double* uin = a.uin + 4 * (size_t)c;
-                const Cell uo = cell_update(g, a.uin, a.fx, a.fy, (size_t)c, qx, qy);
-                st_cell(a.uout + 4 * (size_t)c, uo);
-                const int o = (int)__ldcg(a.order + c);
-                if (o > 1) {
-                    const int r = mood_uout_part(uo, uin, nx, g);
-                    trb = r == 1;
-                    if (r == 2) {
-                        if (g.solo_split && i < TEAM_CROSS) {
-                            trb = sm.flag[0][i] && sm.flag[1][i] && !(g.u2 && (sm.flag[2][i] || sm.flag[3][i]));
-                        } else {
-                            trb = mood_shock_part(uin, nx, g) && !(g.u2 && (mood_u2_smooth<0>(uin, nx, g, w.d2x) ||
-                                                                            mood_u2_smooth<1>(uin, nx, g, w.d2y)));
-                        }
-                    }
-                    if (trb) __stcg(a.order + c, (int8_t)(o == 3 ? 1 : 3));  // the cascade of cascade_order
-                } else if (inadmissible(uo)) {
-                    atomicOr(&a.sc->status, GPM_STATUS_NAN);
-                }
-            }
+            const int flags = g.solo_split && i < TEAM_CROSS
+                                  ? sm.flag[0][i] | sm.flag[1][i] << 1 | sm.flag[2][i] << 2 | sm.flag[3][i] << 3
+                                  : -1;
+            if (own) trb = cross_update(a, w, c, flags, qx, qy);
         }
-        // warp-aggregated append to the next list, shared and global
+        // warp-aggregated append to the next list, of every member and global
         const unsigned m = __ballot_sync(0xffffffffu, trb);
         if (m) {
             int b0 = 0;
@@ -1273,31 +1300,31 @@ __device__ __forceinline__ void team_cells(const StageArgs& a, const GpWeights& 
             if (trb) {
                 const int idx = b0 + __popc(m & ((1u << lane) - 1));
                 __stcg(a.tlist[nxt] + idx, c);
-                if (idx < TEAM_LIST_CAP) sm.list[nxt][idx] = c;
+                if (idx < TEAM_LIST_CAP)
+#pragma unroll
+                    for (int r = 0; r < TEAM; r++)
+                        cooperative_groups::this_cluster().map_shared_rank(&sm, r)->list[nxt][idx] = c;
             }
         }
     }
+    __syncthreads();
+    if (threadIdx.x >= 1 && threadIdx.x < TEAM)
+        cooperative_groups::this_cluster().map_shared_rank(&sm, (int)threadIdx.x)->count[nxt] = sm.count[nxt];
 }
 
 // Passes pass+1, ... on the first cluster until the list is empty; returns the
-// pass count.  sm0: CTA 0's shared memory, seen from this CTA.
+// pass count.
 template <int NGP>
-__device__ __forceinline__ int team_loop(const StageArgs& a, const GpWeights& w, TeamSmem& sm, TeamSmem* sm0, int cur,
-                                         int nt, int pass, int max_pass, unsigned epoch, double qx, double qy) {
+__device__ __forceinline__ int team_loop(const StageArgs& a, const GpWeights& w, TeamSmem& sm, int cur, int nt, int pass,
+                                         int max_pass, unsigned epoch, double qx, double qy) {
     const int rank = (int)blockIdx.x, tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr int FPW = 32 / (2 * NGP);
-    for (int i = tid; i < 4 * NGP * 5; i += MOOD_THREADS) {
-        const int f = i / (5 * NGP), gp = (i / 5) % NGP, m = i % 5;
-        sm.z3[f][gp][m] = w.zt[1][f][gp][m];
-        if (m == 0) sm.z1[f][gp] = w.zt[0][f][gp][0];
-    }
-    if (rank == 0) {
-        for (int i = tid; i < nt && i < TEAM_LIST_CAP; i += MOOD_THREADS) sm.list[cur][i] = __ldcg(a.tlist[cur] + i);
-        if (tid == 0) sm.count[cur] = nt;
-    }
+    TeamSmem* sm0 = cooperative_groups::this_cluster().map_shared_rank(&sm, 0);
+    for (int i = tid; i < nt && i < TEAM_LIST_CAP; i += MOOD_THREADS) sm.list[cur][i] = __ldcg(a.tlist[cur] + i);
+    if (tid == 0) sm.count[cur] = nt;
     team_sync();
     for (;;) {
-        nt = *(volatile int*)&sm0->count[cur];
+        nt = *(volatile int*)&sm.count[cur];
         if (nt == 0) break;
         if (pass >= max_pass) {
             if (rank == 0 && tid == 0) a.sc->status |= GPM_STATUS_MOODCAP;
@@ -1308,7 +1335,7 @@ __device__ __forceinline__ int team_loop(const StageArgs& a, const GpWeights& w,
             sm.count[cur ^ 1] = 0;  // read last before the two barriers of the pass before
             a.sc->detected_step += (unsigned long long)nt;
         }
-        const int* lst = nt <= TEAM_LIST_CAP ? sm0->list[cur] : a.tlist[cur];
+        const int* lst = nt <= TEAM_LIST_CAP ? sm.list[cur] : a.tlist[cur];
         const int nface = (4 * nt + FPW - 1) / FPW, ncross = a.g.solo_split ? min(5 * nt, TEAM_CROSS) : 0;
         const int chunks = (ncross + 31) / 32;
         for (int task = warp * TEAM + rank; task < nface + 4 * chunks; task += (MOOD_THREADS / 32) * TEAM) {
@@ -1317,13 +1344,8 @@ __device__ __forceinline__ int team_loop(const StageArgs& a, const GpWeights& w,
             } else {
                 const int t = (task - nface) & 3, i = ((task - nface) >> 2) * 32 + lane;
                 int c;
-                if (i < ncross && cross_cell(a.g, lst[i / 5], i % 5, &c)) {
-                    const double* u = a.uin + 4 * (size_t)c;
-                    sm0->flag[t][i] = t == 0   ? mood_shock_flow_part(u, a.g.nx, a.g)
-                                      : t == 1 ? mood_shock_grad_part(u, a.g.nx, a.g)
-                                      : t == 2 ? mood_u2_smooth<0>(u, a.g.nx, a.g, w.d2x)
-                                               : mood_u2_smooth<1>(u, a.g.nx, a.g, w.d2y);
-                }
+                if (i < ncross && cross_cell(a.g, lst[i / 5], i % 5, &c))
+                    sm0->flag[t][i] = cross_test(a.g, w, a.uin + 4 * (size_t)c, t);
             }
         }
         team_sync();
@@ -1331,7 +1353,7 @@ __device__ __forceinline__ int team_loop(const StageArgs& a, const GpWeights& w,
         team_sync();
         cur ^= 1;
     }
-    team_sync();  // CTA 0's shared memory stays until everyone has left it
+    team_sync();  // a member's shared memory stays until no one writes to it
     return pass;
 }
 
@@ -1342,16 +1364,26 @@ __global__ void __launch_bounds__(MOOD_THREADS, 1) k_mood_loop(StageArgs a, cons
     const GridGeom& g = a.g;
     const double qx = a.sc->qx, qy = a.sc->qy;
     const unsigned epoch = a.sc->stamp_epoch;  // stamps epoch+2, epoch+3, ... are new
-    const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gstride = gridDim.x * blockDim.x;
-    const int stid = pack_tid();  // whole warps of work items, dealt over all SMs
+    const int tid = (int)threadIdx.x, lane = tid & 31, gtid = blockIdx.x * MOOD_THREADS + tid;
+    const int slot = (tid >> 5) * (int)gridDim.x + (int)blockIdx.x;  // warp tasks are dealt over the SMs first
+    const int slots = (MOOD_THREADS / 32) * (int)gridDim.x;
+    constexpr int FPW = 32 / (2 * NGP);
     int cur = 0, pass = 1;  // pass 1 (all faces) ran before this kernel
+    int nt = *(volatile int*)&a.sc->ntrb[cur];
+    if (nt != 0) {
+        for (int i = tid; i < 4 * NGP * 5; i += MOOD_THREADS) {
+            const int f = i / (5 * NGP), gp = (i / 5) % NGP, m = i % 5;
+            team_sm.z3[f][gp][m] = w.zt[1][f][gp][m];
+            if (m == 0) team_sm.z1[f][gp] = w.zt[0][f][gp][0];
+        }
+        __syncthreads();
+    }
+    GridWait wait = grid_start(bar);
     for (;;) {
-        const int nt = *(volatile int*)&a.sc->ntrb[cur];
         if (nt == 0) break;
         if (nt <= g.mood_solo) {
             if (blockIdx.x >= TEAM) return;
-            TeamSmem* sm0 = cooperative_groups::this_cluster().map_shared_rank(&team_sm, 0);
-            pass = team_loop<NGP>(a, w, team_sm, sm0, cur, nt, pass, max_pass, epoch, qx, qy);
+            pass = team_loop<NGP>(a, w, team_sm, cur, nt, pass, max_pass, epoch, qx, qy);
             break;
         }
         if (pass >= max_pass) {
@@ -1364,37 +1396,36 @@ __global__ void __launch_bounds__(MOOD_THREADS, 1) k_mood_loop(StageArgs a, cons
             a.sc->ntrb[cur ^ 1] = 0;  // nobody appends to it before the next barrier
             a.sc->detected_step += (unsigned long long)nt;
         }
-        // the four faces of every troubled cell at the new orders
-        // x and y faces share warps (face_gp_dyn): 4*nt items packed densely
-        face_phase_gp<NGP>(4 * nt, 4 * nt, stid, gstride, [&](int i, int gp, FaceGp& f) {
-            int dir, side;
-            const size_t c = (size_t)a.tlist[cur][face_item(i, nt, &dir, &side)];
-            face_gp_dyn(a, w, side == 0 ? (dir == 0 ? c - 1 : c - g.nx) : c, dir, gp, f);
-        });
-        if (!grid_sync(bar)) return;
+        const int* lst = a.tlist[cur];
+        const int nface = (4 * nt + FPW - 1) / FPW, total = 5 * nt, chunks = (total + 31) / 32;
+        for (int task = slot; task < nface + 4 * chunks; task += slots) {
+            if (task < nface) {
+                team_faces<NGP>(a, w, team_sm, lst, nt, task);
+            } else {  // a cell's results are the same from whichever cross they come
+                const int t = (task - nface) & 3, i = ((task - nface) >> 2) * 32 + lane;
+                int c;
+                if (i < total && cross_cell(g, __ldcg(lst + i / 5), i % 5, &c))
+                    __stcg(a.tests + 4 * (size_t)c + t, (unsigned char)cross_test(g, w, a.uin + 4 * (size_t)c, t));
+            }
+        }
+        if (!grid_sync(bar, wait)) return;
         // the 5-point crosses: Uout from Uin and the current fluxes, DETECTION
         const unsigned pid = epoch + (unsigned)pass;
-        const int nxt = cur ^ 1, total = 5 * nt;
-        const int lim = ((total + gstride - 1) / gstride) * gstride;
-        for (int base = 0; base < lim; base += gstride) {
-            const int i = base + stid;
+        const int nxt = cur ^ 1;
+        for (int task = slot; task < chunks; task += slots) {
+            const int i = task * 32 + lane;
             bool trb = false;
-            int cval = 0;
-            if (i < total) {
-                int c;
-                if (cross_cell(g, a.tlist[cur][i / 5], i % 5, &c) && atomicExch(&a.stamp[c], pid) != pid) {
-                    const Cell uo = cell_update(g, a.uin, a.fx, a.fy, (size_t)c, qx, qy);
-                    st_cell(a.uout + 4 * (size_t)c, uo);
-                    if (a.order[c] > 1) trb = mood_troubled(uo, a.uin + 4 * (size_t)c, g.nx, g, w.d2x, w.d2y);
-                    else if (inadmissible(uo)) atomicOr(&a.sc->status, GPM_STATUS_NAN);
-                    cval = c;
-                }
+            int c = 0;
+            if (i < total && cross_cell(g, __ldcg(lst + i / 5), i % 5, &c)) {
+                const unsigned f = __ldcg(reinterpret_cast<const unsigned*>(a.tests) + c);
+                const int flags = (int)((f & 1) | (f >> 7 & 2) | (f >> 14 & 4) | (f >> 21 & 8));
+                if (atomicExch(&a.stamp[c], pid) != pid) trb = cross_update(a, w, c, flags, qx, qy);
             }
-            if (trb) cascade_order(&a.order[cval]);
-            list_append(trb, a.tlist[nxt], &a.sc->ntrb[nxt], cval);
+            list_append(trb, a.tlist[nxt], &a.sc->ntrb[nxt], c);
         }
-        if (!grid_sync(bar)) return;
+        if (!grid_sync(bar, wait)) return;
         cur ^= 1;
+        nt = *(volatile int*)&a.sc->ntrb[cur];
     }
     if (gtid == 0) {  // every CTA read the epoch before the first barrier
         a.sc->passes_stage[stage] = pass;
@@ -2046,6 +2077,7 @@ template <int NGP>
 __global__ void __launch_bounds__(MOOD_THREADS, 1) kb_mood_loop(BatchArgs a, GridBar* bar, int max_pass) {
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gstride = gridDim.x * blockDim.x;
     int stid = pack_tid(), wstride = gstride;
+    GridWait wait = grid_start(bar);
     bool solo = false;
     int cur = 0, pass = 1;
     for (;;) {
@@ -2070,7 +2102,7 @@ __global__ void __launch_bounds__(MOOD_THREADS, 1) kb_mood_loop(BatchArgs a, Gri
         }
         face_phase_gp<NGP>(4 * nt, 2 * nt, stid, wstride,
                            [&](int i, int gp, FaceGp& f) { kb_face_gp(a, cur, nt, i, gp, f); });
-        if (!mood_sync(bar, solo)) return;
+        if (!mood_sync(bar, wait, solo)) return;
         const unsigned epoch = (unsigned)*(volatile int*)&a.ntrb[2];
         const int nxt = cur ^ 1, total = 5 * nt;
         const int lim = ((total + wstride - 1) / wstride) * wstride;
@@ -2102,7 +2134,7 @@ __global__ void __launch_bounds__(MOOD_THREADS, 1) kb_mood_loop(BatchArgs a, Gri
             if (trb) cascade_order(a.order + a.prob[val.x].off + val.y);
             list_append2(trb, a.tlist[nxt], &a.ntrb[nxt], val);
         }
-        if (!mood_sync(bar, solo)) return;
+        if (!mood_sync(bar, wait, solo)) return;
         cur ^= 1;
     }
     if (gtid == 0) a.ntrb[5] = pass;
