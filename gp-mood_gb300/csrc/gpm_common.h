@@ -136,6 +136,7 @@ struct DevScalars {
     int ntrb[2];                      // troubled-cell counts, double-buffered lists; the MOOD loop leaves them 0
     int passes_stage[GPM_MAXST];      // MOOD passes of each RK stage of the last step (device loop)
     unsigned stamp_epoch;             // first unused pass stamp of the device MOOD loop
+    int mood_cur, mood_pass;          // k_mood_loop's state for k_mood_team: the current list, the passes so far
     double bcd[4][4];                 // Dirichlet BC (19): the right ghost columns' states, from the host
 };
 
@@ -185,8 +186,8 @@ struct KernelTable {
     void (*dt_finalize)(const GridGeom& g, DevScalars* sc, double dtfinal, cudaStream_t s);
     // a device-resident step's start at time t: dt from Setdt, counters cleared
     void (*step_begin)(const GridGeom& g, DevScalars* sc, double t, cudaStream_t s);
-    // MOOD passes 2, 3, ... of RK stage `stage` in one cooperative launch; the
-    // pass count goes to sc->passes_stage[stage]; returns -1 if the launch failed
+    // MOOD passes 2, 3, ... of RK stage `stage` (a cooperative launch and a cluster); the
+    // pass count goes to sc->passes_stage[stage]; returns -1 if a launch failed
     int (*mood_loop)(const StageArgs& a, const GpWeights& w, GridBar* bar, int max_pass, int stage,
                      cudaStream_t s);
     // y = sum c[i]*x[i], i < n <= 5, left to right; optionally the Setdt reduction of y

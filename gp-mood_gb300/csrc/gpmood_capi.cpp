@@ -231,7 +231,7 @@ int run_stage(gpmood_ctx* c, double* uin, double* uout, int stage, int bc_stage,
         const int max_pass = cap > 0x7fffffff ? 0x7fffffff : (int)cap;
         if (kt.mood_loop(a, c->w, c->dBar, max_pass, stage, s))
             return fail(c, GPMOOD_E_CUDA, "MOOD loop launch: %s", cudaGetErrorString(cudaGetLastError()));
-        c->ctr.kernel_launches += 1;
+        c->ctr.kernel_launches += 2;
     }
     if (c->timing) cudaEventRecord(ev[3], s);
     if (stage == 0 && c->hvX) {  // training samples of stage 1 (mod_FE.f90:176-181)

@@ -14,10 +14,10 @@
 //                         cell, troubled cells (order already lowered 5->3->1)
 //                         compacted into a list
 //   k_mood_loop           while the list is not empty (the MOOD loop,
-//                         mod_FE.f90:69-174), in one cooperative launch:
-//                         recompute the 4 faces of each troubled cell, then
-//                         Uout of its 5-point cross with DETECTION there ->
-//                         next list
+//   k_mood_team           mod_FE.f90:69-174), long lists in a cooperative
+//                         launch, short ones on one cluster: recompute the 4
+//                         faces of each troubled cell, then Uout of its
+//                         5-point cross with DETECTION there -> next list
 //   k_bc                  Boundary_C(Uout)
 //   k_combine_bc          SSP-RK3 combination (mod_SSP_RK3.f90:28,33) with
 //                         Boundary_C(Uout) of the stage before it and, in the
@@ -1103,8 +1103,8 @@ __device__ __forceinline__ bool mood_sync(GridBar* b, GridWait& w, bool solo) {
 //    after the barrier only the update, positivity and the density bounds are
 //    left, one lane a cross cell.
 // Passes over more than GridGeom::mood_solo cells run on all SMs with grid
-// barriers.  Shorter ones run on the first thread-block cluster (the "team")
-// with cluster barriers (~1k cycles with what they wait for, against ~4k):
+// barriers (k_mood_loop).  Shorter ones run on one thread-block cluster (the
+// "team", k_mood_team) with cluster barriers (~1k cycles with what they wait for, against ~4k):
 // 8 SMs take 32 warps side by side, and CTA 0 runs the cells.  The team's lists
 // live in every member's shared memory (and in the global list, which a longer
 // one is read from), the tests' results in CTA 0's, through distributed shared
@@ -1121,8 +1121,10 @@ struct TeamSmem {
     double z1[4][GPM_MAXGP];             // order 1
 };
 
-__device__ __forceinline__ void team_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+__device__ __forceinline__ void team_sync() {  // every thread arrives for itself: no assumption on convergence
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+    __syncwarp();
 }
 
 // The Uin-only test t of a cross cell.
@@ -1312,55 +1314,23 @@ __device__ __forceinline__ void team_cells(const StageArgs& a, const GpWeights& 
         cooperative_groups::this_cluster().map_shared_rank(&sm, (int)threadIdx.x)->count[nxt] = sm.count[nxt];
 }
 
-// Passes pass+1, ... on the first cluster until the list is empty; returns the
-// pass count.
+// Order-3 and order-1 weights into shared memory.
 template <int NGP>
-__device__ __forceinline__ int team_loop(const StageArgs& a, const GpWeights& w, TeamSmem& sm, int cur, int nt, int pass,
-                                         int max_pass, unsigned epoch, double qx, double qy) {
-    const int rank = (int)blockIdx.x, tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    constexpr int FPW = 32 / (2 * NGP);
-    TeamSmem* sm0 = cooperative_groups::this_cluster().map_shared_rank(&sm, 0);
-    for (int i = tid; i < nt && i < TEAM_LIST_CAP; i += MOOD_THREADS) sm.list[cur][i] = __ldcg(a.tlist[cur] + i);
-    if (tid == 0) sm.count[cur] = nt;
-    team_sync();
-    for (;;) {
-        nt = *(volatile int*)&sm.count[cur];
-        if (nt == 0) break;
-        if (pass >= max_pass) {
-            if (rank == 0 && tid == 0) a.sc->status |= GPM_STATUS_MOODCAP;
-            break;
-        }
-        pass++;
-        if (rank == 0 && tid == 0) {
-            sm.count[cur ^ 1] = 0;  // read last before the two barriers of the pass before
-            a.sc->detected_step += (unsigned long long)nt;
-        }
-        const int* lst = nt <= TEAM_LIST_CAP ? sm.list[cur] : a.tlist[cur];
-        const int nface = (4 * nt + FPW - 1) / FPW, ncross = a.g.solo_split ? min(5 * nt, TEAM_CROSS) : 0;
-        const int chunks = (ncross + 31) / 32;
-        for (int task = warp * TEAM + rank; task < nface + 4 * chunks; task += (MOOD_THREADS / 32) * TEAM) {
-            if (task < nface) {
-                team_faces<NGP>(a, w, sm, lst, nt, task);
-            } else {
-                const int t = (task - nface) & 3, i = ((task - nface) >> 2) * 32 + lane;
-                int c;
-                if (i < ncross && cross_cell(a.g, lst[i / 5], i % 5, &c))
-                    sm0->flag[t][i] = cross_test(a.g, w, a.uin + 4 * (size_t)c, t);
-            }
-        }
-        team_sync();
-        if (rank == 0) team_cells(a, w, sm, lst, cur, nt, epoch + (unsigned)pass, qx, qy);
-        team_sync();
-        cur ^= 1;
+__device__ __forceinline__ void team_weights(TeamSmem& sm, const GpWeights& w) {
+    for (int i = (int)threadIdx.x; i < 4 * NGP * 5; i += MOOD_THREADS) {
+        const int f = i / (5 * NGP), gp = (i / 5) % NGP, m = i % 5;
+        sm.z3[f][gp][m] = w.zt[1][f][gp][m];
+        if (m == 0) sm.z1[f][gp] = w.zt[0][f][gp][0];
     }
-    team_sync();  // a member's shared memory stays until no one writes to it
-    return pass;
 }
 
+// Passes 2, 3, ... over lists of more than GridGeom::mood_solo cells, on all SMs
+// (a cooperative launch).  Leaves the list, which of the two it is and the
+// pass count for k_mood_team.
 template <int NGP>
 __global__ void __launch_bounds__(MOOD_THREADS, 1) k_mood_loop(StageArgs a, const __grid_constant__ GpWeights w, GridBar* bar,
-                                                      int max_pass, int stage) {
-    __shared__ TeamSmem team_sm;
+                                                      int max_pass) {
+    __shared__ TeamSmem sm;
     const GridGeom& g = a.g;
     const double qx = a.sc->qx, qy = a.sc->qy;
     const unsigned epoch = a.sc->stamp_epoch;  // stamps epoch+2, epoch+3, ... are new
@@ -1370,26 +1340,10 @@ __global__ void __launch_bounds__(MOOD_THREADS, 1) k_mood_loop(StageArgs a, cons
     constexpr int FPW = 32 / (2 * NGP);
     int cur = 0, pass = 1;  // pass 1 (all faces) ran before this kernel
     int nt = *(volatile int*)&a.sc->ntrb[cur];
-    if (nt != 0) {
-        for (int i = tid; i < 4 * NGP * 5; i += MOOD_THREADS) {
-            const int f = i / (5 * NGP), gp = (i / 5) % NGP, m = i % 5;
-            team_sm.z3[f][gp][m] = w.zt[1][f][gp][m];
-            if (m == 0) team_sm.z1[f][gp] = w.zt[0][f][gp][0];
-        }
-        __syncthreads();
-    }
     GridWait wait = grid_start(bar);
-    for (;;) {
-        if (nt == 0) break;
-        if (nt <= g.mood_solo) {
-            if (blockIdx.x >= TEAM) return;
-            pass = team_loop<NGP>(a, w, team_sm, cur, nt, pass, max_pass, epoch, qx, qy);
-            break;
-        }
-        if (pass >= max_pass) {
-            if (gtid == 0) a.sc->status |= GPM_STATUS_MOODCAP;
-            break;
-        }
+    if (nt > g.mood_solo) team_weights<NGP>(sm, w);
+    __syncthreads();
+    while (nt > g.mood_solo && pass < max_pass) {
         pass++;
         // the listed cells' orders were lowered when they were listed
         if (gtid == 0) {
@@ -1400,7 +1354,7 @@ __global__ void __launch_bounds__(MOOD_THREADS, 1) k_mood_loop(StageArgs a, cons
         const int nface = (4 * nt + FPW - 1) / FPW, total = 5 * nt, chunks = (total + 31) / 32;
         for (int task = slot; task < nface + 4 * chunks; task += slots) {
             if (task < nface) {
-                team_faces<NGP>(a, w, team_sm, lst, nt, task);
+                team_faces<NGP>(a, w, sm, lst, nt, task);
             } else {  // a cell's results are the same from whichever cross they come
                 const int t = (task - nface) & 3, i = ((task - nface) >> 2) * 32 + lane;
                 int c;
@@ -1427,10 +1381,63 @@ __global__ void __launch_bounds__(MOOD_THREADS, 1) k_mood_loop(StageArgs a, cons
         cur ^= 1;
         nt = *(volatile int*)&a.sc->ntrb[cur];
     }
-    if (gtid == 0) {  // every CTA read the epoch before the first barrier
+    if (gtid == 0) {
+        a.sc->mood_cur = cur;
+        a.sc->mood_pass = pass;
+    }
+}
+
+// The rest of the loop, on one cluster (a launch of TEAM CTAs) until the list is
+// empty or max_pass is reached, and the loop's results.
+template <int NGP>
+__global__ void __launch_bounds__(MOOD_THREADS, 1) k_mood_team(StageArgs a, const __grid_constant__ GpWeights w,
+                                                      const GridBar* bar, int max_pass, int stage) {
+    __shared__ TeamSmem sm;
+    if (bar->err) return;  // a grid barrier ran out before: the host reports it and starts over
+    const double qx = a.sc->qx, qy = a.sc->qy;
+    const unsigned epoch = a.sc->stamp_epoch;
+    const int rank = (int)blockIdx.x, tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    constexpr int FPW = 32 / (2 * NGP);
+    TeamSmem* sm0 = cooperative_groups::this_cluster().map_shared_rank(&sm, 0);
+    int cur = a.sc->mood_cur, pass = a.sc->mood_pass;
+    int nt = a.sc->ntrb[cur];
+    if (nt != 0) {
+        team_weights<NGP>(sm, w);
+        for (int i = tid; i < nt && i < TEAM_LIST_CAP; i += MOOD_THREADS) sm.list[cur][i] = __ldcg(a.tlist[cur] + i);
+        if (tid == 0) sm.count[cur] = nt;
+        team_sync();
+        while (nt != 0 && pass < max_pass) {
+            pass++;
+            if (rank == 0 && tid == 0) {
+                sm.count[cur ^ 1] = 0;  // read last before the two barriers of the pass before
+                a.sc->detected_step += (unsigned long long)nt;
+            }
+            const int* lst = nt <= TEAM_LIST_CAP ? sm.list[cur] : a.tlist[cur];
+            const int nface = (4 * nt + FPW - 1) / FPW, ncross = a.g.solo_split ? min(5 * nt, TEAM_CROSS) : 0;
+            const int chunks = (ncross + 31) / 32;
+            for (int task = warp * TEAM + rank; task < nface + 4 * chunks; task += (MOOD_THREADS / 32) * TEAM) {
+                if (task < nface) {
+                    team_faces<NGP>(a, w, sm, lst, nt, task);
+                } else {
+                    const int t = (task - nface) & 3, i = ((task - nface) >> 2) * 32 + lane;
+                    int c;
+                    if (i < ncross && cross_cell(a.g, lst[i / 5], i % 5, &c))
+                        sm0->flag[t][i] = cross_test(a.g, w, a.uin + 4 * (size_t)c, t);
+                }
+            }
+            team_sync();
+            if (rank == 0) team_cells(a, w, sm, lst, cur, nt, epoch + (unsigned)pass, qx, qy);
+            team_sync();
+            cur ^= 1;
+            nt = *(volatile int*)&sm.count[cur];
+        }
+        team_sync();  // a member's shared memory stays until no one writes to it
+    }
+    if (rank == 0 && tid == 0) {
+        if (nt != 0) a.sc->status |= GPM_STATUS_MOODCAP;
         a.sc->passes_stage[stage] = pass;
         a.sc->stamp_epoch = epoch + (unsigned)pass + 1u;
-        a.sc->ntrb[0] = a.sc->ntrb[1] = 0;  // for the next stage; CTAs that still poll leave on 0 as on the end
+        a.sc->ntrb[0] = a.sc->ntrb[1] = 0;  // for the next stage
     }
 }
 
@@ -1440,27 +1447,28 @@ static int launch_mood_loop_n(const StageArgs& a, const GpWeights& w, GridBar* b
     static std::atomic<int> grids[GPM_MAX_DEVICES];
     const int dev = gpm_device();
     int grid = grids[dev].load(std::memory_order_relaxed);
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = TEAM;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeCooperative;
-    at[1].val.cooperative = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(MOOD_THREADS);
-    cfg.stream = s;
-    cfg.attrs = at;
-    if (!grid) {  // every cluster that fits at once: the grid barrier needs all CTAs resident
-        int clusters = 0;
-        cfg.gridDim = dim3(TEAM);
-        cfg.numAttrs = 1;
-        if (cudaOccupancyMaxActiveClusters(&clusters, k_mood_loop<NGP>, &cfg) != cudaSuccess || clusters < 1) return -1;
-        grid = clusters * TEAM;
+    if (!grid) {
+        int sms = 0, occ = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_mood_loop<NGP>, MOOD_THREADS, 0);
+        grid = sms * (occ > 0 ? occ : 1);
         grids[dev].store(grid, std::memory_order_relaxed);
     }
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+    cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, k_mood_loop<NGP>, a, w, bar, max_pass, stage) == cudaSuccess ? 0 : -1;
+    cfg.blockDim = dim3(MOOD_THREADS);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, k_mood_loop<NGP>, a, w, bar, max_pass) != cudaSuccess) return -1;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = TEAM;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(TEAM);
+    return cudaLaunchKernelEx(&cfg, k_mood_team<NGP>, a, w, (const GridBar*)bar, max_pass, stage) == cudaSuccess ? 0 : -1;
 }
 
 int launch_mood_loop(const StageArgs& a, const GpWeights& w, GridBar* bar, int max_pass, int stage,
