@@ -8,8 +8,8 @@
 // One stage (Forward_Euler, gp-mood-code/mod_FE.f90:20-190) runs as:
 //   k_bc                  Boundary_C(Uin)                      BC.f90:10-421
 //   k_flux_xy_tma         every face: GP recon + HLLC + quadrature, stored
-//   (k_flux_tile<x|y>)    (the first MOOD pass, mod_FE.f90:73-145); fast mode
-//                         both directions per tile, exact mode one per launch
+//   (k_flux_gp)           (the first MOOD pass, mod_FE.f90:73-145); fast mode
+//                         by tiles of cells, exact mode by Gauss points
 //   k_update_detect       Uout = Uin + flux differences, DETECTION on every
 //                         cell, troubled cells (order already lowered 5->3->1)
 //                         compacted into a list
@@ -41,6 +41,7 @@
 #include <cooperative_groups.h>
 
 #include <mutex>
+#include <type_traits>
 
 #if GPM_EXACT
 #define GPM_NS gpm_exact
@@ -49,9 +50,6 @@
 #endif
 
 namespace GPM_NS {
-
-constexpr int TX = 32, TY = 8;           // faces per CTA tile
-constexpr int HX = TX + 5, HY = TY + 5;  // cells staged per tile (halo 2 below, 3 above)
 
 __device__ __forceinline__ size_t cidx(const GridGeom& g, int l, int n) {
     return (size_t)(n + 3) * (size_t)g.nx + (size_t)(l + 3);
@@ -195,10 +193,8 @@ void launch_bc(const GridGeom& g, double* u, const DevScalars* sc, int stage, cu
 }
 
 // ---------------------------------------------------------------------------
-// First MOOD pass: every face of the stage.  One thread per face; the CTA
-// stages its (TX+5) x (TY+5) cells of Uin in shared memory, then each thread
-// reconstructs the two face states at every Gauss point (13-point GP dot
-// products), solves HLLC and integrates along the face.
+// First MOOD pass: every face of the stage (k_flux_gp; k_flux_xy in fast mode
+// where it applies).
 
 // Gauss-point states of face `face` of one cell at order index o: the fast
 // kernels use the mirror-symmetric split for ngp = 3 above first order.
@@ -238,70 +234,88 @@ __device__ __forceinline__ void cc_blend(double v1, double v2, const Cell& c, do
     for (int k = 0; k < 4; k++) u[k] = NP == 1 ? cv[k] : v1 * cv[k] + v2 * u[k];
 }
 
-// ccw != NULL (NN_GP_MOOD_CC): (l, n) is the low cell of the face.
-template <int DIR, int NP, int NGP>
-__device__ __forceinline__ void face_from_tile(const GpWeights& w, int o, const Cell (*tile)[HX], int tx, int ty,
-                                               double* F, int nflux, const float* ccw = nullptr,
-                                               const GridGeom* g = nullptr, int l = 0, int n = 0) {
-    constexpr int FL = DIR == 0 ? 2 : 1;  // iR (x) / iT (y) face of the low cell
-    constexpr int FH = DIR == 0 ? 0 : 3;  // iL (x) / iB (y) face of the high cell
-    constexpr int hx = DIR == 0 ? 1 : 0, hy = DIR == 0 ? 0 : 1;
-    double uL[NGP][4], uR[NGP][4];
-    {
-        Cell q[NP];
-#pragma unroll
-        for (int m = 0; m < NP; m++) q[m] = tile[ty + st_oy(m)][tx + st_ox(m)];
-        recon_face<DIR, NP, NGP>(w, o, FL, q, uL);
-        if (ccw) {
-            double v1, v2;
-            cc_weights(*g, ccw, l, n, &v1, &v2);
-#pragma unroll
-            for (int j = 0; j < NGP; j++) cc_blend<NP>(v1, v2, q[0], uL[j]);
-        }
-    }
-    {
-        Cell q[NP];
-#pragma unroll
-        for (int m = 0; m < NP; m++) q[m] = tile[ty + hy + st_oy(m)][tx + hx + st_ox(m)];
-        recon_face<DIR, NP, NGP>(w, o, FH, q, uR);
-        if (ccw) {
-            double v1, v2;
-            cc_weights(*g, ccw, l + hx, n + hy, &v1, &v2);
-#pragma unroll
-            for (int j = 0; j < NGP; j++) cc_blend<NP>(v1, v2, q[0], uR[j]);
-        }
-    }
-    quad_flux<DIR, NGP>(uL, uR, w.gw, F, nflux);
-}
-
-template <int DIR, int NGP, int UORD>  // UORD: uniform order (1,3,5) or 0 = per-face from the order array
-__global__ void __launch_bounds__(TX * TY) k_flux_tile(StageArgs a, const __grid_constant__ GpWeights w) {
-    __shared__ Cell tile[HY][HX];
+// One lane per Gauss point of a face, 32/NGP faces per warp, x faces first (a
+// warp holds one direction): each lane reconstructs both sides at its point,
+// solves its Riemann problem, and the face's lanes sum the quadrature by
+// shuffles in Gauss-point order, quad_flux's expression, so the bits are those
+// of a thread per face.  That form ran 1100 FP64 instructions in a row in the
+// exact mode, 64 cycles each for a lone warp, in two launches (two directions)
+// of few large CTAs: 88 us each from 48x40 up to 128^2, 393 us each at 400^2
+// (71 % of the FP64 pipe: too few warps at 170 registers, and a tail per
+// direction).  A third of the chain, both directions in one launch of
+// 128-thread CTAs.  Stencils come through L1, whose lines a face's lanes share;
+// the weights from shared memory, where lanes of different points read apart.
+template <int NGP, int UORD>  // UORD: uniform order (1,3,5) or 0 = per-face from the order array
+__global__ void __launch_bounds__(128, 4) k_flux_gp(StageArgs a, const __grid_constant__ GpWeights w) {
+    constexpr int NO = UORD == 0 ? 3 : 1, FPW = 32 / NGP;
+    __shared__ double z[NO][4][NGP][13];
     const GridGeom& g = a.g;
-    const int lmin = DIR == 0 ? 0 : 1, nmin = DIR == 0 ? 1 : 0;
-    const int l0 = lmin + blockIdx.x * TX, n0 = nmin + blockIdx.y * TY;
-    const int tid = threadIdx.y * TX + threadIdx.x;
-    for (int i = tid; i < HX * HY; i += TX * TY) {
-        const int cy = i / HX, cx = i - cy * HX;
-        const int l = l0 - 2 + cx, n = n0 - 2 + cy;
-        if (l >= -3 && l <= g.lf + 4 && n >= -3 && n <= g.nf + 4) tile[cy][cx] = ld_cell(a.uin + 4 * cidx(g, l, n));
+    for (int i = threadIdx.x; i < NO * 4 * NGP * 13; i += 128) {
+        const int o = i / (4 * NGP * 13), r = i - o * (4 * NGP * 13);
+        z[o][r / (NGP * 13)][r / 13 % NGP][r % 13] = w.zt[UORD == 0 ? o : UORD / 2][r / (NGP * 13)][r / 13 % NGP][r % 13];
     }
     __syncthreads();
-    const int l = l0 + threadIdx.x, n = n0 + threadIdx.y;
-    if (l > g.lf || n > g.nf) return;
-    const int tx = threadIdx.x + 2, ty = threadIdx.y + 2;
-    double F[4];
-    if (UORD != 0) {
-        face_from_tile<DIR, np_of(UORD == 0 ? 1 : UORD), NGP>(w, UORD / 2, tile, tx, ty, F, g.num_flux);
-    } else {
-        const size_t c0 = cidx(g, l, n), c1 = DIR == 0 ? c0 + 1 : c0 + g.nx;
-        const int o = min((int)a.order[c0], (int)a.order[c1]);
-        if (o >= 5) face_from_tile<DIR, 13, NGP>(w, 2, tile, tx, ty, F, g.num_flux);
-        else if (o >= 3) face_from_tile<DIR, 5, NGP>(w, 1, tile, tx, ty, F, g.num_flux, a.ccw, &g, l, n);
-        else face_from_tile<DIR, 1, NGP>(w, 0, tile, tx, ty, F, g.num_flux, a.ccw, &g, l, n);
+    const int lane = threadIdx.x & 31, fl = lane / NGP, gp = lane - fl * NGP, lead = lane - gp;
+    const long long nfx = (long long)(g.lf + 1) * g.nf, nfy = (long long)g.lf * (g.nf + 1);
+    const long long nxw = (nfx + FPW - 1) / FPW, wi = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    const int dir = wi < nxw ? 0 : 1;
+    const long long i = (dir == 0 ? wi : wi - nxw) * FPW + fl;
+    const bool act = fl < FPW && gp < NGP && i < (dir == 0 ? nfx : nfy);
+    const int len = dir == 0 ? g.lf + 1 : g.lf;
+    const int row = act ? (int)(i / len) : 0;
+    const int l = dir == 0 ? (act ? (int)(i - (long long)row * len) : 0) : 1 + (act ? (int)(i - (long long)row * len) : 0);
+    const int n = dir == 0 ? 1 + row : row;
+    const size_t c0 = cidx(g, l, n), c1 = dir == 0 ? c0 + 1 : c0 + g.nx;
+    double F[4] = {0., 0., 0., 0.};
+    if (act) {
+        const int FL = dir == 0 ? 2 : 1, FH = dir == 0 ? 0 : 3;
+        double uL[4], uR[4];
+        auto states = [&](auto np, int o) {
+            constexpr int NP = decltype(np)::value;
+            const ptrdiff_t r = g.nx;
+#pragma unroll
+            for (int side = 0; side < 2; side++) {
+                const double* u = a.uin + 4 * (side ? c1 : c0);
+                const double* zz = &z[UORD == 0 ? o : 0][side ? FH : FL][gp][0];
+                double* s = side ? uR : uL;
+                Cell q[NP];
+#pragma unroll
+                for (int m = 0; m < NP; m++) q[m] = ld_cell(u + 4 * (st_ox(m) + r * st_oy(m)));
+                gp_recon_at<NP>(zz, q, s);
+                if (NP < 13 && UORD == 0 && a.ccw) {
+                    double v1, v2;
+                    cc_weights(g, a.ccw, l + (side && dir == 0), n + (side && dir == 1), &v1, &v2);
+                    cc_blend<NP>(v1, v2, q[0], s);
+                }
+            }
+        };
+        if (UORD != 0) {
+            states(std::integral_constant<int, np_of(UORD == 0 ? 1 : UORD)>{}, 0);
+        } else {
+            const int o = min((int)a.order[c0], (int)a.order[c1]);
+            if (o >= 5) states(std::integral_constant<int, 13>{}, 2);
+            else if (o >= 3) states(std::integral_constant<int, 5>{}, 1);
+            else states(std::integral_constant<int, 1>{}, 0);
+        }
+        if (dir == 0) riemann<0>(g.num_flux, uL, uR, F);
+        else riemann<1>(g.num_flux, uL, uR, F);
     }
-    double* out = (DIR == 0 ? a.fx : a.fy) + 4 * cidx(g, l, n);
-    st_cell(out, Cell{F[0], F[1], F[2], F[3]});
+    double acc[4];
+#pragma unroll
+    for (int j = 0; j < NGP; j++) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const double v = __shfl_sync(0xffffffffu, F[k], min(lead + j, 31));
+            acc[k] = (j == 0) ? v * w.gw[0] : acc[k] + v * w.gw[j];
+        }
+    }
+    if (act && gp == 0) {
+#if GPM_EXACT
+#pragma unroll
+        for (int k = 0; k < 4; k++) acc[k] = plus_zero(acc[k]);
+#endif
+        st_cell((dir == 0 ? a.fx : a.fy) + 4 * c0, Cell{acc[0], acc[1], acc[2], acc[3]});
+    }
 }
 
 // The Riemann solve and quadrature a face function uses; the batched form has
@@ -635,21 +649,15 @@ static void launch_flux_xy(const StageArgs& a, const GpWeights& w, cudaStream_t 
 }
 #endif
 
-template <int DIR, int NGP>
-void launch_flux_dir(const StageArgs& a, const GpWeights& w, cudaStream_t s) {
-    const int nl = DIR == 0 ? a.g.lf + 1 : a.g.lf;
-    const int nn = DIR == 0 ? a.g.nf : a.g.nf + 1;
-    const dim3 grid((nl + TX - 1) / TX, (nn + TY - 1) / TY), blk(TX, TY);
-    if (!a.uniform_order) k_flux_tile<DIR, NGP, 0><<<grid, blk, 0, s>>>(a, w);
-    else if (a.g.mord == 5) k_flux_tile<DIR, NGP, 5><<<grid, blk, 0, s>>>(a, w);
-    else if (a.g.mord == 3) k_flux_tile<DIR, NGP, 3><<<grid, blk, 0, s>>>(a, w);
-    else k_flux_tile<DIR, NGP, 1><<<grid, blk, 0, s>>>(a, w);
-}
-
 template <int NGP>
 void launch_flux_ngp(const StageArgs& a, const GpWeights& w, cudaStream_t s) {
-    launch_flux_dir<0, NGP>(a, w, s);
-    launch_flux_dir<1, NGP>(a, w, s);
+    constexpr int FPW = 32 / NGP;
+    const long long nfx = (long long)(a.g.lf + 1) * a.g.nf, nfy = (long long)a.g.lf * (a.g.nf + 1);
+    const unsigned grid = (unsigned)(((nfx + FPW - 1) / FPW + (nfy + FPW - 1) / FPW + 3) / 4);
+    if (!a.uniform_order) k_flux_gp<NGP, 0><<<grid, 128, 0, s>>>(a, w);
+    else if (a.g.mord == 5) k_flux_gp<NGP, 5><<<grid, 128, 0, s>>>(a, w);
+    else if (a.g.mord == 3) k_flux_gp<NGP, 3><<<grid, 128, 0, s>>>(a, w);
+    else k_flux_gp<NGP, 1><<<grid, 128, 0, s>>>(a, w);
 }
 
 int launch_flux_all(const StageArgs& a, const GpWeights& w, cudaStream_t s) {
@@ -670,7 +678,7 @@ int launch_flux_all(const StageArgs& a, const GpWeights& w, cudaStream_t s) {
     case 4: launch_flux_ngp<4>(a, w, s); break;
     default: launch_flux_ngp<5>(a, w, s); break;
     }
-    return 2;
+    return 1;
 }
 
 // ---------------------------------------------------------------------------
