@@ -14,12 +14,66 @@
 
 #include <stddef.h>
 
+#include <memory>
+#include <mutex>
 #include <new>
 
 #include "../../include/gpmood.h"
 #include "gpm_common.h"
 #include "nn_gate.h"
 #include "nn_ref.h"
+
+// One device block of a destroyed adjoint recording, kept for the context's
+// next one (a recording's cudaMalloc and cudaFree calls were 1.5 ms of a 9 ms
+// gradient at 128^2).  Recordings share it with their context, so that either
+// may go first: it is freed with the context, and a recording that outlives
+// the context frees its own block.
+struct AdjPool {
+    std::mutex mu;
+    bool open = true;
+    void* block = nullptr;
+    size_t bytes = 0;
+
+    void* take(size_t need, size_t* got) {  // a kept block of at most twice the need, or a new one
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (block && bytes >= need && bytes / 2 <= need) {
+                void* p = block;
+                *got = bytes;
+                block = nullptr;
+                return p;
+            }
+        }
+        void* p = nullptr;
+        *got = need;
+        if (cudaMalloc(&p, need) == cudaSuccess) return p;
+        cudaGetLastError();
+        give(nullptr, 0);  // the kept block may be what is missing
+        return cudaMalloc(&p, need) == cudaSuccess ? p : nullptr;
+    }
+    void give(void* p, size_t n) {  // keep p in place of what was kept
+        void* old;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (!open) {
+                old = p;
+            } else {
+                old = block;
+                block = p;
+                bytes = n;
+            }
+        }
+        cudaFree(old);
+    }
+    void close() {
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            open = false;
+        }
+        cudaFree(block);
+        block = nullptr;
+    }
+};
 
 struct gpmood_ctx {
     gpmood_params p;
@@ -65,6 +119,7 @@ struct gpmood_ctx {
     cudaEvent_t ev[GPM_MAXST][4]; // per RK stage: flux, update, MOOD loop boundaries
     int flux_nl[GPM_MAXST];       // first-pass face launches of each RK stage
     gpmood_timing tm;
+    std::shared_ptr<AdjPool> adj_pool;
     char err[512];
 };
 
@@ -438,6 +493,7 @@ int validate(const gpmood_params* p, char* why, size_t n) {
 
 void free_all(gpmood_ctx* c) {
     if (!c) return;
+    if (c->adj_pool) c->adj_pool->close();
     cudaFree(c->dU); cudaFree(c->dUr); cudaFree(c->dU1); cudaFree(c->dU2);
     cudaFree(c->dFx); cudaFree(c->dFy); cudaFree(c->dOrder); cudaFree(c->dStamp);
     cudaFree(c->dList[0]); cudaFree(c->dList[1]); cudaFree(c->dTests); cudaFree(c->dSc); cudaFree(c->dStageOrd);
@@ -493,6 +549,7 @@ int gpmood_create(const gpmood_params* p, gpmood_ctx** out) {
     c = new (std::nothrow) gpmood_ctx();
     if (!c) return fail(nullptr, GPMOOD_E_ARG, "out of host memory");
     c->p = *p;
+    c->adj_pool = std::make_shared<AdjPool>();
     c->cc = p->method == GPMOOD_NN_GP_MOOD_CC;
     if (c->cc) {  // the reference's network with its convex-combination reconstruction
         c->p.method = GPMOOD_NN_GP_MOOD;
@@ -1100,6 +1157,9 @@ struct gpmood_adjoint {
     double* dSeg;                // 3*every+1 stage inputs of one segment
     double *dLam, *dLamB, *dTA, *dAcc, *dTmp, *dMu, *dFace;
     DevScalars* dStepSc;         // per step: t, dt, dt/dx, dt/dy of the recording
+    std::shared_ptr<AdjPool> pool;
+    void* block;                 // the device memory of all of the above
+    size_t bytes;
 };
 
 namespace {
@@ -1159,9 +1219,7 @@ void adj_free(gpmood_adjoint* a) {
     if (!a) return;
     delete[] a->t;
     delete[] a->dt;
-    cudaFree(a->dOrd); cudaFree(a->dCk); cudaFree(a->dSeg);
-    cudaFree(a->dLam); cudaFree(a->dLamB); cudaFree(a->dTA); cudaFree(a->dAcc); cudaFree(a->dTmp);
-    cudaFree(a->dMu); cudaFree(a->dFace); cudaFree(a->dStepSc);
+    if (a->block) a->pool->give(a->block, a->bytes);  // every call on a recording has waited for its work
     delete a;
 }
 
@@ -1187,24 +1245,36 @@ int gpmood_adj_record(gpmood_ctx* c, int nsteps, int every, gpmood_adjoint** out
     a->dt = new (std::nothrow) double[nsteps];
     const size_t sb = state_bytes(c);
     bool ok = a->t && a->dt;
-#define AALLOC(ptr, bytes) ok = ok && cudaMalloc((void**)&(ptr), (bytes)) == cudaSuccess
-    AALLOC(a->dOrd, (size_t)nsteps * 3 * c->ncell);
-    AALLOC(a->dCk, (size_t)a->nck * sb);
-    AALLOC(a->dSeg, (size_t)(3 * every + 1) * sb);
-    AALLOC(a->dLam, sb);
-    AALLOC(a->dLamB, sb);
-    AALLOC(a->dTA, sb);
-    AALLOC(a->dAcc, sb);
-    AALLOC(a->dTmp, sb);
-    AALLOC(a->dMu, sb);
-    AALLOC(a->dFace, 2 * c->ncell * 8 * GPM_MAXGP * sizeof(double));
-    AALLOC(a->dStepSc, (size_t)nsteps * sizeof(DevScalars));
-#undef AALLOC
-    if (ok) {  // adjoint buffers keep zero ghosts for their whole life
-        cudaStream_t s = c->stream;
-        ok = cudaMemsetAsync(a->dLam, 0, sb, s) == cudaSuccess && cudaMemsetAsync(a->dLamB, 0, sb, s) == cudaSuccess &&
-             cudaMemsetAsync(a->dTA, 0, sb, s) == cudaSuccess && cudaMemsetAsync(a->dAcc, 0, sb, s) == cudaSuccess &&
-             cudaMemsetAsync(a->dTmp, 0, sb, s) == cudaSuccess && cudaStreamSynchronize(s) == cudaSuccess;
+    a->pool = c->adj_pool;
+    if (ok) {
+        size_t need = 0;
+        auto place = [&](size_t bytes) {
+            const size_t at = need;
+            need += (bytes + 255) & ~(size_t)255;
+            return at;
+        };
+        // adjoint buffers first: their ghosts are zero for their whole life
+        const size_t lam = place(sb), lamb = place(sb), ta = place(sb), acc = place(sb), tmp = place(sb), zeroed = need;
+        const size_t mu = place(sb), ck = place((size_t)a->nck * sb), seg = place((size_t)(3 * every + 1) * sb);
+        const size_t face = place(2 * c->ncell * 8 * GPM_MAXGP * sizeof(double));
+        const size_t ssc = place((size_t)nsteps * sizeof(DevScalars)), ord = place((size_t)nsteps * 3 * c->ncell);
+        char* b = static_cast<char*>(a->pool->take(need, &a->bytes));
+        a->block = b;
+        ok = b != nullptr;
+        if (ok) {
+            a->dLam = reinterpret_cast<double*>(b + lam);
+            a->dLamB = reinterpret_cast<double*>(b + lamb);
+            a->dTA = reinterpret_cast<double*>(b + ta);
+            a->dAcc = reinterpret_cast<double*>(b + acc);
+            a->dTmp = reinterpret_cast<double*>(b + tmp);
+            a->dMu = reinterpret_cast<double*>(b + mu);
+            a->dCk = reinterpret_cast<double*>(b + ck);
+            a->dSeg = reinterpret_cast<double*>(b + seg);
+            a->dFace = reinterpret_cast<double*>(b + face);
+            a->dStepSc = reinterpret_cast<DevScalars*>(b + ssc);
+            a->dOrd = reinterpret_cast<int8_t*>(b + ord);
+            ok = cudaMemsetAsync(b, 0, zeroed, c->stream) == cudaSuccess;
+        }
     }
     if (!ok) {
         adj_free(a);
@@ -1238,7 +1308,8 @@ int gpmood_adj_record(gpmood_ctx* c, int nsteps, int every, gpmood_adjoint** out
         hs[s].qx = a->dt[s] / c->g.dx;  // the division of k_dt_finalize
         hs[s].qy = a->dt[s] / c->g.dy;
     }
-    const cudaError_t es = cudaMemcpy(a->dStepSc, hs, (size_t)done * sizeof(DevScalars), cudaMemcpyHostToDevice);
+    cudaError_t es = cudaMemcpyAsync(a->dStepSc, hs, (size_t)done * sizeof(DevScalars), cudaMemcpyHostToDevice, c->stream);
+    if (es == cudaSuccess) es = cudaStreamSynchronize(c->stream);
     delete[] hs;
     if (es != cudaSuccess) { adj_free(a); return fail(c, GPMOOD_E_CUDA, "adjoint scalars: %s", cudaGetErrorString(es)); }
     a->nsteps = done;
