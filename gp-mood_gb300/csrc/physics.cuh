@@ -55,6 +55,25 @@ __device__ __forceinline__ bool le_zero_or_nan(double x) {
     return (__double_as_longlong(x) <= 0LL) || is_nan(x);
 }
 
+__device__ __forceinline__ unsigned long long bits_of(double x) { return (unsigned long long)__double_as_longlong(x); }
+
+// A double's bits as an integer whose signed order is the double's order
+// (negative values have their magnitude bits flipped); its own inverse.
+__device__ __forceinline__ long long ord_key(double x) {
+    const long long b = __double_as_longlong(x);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+__device__ __forceinline__ double key_val(long long k) {
+    return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL));
+}
+
+// Comparisons of doubles that are not NaN on the integer pipe (an FP64 compare,
+// minimum or maximum costs an FP64 instruction): the same result, except that
+// a minimum of zeros of both signs is -0 and a maximum +0.
+__device__ __forceinline__ bool negative(double x) { return bits_of(x) > 0x8000000000000000ULL; }  // x < 0
+__device__ __forceinline__ double key_min(double a, double b) { return ord_key(b) < ord_key(a) ? b : a; }
+__device__ __forceinline__ double key_max(double a, double b) { return ord_key(b) > ord_key(a) ? b : a; }
+
 // pressure(u), physics.f90:132-143: (y-1)*(E - 0.5*(mx^2+my^2)/rho)
 __device__ __forceinline__ double pressure(const Cell& u) {
     return (GPM_GAMMA - 1.) * (u.e - (0.5 * (u.mx * u.mx + u.my * u.my) / u.r));
@@ -190,14 +209,14 @@ template <int DIR>
 __device__ __forceinline__ void hllc(const double* ul, const double* ur, double* F) {
     const Prim L = c2p<DIR>(ul);
     const Prim R = c2p<DIR>(ur);
-    const double SL = fmin(L.vn - L.c, R.vn - R.c);
-    const double SR = fmax(L.vn + L.c, R.vn + R.c);
     if (!(L.adm && R.adm)) {  // :166
         const double bad = 1. / (R.vx - R.vx);
         F[0] = F[1] = F[2] = F[3] = bad;
         return;
     }
-    if (SL >= 0.) {
+    const double SL = key_min(L.vn - L.c, R.vn - R.c);
+    const double SR = key_max(L.vn + L.c, R.vn + R.c);
+    if (!negative(SL)) {
         phys_flux<DIR>(ul, L, F);
         return;
     }
@@ -206,8 +225,8 @@ __device__ __forceinline__ void hllc(const double* ul, const double* ur, double*
     uStar = (R.p - L.p) + uStar;
     const double aL = ul[0] * numerL, aR = ur[0] * numerR;
     uStar = uStar / (aL - aR);
-    const bool left = (SL < 0.) && (uStar >= 0.);
-    const bool right = (uStar < 0.) && (SR >= 0.);
+    const bool left = !negative(uStar);
+    const bool right = !left && !negative(SR);
     if (!left && !right) {
         phys_flux<DIR>(ur, R, F);
         return;
@@ -228,8 +247,6 @@ __device__ __forceinline__ void hllc(const double* ul, const double* ur, double*
     for (int k = 0; k < 4; k++) F[k] = Fk[k] + S * (st[k] * dStar - u[k]);
 }
 #else
-__device__ __forceinline__ unsigned long long bits_of(double x) { return (unsigned long long)__double_as_longlong(x); }
-
 // Fast mode: HLLC in 60 FP64 instructions and no branch.  The FP64 pipe bounds
 // every caller (an instruction costs an SM 16-19 cycles, an integer one half a
 // cycle), so the flux is arranged for few FP64 instructions:
@@ -360,14 +377,14 @@ __device__ __forceinline__ void phys_flux_dyn(const double* u, const Prim& s, in
 
 __device__ __forceinline__ void hllc_join(const double* ul, const double* ur, const Prim& L, const Prim& R, int dir,
                                           double* F) {
-    const double SL = fmin(L.vn - L.c, R.vn - R.c);
-    const double SR = fmax(L.vn + L.c, R.vn + R.c);
     if (!(L.adm && R.adm)) {
         const double bad = 1. / (R.vx - R.vx);
         F[0] = F[1] = F[2] = F[3] = bad;
         return;
     }
-    if (SL >= 0.) {
+    const double SL = key_min(L.vn - L.c, R.vn - R.c);
+    const double SR = key_max(L.vn + L.c, R.vn + R.c);
+    if (!negative(SL)) {
         phys_flux_dyn(ul, L, dir, F);
         return;
     }
@@ -376,8 +393,8 @@ __device__ __forceinline__ void hllc_join(const double* ul, const double* ur, co
     uStar = (R.p - L.p) + uStar;
     const double aL = ul[0] * numerL, aR = ur[0] * numerR;
     uStar = uStar / (aL - aR);
-    const bool left = (SL < 0.) && (uStar >= 0.);
-    const bool right = (uStar < 0.) && (SR >= 0.);
+    const bool left = !negative(uStar);
+    const bool right = !left && !negative(SR);
     if (!left && !right) {
         phys_flux_dyn(ur, R, dir, F);
         return;
@@ -683,16 +700,6 @@ __device__ __forceinline__ int mood_uout_part(const Cell& uo, const double* __re
     return ((uo.r > mx) || (uo.r < mn)) ? 2 : 0;        // :70
 }
 #else
-// A double's bits as an integer whose signed order is the double's order
-// (negative values have their magnitude bits flipped); its own inverse.
-__device__ __forceinline__ long long ord_key(double x) {
-    const long long b = __double_as_longlong(x);
-    return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
-}
-__device__ __forceinline__ double key_val(long long k) {
-    return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL));
-}
-
 // Fast mode: the same tests in ~9 FP64-pipe instructions instead of ~24 (each
 // double min, max and compare is one).  For rho > 0, p > 0 iff
 // rho*E - (mx^2 + my^2)/2 > 0, so positivity needs no reciprocal; the DMP

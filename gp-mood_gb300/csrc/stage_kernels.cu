@@ -55,6 +55,18 @@ __device__ __forceinline__ size_t cidx(const GridGeom& g, int l, int n) {
     return (size_t)(n + 3) * (size_t)g.nx + (size_t)(l + 3);
 }
 
+static int sm_count() {
+    static std::atomic<int> sms[GPM_MAX_DEVICES];
+    const int dev = gpm_device();
+    int n = sms[dev].load(std::memory_order_relaxed);
+    if (!n) {
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        if (n <= 0) n = 1;
+        sms[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 // ---------------------------------------------------------------------------
 // Boundary_C, BC.f90:10-421.  Pass 1 fills the ghost columns of interior rows,
 // pass 2 the ghost rows of every column (so corners come from pass 1 values,
@@ -358,9 +370,9 @@ __device__ __forceinline__ void face_global(const GridGeom& g, const GpWeights& 
 // those faces (done by the low-edge tiles themselves, or by a launch of their
 // own, they were 20 us of dependent FP64 at the end of a 256^2 first pass).
 //
-// R = 4 rows, 128 threads, five CTAs an SM keep some CTAs in the FP64 phase
-// while others are in the integer phase (2048^2 Sedov step at order 5: 11.3 ms;
-// four CTAs 12.6, 32 x 8 tiles two to an SM 13.5).
+// Several small CTAs an SM keep some in the FP64 phase while others are in the
+// integer phase, and hide its latency: 2048^2 Sedov, order 5, 2 steps: 20.3 ms
+// with five of 4 rows, 24.5 with four, 19.6 with three of 8 rows.
 constexpr int XT = 32, XY = 8;  // cells per tile of the batched form; XT is also the width here
 constexpr int TW = XT + 6;      // tile width with halo: 3 cells below, 3 above
 
@@ -509,8 +521,9 @@ __device__ __forceinline__ void edge_faces(const GridGeom& g, const GpWeights& w
     }
 }
 
-// CTAs an SM should hold: 20 warps at 102 registers a thread.
-constexpr int xy_ctas(int R) { return 20 / R; }
+// CTAs an SM should hold: five of 4 rows (20 warps at 96 registers a thread),
+// three of 8 (24 warps at 80).
+constexpr int xy_ctas(int R) { return R == 8 ? 3 : 20 / R; }
 
 // The tile of a block: the edge blocks come first (one per row of tiles for
 // the x faces, one per column for the y faces), then one per tile, x fastest.
@@ -645,7 +658,11 @@ static void launch_flux_xy_t(const StageArgs& a, const GpWeights& w, cudaStream_
 
 template <int ORD, int NGP>
 static void launch_flux_xy(const StageArgs& a, const GpWeights& w, cudaStream_t s) {
-    launch_flux_xy_t<ORD, NGP, 4>(a, w, s);
+    // 8-row tiles do less work twice and run 24 warps an SM for 20, but in coarser pieces: 2048^2 (36 waves of
+    // them) 20.3 -> 19.6 ms per 2 steps, 701x499 (3 waves) 1.23 -> 1.25, 397x203 radius 1 1.08 -> 1.21.
+    const long long tiles8 = (long long)((a.g.lf + XT - 1) / XT) * ((a.g.nf + 7) / 8);
+    if (tiles8 >= 8LL * xy_ctas(8) * sm_count()) launch_flux_xy_t<ORD, NGP, 8>(a, w, s);
+    else launch_flux_xy_t<ORD, NGP, 4>(a, w, s);
 }
 #endif
 
@@ -1898,18 +1915,6 @@ __global__ void __launch_bounds__(EDGE_T) kb_flux_edge(BatchArgs a) {
     }
 }
 #endif
-
-static int sm_count() {
-    static std::atomic<int> sms[GPM_MAX_DEVICES];
-    const int dev = gpm_device();
-    int n = sms[dev].load(std::memory_order_relaxed);
-    if (!n) {
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 1;
-        sms[dev].store(n, std::memory_order_relaxed);
-    }
-    return n;
-}
 
 template <int TXB, int TYB, int NGP>
 static void blaunch_flux_t(const BatchArgs& a, cudaStream_t s) {
