@@ -34,6 +34,7 @@ struct gpmood_batch {
     int8_t* order = nullptr;
     unsigned* stamp = nullptr;
     int2* list[2] = {nullptr, nullptr};
+    unsigned char* tests = nullptr;
     int* ntrb = nullptr;
     int* hntrb = nullptr;  // pinned
     GridBar* bar = nullptr;
@@ -101,6 +102,7 @@ BatchArgs make_args(gpmood_batch* b, const double* uin, double* uout, int stage)
     a.stamp = b->stamp;
     a.tlist[0] = b->list[0];
     a.tlist[1] = b->list[1];
+    a.tests = b->tests;
     a.ntrb = b->ntrb;
     a.ftiles = b->ftiles[b->tile];
     a.nftiles = b->nft[b->tile];
@@ -182,7 +184,7 @@ void free_batch(gpmood_batch* b) {
         if (b->graph[par]) cudaGraphExecDestroy(b->graph[par]);
     cudaFree(b->dprob); cudaFree(b->dwtab); cudaFree(b->dsc);
     cudaFree(b->U); cudaFree(b->Ur); cudaFree(b->U1); cudaFree(b->U2); cudaFree(b->Fx); cudaFree(b->Fy);
-    cudaFree(b->order); cudaFree(b->stamp); cudaFree(b->list[0]); cudaFree(b->list[1]);
+    cudaFree(b->order); cudaFree(b->stamp); cudaFree(b->list[0]); cudaFree(b->list[1]); cudaFree(b->tests);
     cudaFree(b->ntrb); cudaFree(b->bar); cudaFree(b->cblocks); cudaFree(b->pblocks);
     for (int k = 0; k < GPM_NTILES; k++) cudaFree(b->ftiles[k]);
     cudaFree(b->etiles);
@@ -311,6 +313,7 @@ int gpmood_batch_create(const gpmood_params* p, int nprob, const int* lf, const 
     BALLOC(b->stamp, (size_t)b->ncell * sizeof(unsigned));
     BALLOC(b->list[0], (size_t)b->ninterior * sizeof(int2));
     BALLOC(b->list[1], (size_t)b->ninterior * sizeof(int2));
+    BALLOC(b->tests, (size_t)b->ncell * 4);
     BALLOC(b->ntrb, 8 * sizeof(int));
     BALLOC(b->bar, sizeof(GridBar));
     BALLOC(b->cblocks, sizeof(int2) * cb.size());

@@ -39,6 +39,7 @@ struct BatchArgs {
     int8_t* order;
     unsigned* stamp;
     int2* tlist[2];
+    unsigned char* tests; // 4 bytes per cell: results of the Uin-only DETECTION tests in a MOOD pass
     int* ntrb;            // [0..1] list counts, [2] pass epoch, [3] cap flag, [4] detected, [5] passes,
                           // [6] NaN or inadmissible state left in an order-1 cell (sticky)
     const int4* ftiles;
@@ -68,10 +69,6 @@ struct BatchTable {
     void (*bc)(const BatchArgs& a, double* u, cudaStream_t s);
     void (*flux)(const BatchArgs& a, cudaStream_t s);
     void (*update)(const BatchArgs& a, cudaStream_t s);
-    // one MOOD pass that reads the list count on the device and returns at
-    // once when it is zero (so a fixed number of passes can be captured)
-    void (*mood_pass)(const BatchArgs& a, int cur, cudaStream_t s);
-    void (*leftover)(const BatchArgs& a, int cur, cudaStream_t s);
     void (*combine)(const BatchArgs& a, const double* x, double* y, double ca, double cb, int with_cfl,
                     cudaStream_t s);
     void (*cfl)(const BatchArgs& a, const double* u, cudaStream_t s);

@@ -682,6 +682,13 @@ __global__ void __launch_bounds__(THREADS) k_train(const float* __restrict__ p, 
     }
 }
 
+// The accumulators of a mini-batch (one launch for two memsets).
+__global__ void k_clear_grad(float* __restrict__ grad, float* __restrict__ loss) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < NN_GATE_NPARAMS) grad[i] = 0.f;
+    if (i == 0) *loss = 0.f;
+}
+
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ gr, float* __restrict__ m, float* __restrict__ v,
                        float lr_t, float beta1, float beta2, float eps) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -787,8 +794,7 @@ int nn_forward(const float* params, const float* x, int n, float* logits, cudaSt
 
 int nn_loss_grad(const float* params, const float* x, const float* y, int n, float pos_weight, float* grad, float* loss,
                  cudaStream_t s) {
-    if (cudaMemsetAsync(grad, 0, sizeof(float) * NN_GATE_NPARAMS, s) != cudaSuccess) return -1;
-    if (cudaMemsetAsync(loss, 0, sizeof(float), s) != cudaSuccess) return -1;
+    k_clear_grad<<<(NN_GATE_NPARAMS + 255) / 256, 256, 0, s>>>(grad, loss);
     return train_launch(params, x, y, n, pos_weight, grad, loss, 0, nullptr, s);
 }
 

@@ -2003,9 +2003,6 @@ void blaunch_update(const BatchArgs& a, cudaStream_t s) {
     kb_update<<<grid, 256, 0, s>>>(a);
 }
 
-// One MOOD pass over every problem's list: cascade, the troubled cells' faces,
-// then their 5-point crosses.  Each kernel returns at once on an empty list,
-// so a captured graph holds a fixed number of passes at almost no cost.
 // Face i of the batch's face list at Gauss point gp (face_phase_gp item).
 __device__ __forceinline__ void kb_face_gp(const BatchArgs& a, int cur, int nt, int i, int gp, FaceGp& f) {
     int dir, side;
@@ -2022,73 +2019,6 @@ __device__ __forceinline__ void kb_face_gp(const BatchArgs& a, int cur, int nt, 
     const size_t c = (size_t)e.y;
     if (dir == 0) face_gp_any<0, EnsMath>(sa, w, side == 0 ? c - 1 : c, gp, f);
     else face_gp_any<1, EnsMath>(sa, w, side == 0 ? c - sa.g.nx : c, gp, f);
-}
-
-__global__ void kb_mood_mark(BatchArgs a, int cur) {  // the listed cells' orders are already lowered
-    const int nt = a.ntrb[cur];
-    if (nt == 0) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        a.ntrb[cur ^ 1] = 0;
-        a.ntrb[2] += 1;  // pass epoch for the de-duplication stamps
-    }
-}
-
-template <int NGP>
-__global__ void __launch_bounds__(128) kb_mood_faces(BatchArgs a, int cur) {
-    const int nt = a.ntrb[cur];
-    face_phase_gp<NGP>(4 * nt, 2 * nt, pack_tid(), gridDim.x * blockDim.x,
-                       [&](int i, int gp, FaceGp& f) { kb_face_gp(a, cur, nt, i, gp, f); });
-}
-
-__global__ void __launch_bounds__(256) kb_mood_cells(BatchArgs a, int cur) {
-    const int nt = a.ntrb[cur];
-    if (nt == 0) return;
-    const unsigned epoch = (unsigned)a.ntrb[2];
-    const int nxt = cur ^ 1;
-    const int total = 5 * nt;
-    const int stride = gridDim.x * blockDim.x;
-    const int lim = ((total + stride - 1) / stride) * stride;
-    const int st = pack_tid();
-    for (int base = 0; base < lim; base += stride) {
-        const int i = base + st;
-        bool trb = false;
-        int2 val = make_int2(0, 0);
-        if (i < total) {
-            const int2 e = a.tlist[cur][i / 5];
-            const BProb P = a.prob[e.x];
-            const GridGeom g = bgeom(a, P);
-            const size_t t = (size_t)e.y;
-            const int k = i % 5;
-            const size_t c = k == 0 ? t - g.nx : k == 1 ? t - 1 : k == 2 ? t : k == 3 ? t + 1 : t + g.nx;
-            const int l = (int)(c % (size_t)g.nx) - 3, n = (int)(c / (size_t)g.nx) - 3;
-            if (l >= 1 && l <= g.lf && n >= 1 && n <= g.nf &&
-                atomicExch(&a.stamp[P.off + (long long)c], epoch) != epoch) {
-                const double* ub = a.uin + 4 * P.off;
-                const Cell uo = cell_update(g, ub, a.fx + 4 * P.off, a.fy + 4 * P.off, c, a.sc[e.x].qx, a.sc[e.x].qy);
-                st_cell(a.uout + 4 * (P.off + (long long)c), uo);
-                if (a.order[P.off + (long long)c] > 1)
-                    trb = mood_troubled(uo, ub + 4 * c, g.nx, g, a.wtab[P.wc].d2x, a.wtab[P.wc].d2y);
-                else if (inadmissible(uo))
-                    atomicOr(&a.ntrb[6], 1);
-                val = make_int2(e.x, (int)c);
-            }
-        }
-        if (trb) cascade_order(a.order + a.prob[val.x].off + val.y);
-        list_append2(trb, a.tlist[nxt], &a.ntrb[nxt], val);
-    }
-}
-
-void blaunch_mood_pass(const BatchArgs& a, int cur, cudaStream_t s) {
-    const int g = sm_count() * 4;
-    kb_mood_mark<<<g, 256, 0, s>>>(a, cur);
-    switch (a.ngp) {
-    case 1: kb_mood_faces<1><<<g, 128, 0, s>>>(a, cur); break;
-    case 2: kb_mood_faces<2><<<g, 128, 0, s>>>(a, cur); break;
-    case 3: kb_mood_faces<3><<<g, 128, 0, s>>>(a, cur); break;
-    case 4: kb_mood_faces<4><<<g, 128, 0, s>>>(a, cur); break;
-    default: kb_mood_faces<5><<<g, 128, 0, s>>>(a, cur); break;
-    }
-    kb_mood_cells<<<g, 256, 0, s>>>(a, cur);
 }
 
 // The batch's whole MOOD loop in one cooperative launch (see k_mood_loop):
@@ -2123,9 +2053,26 @@ __global__ void __launch_bounds__(MOOD_THREADS, 1) kb_mood_loop(BatchArgs a, Gri
         }
         face_phase_gp<NGP>(4 * nt, 2 * nt, stid, wstride,
                            [&](int i, int gp, FaceGp& f) { kb_face_gp(a, cur, nt, i, gp, f); });
+        // the crosses' Uin-only tests beside the faces, on the warps after theirs (k_mood_loop's cut: behind the
+        // update they were ~150 FP64 instructions in a row, a pass of all SMs 45k cycles for 26k)
+        const int total = 5 * nt, chunks = (total + 31) / 32, nwarp = wstride >> 5;
+        constexpr int FPW = 32 / NGP;
+        const int first = 2 * ((2 * nt + FPW - 1) / FPW) % nwarp;
+        for (int task = ((stid >> 5) + nwarp - first) % nwarp; task < 4 * chunks; task += nwarp) {
+            const int t = task & 3, i = (task >> 2) * 32 + (threadIdx.x & 31);
+            int c;
+            if (i < total) {
+                const int2 e = a.tlist[cur][i / 5];
+                const BProb P = a.prob[e.x];
+                const GridGeom g = bgeom(a, P);
+                if (cross_cell(g, e.y, i % 5, &c))
+                    __stcg(a.tests + 4 * (P.off + c) + t,
+                           (unsigned char)cross_test(g, a.wtab[P.wc], a.uin + 4 * (P.off + c), t));
+            }
+        }
         if (!mood_sync(bar, wait, solo)) return;
         const unsigned epoch = (unsigned)*(volatile int*)&a.ntrb[2];
-        const int nxt = cur ^ 1, total = 5 * nt;
+        const int nxt = cur ^ 1;
         const int lim = ((total + wstride - 1) / wstride) * wstride;
         for (int base = 0; base < lim; base += wstride) {
             const int i = base + stid;
@@ -2135,21 +2082,20 @@ __global__ void __launch_bounds__(MOOD_THREADS, 1) kb_mood_loop(BatchArgs a, Gri
                 const int2 e = a.tlist[cur][i / 5];
                 const BProb P = a.prob[e.x];
                 const GridGeom g = bgeom(a, P);
-                const size_t t = (size_t)e.y;
-                const int k = i % 5;
-                const size_t c = k == 0 ? t - g.nx : k == 1 ? t - 1 : k == 2 ? t : k == 3 ? t + 1 : t + g.nx;
-                const int l = (int)(c % (size_t)g.nx) - 3, n = (int)(c / (size_t)g.nx) - 3;
-                if (l >= 1 && l <= g.lf && n >= 1 && n <= g.nf &&
-                    atomicExch(&a.stamp[P.off + (long long)c], epoch) != epoch) {
+                int c;
+                if (cross_cell(g, e.y, i % 5, &c) && atomicExch(&a.stamp[P.off + c], epoch) != epoch) {
                     const double* ub = a.uin + 4 * P.off;
-                    const Cell uo =
-                        cell_update(g, ub, a.fx + 4 * P.off, a.fy + 4 * P.off, c, a.sc[e.x].qx, a.sc[e.x].qy);
-                    st_cell(a.uout + 4 * (P.off + (long long)c), uo);
-                    if (a.order[P.off + (long long)c] > 1)
-                        trb = mood_troubled(uo, ub + 4 * c, g.nx, g, a.wtab[P.wc].d2x, a.wtab[P.wc].d2y);
-                    else if (inadmissible(uo))
+                    const Cell uo = cell_update(g, ub, a.fx + 4 * P.off, a.fy + 4 * P.off, (size_t)c, a.sc[e.x].qx,
+                                                a.sc[e.x].qy);
+                    st_cell(a.uout + 4 * (P.off + c), uo);
+                    if (a.order[P.off + c] > 1) {
+                        const int r = mood_uout_part(uo, ub + 4 * (size_t)c, g.nx, g);
+                        const unsigned f = __ldcg(reinterpret_cast<const unsigned*>(a.tests) + P.off + c);
+                        trb = r == 1 || (r == 2 && (f & 0x101) == 0x101 && !(g.u2 && (f & 0x1010000)));
+                    } else if (inadmissible(uo)) {
                         atomicOr(&a.ntrb[6], 1);
-                    val = make_int2(e.x, (int)c);
+                    }
+                    val = make_int2(e.x, c);
                 }
             }
             if (trb) cascade_order(a.order + a.prob[val.x].off + val.y);
@@ -2193,12 +2139,6 @@ int blaunch_mood_loop(const BatchArgs& a, GridBar* bar, int max_pass, cudaStream
     default: return blaunch_mood_loop_n<5>(a, bar, max_pass, s);
     }
 }
-
-// After the last captured pass: a non-empty list means the stage hit the cap.
-__global__ void kb_leftover(BatchArgs a, int cur) {
-    if (a.ntrb[cur] != 0) a.ntrb[3] = 1;
-}
-void blaunch_leftover(const BatchArgs& a, int cur, cudaStream_t s) { kb_leftover<<<1, 1, 0, s>>>(a, cur); }
 
 // Per-problem CFL minimum: every block of padded cells belongs to one problem.
 __device__ __forceinline__ void bdt_reduce(double v, BScal* sc) {
@@ -2279,8 +2219,7 @@ void blaunch_advance_t(const BatchArgs& a, cudaStream_t s) { kb_advance_t<<<(a.n
 
 void batch_set_max_nx(int nx) { g_max_nx = nx; }
 
-const BatchTable batch_table = {blaunch_bc,      blaunch_flux,        blaunch_update,    blaunch_mood_pass,
-                                blaunch_leftover, blaunch_combine,     blaunch_cfl,       blaunch_dt_finalize,
-                                blaunch_advance_t, blaunch_mood_loop};
+const BatchTable batch_table = {blaunch_bc,  blaunch_flux,        blaunch_update,    blaunch_combine,
+                                blaunch_cfl, blaunch_dt_finalize, blaunch_advance_t, blaunch_mood_loop};
 
 }  // namespace GPM_NS
