@@ -1169,10 +1169,12 @@ __device__ __forceinline__ void team_faces(const StageArgs& a, const GpWeights& 
     const int lane = threadIdx.x & 31, fl = lane / LPF, j = lane - fl * LPF, gp = j >> 1, side = j & 1;
     const int base = lane - j, i = task * FPW + fl;
     const bool act = fl < FPW && i < 4 * nt;
-    int dir = 0, sd = 0, lcell = 0;
-    if (act) lcell = *(volatile const int*)(lst + face_item(i, nt, &dir, &sd));
+    int dir, sd;
+    // idle lanes repeat the warp's last face: another face's order would cost the
+    // warp that order's sums too (one at order 5: 52 instructions, 3.3k cycles)
+    const int lcell = *(volatile const int*)(lst + face_item(min(task * FPW + min(fl, FPW - 1), 4 * nt - 1), nt, &dir, &sd));
     const size_t step = dir == 0 ? (size_t)1 : (size_t)g.nx;
-    const size_t c0 = act ? (size_t)lcell - (sd == 0 ? step : 0) : cidx(g, 1, 1);  // idle lanes: any valid face
+    const size_t c0 = (size_t)lcell - (sd == 0 ? step : 0);
     const size_t cs = c0 + (side ? step : 0);                                     // this lane's cell
     const int face = dir == 0 ? (side ? 0 : 2) : (side ? 3 : 1);
     const ptrdiff_t row = g.nx;
