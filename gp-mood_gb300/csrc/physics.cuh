@@ -685,19 +685,10 @@ __device__ __forceinline__ bool inadmissible(const Cell& uo) {
 // reference's decision.  uin points at Uin(1, l, n) of a padded array of row
 // pitch 4*nx doubles.
 #if GPM_EXACT
-__device__ __forceinline__ int mood_uout_part(const Cell& uo, const double* __restrict__ uin, int nx,
-                                              const GridGeom& g) {
-    if (le_zero_or_nan(uo.r)) return 1;
-    const double p = pressure(uo);
-    if (le_zero_or_nan(p)) return 1;
-    if (!g.dmp) return 0;
-    const size_t row = (size_t)4 * nx;
-    const double c = __ldg(uin), l = __ldg(uin - 4), r = __ldg(uin + 4), b = __ldg(uin - row), t = __ldg(uin + row);
-    const double mn = fmin(fmin(fmin(fmin(c, l), b), t), r);
-    const double mx = fmax(fmax(fmax(fmax(c, l), b), t), r);
-    const double Mm = mx - mn;
-    if (!(Mm > g.dx * g.dx * g.dx)) return 0;          // plateau, :68
-    return ((uo.r > mx) || (uo.r < mn)) ? 2 : 0;        // :70
+using Bound = double;
+__device__ __forceinline__ Bound bound_key(double r) { return r; }
+__device__ __forceinline__ bool mood_positive(const Cell& uo) {
+    return !le_zero_or_nan(uo.r) && !le_zero_or_nan(pressure(uo));
 }
 #else
 // Fast mode: the same tests in ~9 FP64-pipe instructions instead of ~24 (each
@@ -707,23 +698,41 @@ __device__ __forceinline__ int mood_uout_part(const Cell& uo, const double* __re
 // bound test compares keys.  The decisions are the exact form's except where
 // p is within rounding of 0, or a density of Uin is NaN (which fmin/fmax
 // would skip).
-__device__ __forceinline__ int mood_uout_part(const Cell& uo, const double* __restrict__ uin, int nx,
-                                              const GridGeom& g) {
-    if (le_zero_or_nan(uo.r)) return 1;
+using Bound = long long;
+__device__ __forceinline__ Bound bound_key(double r) { return ord_key(r); }
+__device__ __forceinline__ bool mood_positive(const Cell& uo) {
     const double ke2 = uo.mx * uo.mx + uo.my * uo.my;
-    if (!(uo.r * uo.e - 0.5 * ke2 > 0.)) return 1;     // p <= 0 or NaN
-    if (!g.dmp) return 0;
-    const size_t row = (size_t)4 * nx;
-    const long long c = ord_key(__ldg(uin)), l = ord_key(__ldg(uin - 4)), r = ord_key(__ldg(uin + 4));
-    const long long b = ord_key(__ldg(uin - row)), t = ord_key(__ldg(uin + row));
-    const long long mn = llmin(llmin(llmin(llmin(c, l), b), t), r);
-    const long long mx = llmax(llmax(llmax(llmax(c, l), b), t), r);
-    const double Mm = key_val(mx) - key_val(mn);
-    if (!(Mm > g.dx * g.dx * g.dx)) return 0;          // plateau, :68
-    const long long k = ord_key(uo.r);
-    return (k > mx || k < mn) ? 2 : 0;                 // :70
+    return !le_zero_or_nan(uo.r) && uo.r * uo.e - 0.5 * ke2 > 0.;  // p <= 0 or NaN: false
 }
 #endif
+
+// The DMP bounds of a cell; false on a plateau (:68), where nothing is out of bounds.
+__device__ __forceinline__ bool mood_bounds(const double* __restrict__ uin, int nx, const GridGeom& g, Bound* lo,
+                                            Bound* hi) {
+    const size_t row = (size_t)4 * nx;
+#if GPM_EXACT
+    const double c = __ldg(uin), l = __ldg(uin - 4), r = __ldg(uin + 4), b = __ldg(uin - row), t = __ldg(uin + row);
+    *lo = fmin(fmin(fmin(fmin(c, l), b), t), r);
+    *hi = fmax(fmax(fmax(fmax(c, l), b), t), r);
+    const double Mm = *hi - *lo;
+#else
+    const long long c = ord_key(__ldg(uin)), l = ord_key(__ldg(uin - 4)), r = ord_key(__ldg(uin + 4));
+    const long long b = ord_key(__ldg(uin - row)), t = ord_key(__ldg(uin + row));
+    *lo = llmin(llmin(llmin(llmin(c, l), b), t), r);
+    *hi = llmax(llmax(llmax(llmax(c, l), b), t), r);
+    const double Mm = key_val(*hi) - key_val(*lo);
+#endif
+    return Mm > g.dx * g.dx * g.dx;
+}
+
+__device__ __forceinline__ int mood_uout_part(const Cell& uo, const double* __restrict__ uin, int nx,
+                                              const GridGeom& g) {
+    if (!mood_positive(uo)) return 1;
+    Bound lo, hi;
+    if (!g.dmp || !mood_bounds(uin, nx, g, &lo, &hi)) return 0;
+    const Bound k = bound_key(uo.r);
+    return (k > hi || k < lo) ? 2 : 0;  // :70
+}
 
 __device__ __forceinline__ bool mood_shock_part(const double* __restrict__ uin, int nx, const GridGeom& g) {
     const size_t row = (size_t)4 * nx;

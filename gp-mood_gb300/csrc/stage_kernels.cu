@@ -1123,10 +1123,11 @@ __device__ __forceinline__ bool mood_sync(GridBar* b, GridWait& w, bool solo) {
 //    side's state and its primitive quantities; they swap them by shuffles,
 //    both run the Riemann join, and the face's lanes sum the quadrature, one
 //    variable a lane (~70 instructions in a row for ~112 on one lane);
-//  * the tests of the crosses that read only Uin (the shock detector's halves,
-//    U2 in x and in y) run beside the faces on warps of their own, so that
-//    after the barrier only the update, positivity and the density bounds are
-//    left, one lane a cross cell.
+//  * what a cross needs of Uin alone (the shock detector's halves, U2 in x and
+//    in y; in the team also the density bounds and which list entry takes a
+//    shared cell) runs beside the faces on warps of its own, so that after the
+//    barrier only the update, positivity and two comparisons are left, one lane
+//    a cross cell or, for up to TEAM_QUAD of them, one a variable.
 // Passes over more than GridGeom::mood_solo cells run on all SMs with grid
 // barriers (k_mood_loop).  Shorter ones run on one thread-block cluster (the
 // "team", k_mood_team) with cluster barriers (~1k cycles with what they wait for, against ~4k):
@@ -1137,11 +1138,17 @@ __device__ __forceinline__ bool mood_sync(GridBar* b, GridWait& w, bool solo) {
 constexpr int TEAM = 8;                  // CTAs of the cluster
 constexpr int TEAM_CROSS = 512;          // cross cells whose tests run beside the faces (one per thread of CTA 0)
 constexpr int TEAM_LIST_CAP = 1024;
+// Up to here a cross cell is updated by four lanes (4 FP64 instructions in a row
+// for 16, the tests after it on every lane): at most two warps per SM quarter.
+constexpr int TEAM_QUAD = 64;
 
 struct TeamSmem {
     int list[2][TEAM_LIST_CAP];
     int count[2];                        // the team's count: appended to in CTA 0, then copied to every member
     bool flag[4][TEAM_CROSS];            // shock flow half, pressure-jump half, U2 smooth in x, in y
+    int cross[TEAM_CROSS];               // the cross cell; -1: outside, or another entry's
+    Bound lo[TEAM_CROSS], hi[TEAM_CROSS];  // its density bounds; lo > hi: none
+    alignas(16) double F[MOOD_THREADS / 32][16][4];  // a warp's fluxes at its Gauss points, for the quadrature
     double z3[4][GPM_MAXGP][5];          // order-3 weights, read by lanes of mixed faces and Gauss points
     double z1[4][GPM_MAXGP];             // order 1
 };
@@ -1162,7 +1169,7 @@ __device__ __forceinline__ bool cross_test(const GridGeom& g, const GpWeights& w
 
 // Warp task `task` of the 4*nt faces of the listed cells.
 template <int NGP>
-__device__ __forceinline__ void team_faces(const StageArgs& a, const GpWeights& w, const TeamSmem& sm, const int* lst,
+__device__ __forceinline__ void team_faces(const StageArgs& a, const GpWeights& w, TeamSmem& sm, const int* lst,
                                            int nt, int task) {
     constexpr int LPF = 2 * NGP, FPW = 32 / LPF;  // lanes per face, faces per warp
     const GridGeom& g = a.g;
@@ -1242,17 +1249,16 @@ __device__ __forceinline__ void team_faces(const StageArgs& a, const GpWeights& 
         else riemann<1>(g.num_flux, ul, ur, F);
     }
     // quadrature (quad_flux's expression): variable k on lane k of the face; two rounds of two with one Gauss point
+    double(*Fw)[4] = sm.F[threadIdx.x >> 5];
+    __syncwarp();
+    if (side == 0) st_cell(&Fw[lane >> 1][0], Cell{F[0], F[1], F[2], F[3]});
+    __syncwarp();
 #pragma unroll
     for (int k0 = 0; k0 < 4; k0 += (LPF < 4 ? LPF : 4)) {
         double acc = 0.;
 #pragma unroll
         for (int gg = 0; gg < NGP; gg++) {
-            double x = 0.;
-#pragma unroll
-            for (int k = 0; k < (LPF < 4 ? LPF : 4); k++) {
-                const double y = __shfl_sync(0xffffffffu, F[k0 + k], min(base + 2 * gg, 31));
-                if (j == k) x = y;
-            }
+            const double x = Fw[min((base >> 1) + gg, 15)][(k0 + j) & 3];
             acc = gg == 0 ? x * w.gw[0] : acc + x * w.gw[gg];
         }
 #if GPM_EXACT
@@ -1294,32 +1300,88 @@ __device__ __forceinline__ bool cross_update(const StageArgs& a, const GpWeights
     return trb;
 }
 
-// The crosses of a team pass, by CTA 0.  A cross cell that several listed cells
-// share is taken by the first of them (a scan of a short list), or by whoever
-// stamps it first.
-__device__ __forceinline__ void team_cells(const StageArgs& a, const GpWeights& w, TeamSmem& sm, const int* lst,
-                                           int cur, int nt, unsigned pid, double qx, double qy) {
+// What a team pass needs of cross i before the fluxes: its cell, if this entry
+// takes it, and the density bounds.  A cross cell that several listed cells share
+// is taken by the first of them (a scan of a short list), or by whoever stamps
+// it first.
+__device__ __forceinline__ bool team_own(const StageArgs& a, const int* lst, int nt, int i, unsigned pid, int* c) {
+    const int q = i / 5, nx = a.g.nx;
+    if (!cross_cell(a.g, lst[q], i - 5 * q, c)) return false;
+    if (nt > 24) return atomicExch(&a.stamp[*c], pid) != pid;
+    bool own = true;
+    for (int q2 = 0; q2 < q; q2++) {
+        const int d = *c - lst[q2];
+        if (d == 0 || d == 1 || d == -1 || d == nx || d == -nx) own = false;
+    }
+    return own;
+}
+__device__ __forceinline__ void team_prepare(const StageArgs& a, TeamSmem* sm0, const int* lst, int nt, int i,
+                                             unsigned pid) {
+    int c;
+    const bool own = team_own(a, lst, nt, i, pid, &c);
+    sm0->cross[i] = own ? c : -1;
+    if (!own) return;
+    Bound lo = 0, hi = 0;
+    const bool dmp = a.g.dmp && mood_bounds(a.uin + 4 * (size_t)c, a.g.nx, a.g, &lo, &hi);
+    sm0->lo[i] = dmp ? lo : (Bound)1;
+    sm0->hi[i] = dmp ? hi : (Bound)0;
+}
+
+// cross_update of a prepared cross i by L lanes (1 or 4, this one's variable k);
+// all return the same.
+template <int L>
+__device__ __forceinline__ bool cross_finish(const StageArgs& a, const TeamSmem& sm, int i, int k, double qx,
+                                             double qy) {
     const GridGeom& g = a.g;
-    const int nxt = cur ^ 1, total = 5 * nt, lane = threadIdx.x & 31, nx = g.nx;
-    for (int i0 = (int)threadIdx.x - lane; i0 < total; i0 += MOOD_THREADS) {
-        const int i = i0 + lane, q = i / 5;
+    const int c = sm.cross[i], o = (int)__ldcg(a.order + c);
+    Cell uo;
+    if (L == 4) {  // cell_update's sum for variable k
+        const size_t at = 4 * (size_t)c + k, row = 4 * (size_t)g.nx;
+        const double fb = __ldcg(a.fy + at - row), fl = __ldcg(a.fx + at - 4);
+        const double fr = __ldcg(a.fx + at), ft = __ldcg(a.fy + at);
+        double x = __ldg(a.uin + at);
+        x = x + qy * fb;
+        x = x + qx * fl;
+        x = x - qx * fr;
+        x = x - qy * ft;
+        a.uout[at] = x;
+        const unsigned m = 0xfu << (threadIdx.x & 28);
+        uo.r = __shfl_sync(m, x, 0, 4);
+        uo.mx = __shfl_sync(m, x, 1, 4);
+        uo.my = __shfl_sync(m, x, 2, 4);
+        uo.e = __shfl_sync(m, x, 3, 4);
+    } else {
+        uo = cell_update(g, a.uin, a.fx, a.fy, (size_t)c, qx, qy);
+        st_cell(a.uout + 4 * (size_t)c, uo);
+    }
+    if (o <= 1) {
+        if (inadmissible(uo)) atomicOr(&a.sc->status, GPM_STATUS_NAN);
+        return false;
+    }
+    bool trb = !mood_positive(uo);
+    const Bound key = bound_key(uo.r);
+    if (!trb && sm.lo[i] <= sm.hi[i] && (key > sm.hi[i] || key < sm.lo[i]))
+        trb = sm.flag[0][i] && sm.flag[1][i] && !(g.u2 && (sm.flag[2][i] || sm.flag[3][i]));
+    if (trb && k == 0) __stcg(a.order + c, (int8_t)(o == 3 ? 1 : 3));  // the cascade of cascade_order
+    return trb;
+}
+
+// The crosses of a team pass, by CTA 0; those from ncross on were not prepared.
+__device__ __forceinline__ void team_cells(const StageArgs& a, const GpWeights& w, TeamSmem& sm, const int* lst,
+                                           int cur, int nt, int ncross, unsigned pid, double qx, double qy) {
+    const int nxt = cur ^ 1, total = 5 * nt, lane = threadIdx.x & 31;
+    const int quad = total <= TEAM_QUAD && ncross == total ? 2 : 0;  // log2 of the lanes per cell
+    for (int i0 = (int)threadIdx.x - lane; i0 < total << quad; i0 += MOOD_THREADS) {
+        const int i = (i0 + lane) >> quad, k = quad ? lane & 3 : 0;
         bool trb = false;
         int c = 0;
-        if (i < total && cross_cell(g, lst[q], i - 5 * q, &c)) {
-            bool own = true;
-            if (nt <= 24) {
-                for (int q2 = 0; q2 < q; q2++) {
-                    const int d = c - lst[q2];
-                    if (d == 0 || d == 1 || d == -1 || d == nx || d == -nx) own = false;
-                }
-            } else {
-                own = atomicExch(&a.stamp[c], pid) != pid;
-            }
-            const int flags = g.solo_split && i < TEAM_CROSS
-                                  ? sm.flag[0][i] | sm.flag[1][i] << 1 | sm.flag[2][i] << 2 | sm.flag[3][i] << 3
-                                  : -1;
-            if (own) trb = cross_update(a, w, c, flags, qx, qy);
+        if (i < ncross) {
+            c = sm.cross[i];
+            if (c >= 0) trb = quad ? cross_finish<4>(a, sm, i, k, qx, qy) : cross_finish<1>(a, sm, i, k, qx, qy);
+        } else if (i < total && team_own(a, lst, nt, i, pid, &c)) {
+            trb = cross_update(a, w, c, -1, qx, qy);
         }
+        trb = trb && k == 0;
         // warp-aggregated append to the next list, of every member and global
         const unsigned m = __ballot_sync(0xffffffffu, trb);
         if (m) {
@@ -1442,18 +1504,21 @@ __global__ void __launch_bounds__(MOOD_THREADS, 1) k_mood_team(StageArgs a, cons
             const int* lst = nt <= TEAM_LIST_CAP ? sm.list[cur] : a.tlist[cur];
             const int nface = (4 * nt + FPW - 1) / FPW, ncross = a.g.solo_split ? min(5 * nt, TEAM_CROSS) : 0;
             const int chunks = (ncross + 31) / 32;
-            for (int task = warp * TEAM + rank; task < nface + 4 * chunks; task += (MOOD_THREADS / 32) * TEAM) {
+            for (int task = warp * TEAM + rank; task < nface + 5 * chunks; task += (MOOD_THREADS / 32) * TEAM) {
                 if (task < nface) {
                     team_faces<NGP>(a, w, sm, lst, nt, task);
                 } else {
-                    const int t = (task - nface) & 3, i = ((task - nface) >> 2) * 32 + lane;
+                    const int t = (task - nface) % 5, i = (task - nface) / 5 * 32 + lane;
                     int c;
-                    if (i < ncross && cross_cell(a.g, lst[i / 5], i % 5, &c))
+                    if (t == 4) {
+                        if (i < ncross) team_prepare(a, sm0, lst, nt, i, epoch + (unsigned)pass);
+                    } else if (i < ncross && cross_cell(a.g, lst[i / 5], i % 5, &c)) {
                         sm0->flag[t][i] = cross_test(a.g, w, a.uin + 4 * (size_t)c, t);
+                    }
                 }
             }
             team_sync();
-            if (rank == 0) team_cells(a, w, sm, lst, cur, nt, epoch + (unsigned)pass, qx, qy);
+            if (rank == 0) team_cells(a, w, sm, lst, cur, nt, ncross, epoch + (unsigned)pass, qx, qy);
             team_sync();
             cur ^= 1;
             nt = *(volatile int*)&sm.count[cur];
