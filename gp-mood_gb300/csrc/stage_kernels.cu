@@ -2118,23 +2118,27 @@ __global__ void __launch_bounds__(MOOD_THREADS, 1) kb_mood_loop(BatchArgs a, Gri
             a.ntrb[2] += 1;       // stamp epoch, read after the next barrier
             a.ntrb[4] += nt;
         }
+        const int total = 5 * nt;
         face_phase_gp<NGP>(4 * nt, 2 * nt, stid, wstride,
                            [&](int i, int gp, FaceGp& f) { kb_face_gp(a, cur, nt, i, gp, f); });
-        // the crosses' Uin-only tests beside the faces, on the warps after theirs (k_mood_loop's cut: behind the
-        // update they were ~150 FP64 instructions in a row, a pass of all SMs 45k cycles for 26k)
-        const int total = 5 * nt, chunks = (total + 31) / 32, nwarp = wstride >> 5;
-        constexpr int FPW = 32 / NGP;
-        const int first = 2 * ((2 * nt + FPW - 1) / FPW) % nwarp;
-        for (int task = ((stid >> 5) + nwarp - first) % nwarp; task < 4 * chunks; task += nwarp) {
-            const int t = task & 3, i = (task >> 2) * 32 + (threadIdx.x & 31);
-            int c;
-            if (i < total) {
-                const int2 e = a.tlist[cur][i / 5];
-                const BProb P = a.prob[e.x];
-                const GridGeom g = bgeom(a, P);
-                if (cross_cell(g, e.y, i % 5, &c))
-                    __stcg(a.tests + 4 * (P.off + c) + t,
-                           (unsigned char)cross_test(g, a.wtab[P.wc], a.uin + 4 * (P.off + c), t));
+        if (solo) {
+            // The crosses' Uin-only tests beside the faces, on the warps after theirs.  On a long list
+            // they stay behind the update, for the few cells that need them: 48 problems, 3 steps, the loop's
+            // nine launches take 6.87 ms with all tests behind it, 7.13 with all beside the faces, 6.51 so.
+            constexpr int FPW = 32 / NGP;
+            const int chunks = (total + 31) / 32, nwarp = wstride >> 5;
+            const int first = 2 * ((2 * nt + FPW - 1) / FPW) % nwarp;
+            for (int task = ((stid >> 5) + nwarp - first) % nwarp; task < 4 * chunks; task += nwarp) {
+                const int t = task & 3, i = (task >> 2) * 32 + (threadIdx.x & 31);
+                int c;
+                if (i < total) {
+                    const int2 e = a.tlist[cur][i / 5];
+                    const BProb P = a.prob[e.x];
+                    const GridGeom g = bgeom(a, P);
+                    if (cross_cell(g, e.y, i % 5, &c))
+                        __stcg(a.tests + 4 * (P.off + c) + t,
+                               (unsigned char)cross_test(g, a.wtab[P.wc], a.uin + 4 * (P.off + c), t));
+                }
             }
         }
         if (!mood_sync(bar, wait, solo)) return;
@@ -2156,9 +2160,13 @@ __global__ void __launch_bounds__(MOOD_THREADS, 1) kb_mood_loop(BatchArgs a, Gri
                                                 a.sc[e.x].qy);
                     st_cell(a.uout + 4 * (P.off + c), uo);
                     if (a.order[P.off + c] > 1) {
-                        const int r = mood_uout_part(uo, ub + 4 * (size_t)c, g.nx, g);
-                        const unsigned f = __ldcg(reinterpret_cast<const unsigned*>(a.tests) + P.off + c);
-                        trb = r == 1 || (r == 2 && (f & 0x101) == 0x101 && !(g.u2 && (f & 0x1010000)));
+                        const int r = solo ? mood_uout_part(uo, ub + 4 * (size_t)c, g.nx, g) : 0;
+                        if (r == 2) {
+                            const unsigned f = __ldcg(reinterpret_cast<const unsigned*>(a.tests) + P.off + c);
+                            trb = (f & 0x101) == 0x101 && !(g.u2 && (f & 0x1010000));
+                        } else {
+                            trb = solo ? r == 1 : mood_troubled(uo, ub + 4 * (size_t)c, g.nx, g, a.wtab[P.wc].d2x, a.wtab[P.wc].d2y);
+                        }
                     } else if (inadmissible(uo)) {
                         atomicOr(&a.ntrb[6], 1);
                     }
