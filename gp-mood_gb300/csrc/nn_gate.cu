@@ -54,16 +54,40 @@ __device__ __forceinline__ uint32_t ld32(const __nv_bfloat16* p) { return *reint
 __device__ __forceinline__ int cx_(int j) { return j == 1 ? -1 : j == 2 ? 1 : j == 5 ? -2 : j == 6 ? 2 : 0; }
 __device__ __forceinline__ int cy_(int j) { return j == 3 ? -1 : j == 4 ? 1 : j == 7 ? -2 : j == 8 ? 2 : 0; }
 
+// (float)d in integer instructions: cvt.f32.f64 runs on the FP64 pipe, 64
+// cycles a warp on its SM quarter, and a cell has 36 of them.  Exact for zeros and
+// for results that are normal floats or infinities rounded up to; `other` is set
+// for the rest (subnormal results, larger values, infinities, NaN).
+__device__ __forceinline__ float narrow(double d, bool* other) {
+    const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+    const unsigned mag = hi & 0x7fffffffu, e = mag >> 20;
+    const unsigned f = ((mag - (896u << 20)) << 3) | (lo >> 29);
+    const unsigned r = f + (((lo & 0x1fffffffu) + 0x0fffffffu + (f & 1u)) >> 29);  // to nearest, ties to even
+    const bool zero = (mag | lo) == 0;
+    if (!zero && e - 897u > 253u) *other = true;
+    return __uint_as_float((hi & 0x80000000u) | (zero ? 0u : r));
+}
+
 // Features of interior cell (l, n); returns true when every variable is
 // constant over the stencil (max - min < 1e-10 in FP32, mod_append_NN_dataset.f90:101).
 __device__ bool cell_features(const GridGeom& g, const double* __restrict__ u, int l, int n, float* x) {
     float q[4][9];
+    bool other = false;
 #pragma unroll
     for (int j = 0; j < 9; j++) {
         const size_t c = (size_t)(n + cy_(j) + 3) * g.nx + (size_t)(l + cx_(j) + 3);
         const double2 a = __ldg(reinterpret_cast<const double2*>(u + 4 * c));
         const double2 b = __ldg(reinterpret_cast<const double2*>(u + 4 * c) + 1);
-        q[0][j] = (float)a.x; q[1][j] = (float)a.y; q[2][j] = (float)b.x; q[3][j] = (float)b.y;
+        q[0][j] = narrow(a.x, &other); q[1][j] = narrow(a.y, &other);
+        q[2][j] = narrow(b.x, &other); q[3][j] = narrow(b.y, &other);
+    }
+    if (other) {
+#pragma unroll
+        for (int j = 0; j < 9; j++) {
+            const double* c = u + 4 * ((size_t)(n + cy_(j) + 3) * g.nx + (size_t)(l + cx_(j) + 3));
+#pragma unroll
+            for (int v = 0; v < 4; v++) q[v][j] = (float)__ldg(c + v);
+        }
     }
     bool cst = true;
 #pragma unroll
@@ -192,13 +216,15 @@ constexpr uint32_t TC_IDESC =        // kind::f16: D F32, A and B BF16, both K-m
 struct __align__(1024) SmemTc {
     unsigned char w0[64 * 48 * 2];    // B of layer 0: 8 row groups x 6 k-chunks
     unsigned char w1[64 * 64 * 2];    // B of layer 1: 8 x 8
-    unsigned char x[128 * 48 * 2];    // A of layer 0: 16 x 6
+    float b0[64], b1[64], w2[64], b2[4];  // up to here the image that k_gate_image makes
+    __align__(128) unsigned char x[128 * 48 * 2];  // A of layer 0: 16 x 6
     unsigned char h[128 * 64 * 2];    // A of layer 1: 16 x 8
-    float b0[64], b1[64], w2[64];
     unsigned long long mbar;
     uint32_t tmem;
 };
 static_assert(sizeof(SmemTc) <= TC_SMEM, "gate shared memory");
+constexpr int TC_IMAGE = 64 * 48 * 2 + 64 * 64 * 2 + (3 * 64 + 4) * 4;  // bytes of a CTA's weights
+static_assert(offsetof(SmemTc, b2) + 16 == TC_IMAGE && TC_IMAGE % 16 == 0, "weights first, whole 16-byte words");
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -279,28 +305,41 @@ __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.a
 __device__ __forceinline__ void tc_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// The gate's weights as a CTA holds them: BF16 in the K-major core-matrix
+// layout, then the FP32 vectors.  Made once per set of parameters; each CTA
+// converting them for itself took 56 scalar loads a thread, most of
+// the 25.6 us of a 512x128 gate (10.5 us with the copy and `narrow`).
+__global__ void __launch_bounds__(256) k_gate_image(const float* __restrict__ p, unsigned char* __restrict__ image) {
+    SmemTc& s = *reinterpret_cast<SmemTc*>(image);
+    const int tid = threadIdx.x;
+    for (int i = tid; i < 64 * 48; i += 256) {
+        const int o = i / 48, k = i % 48;
+        *reinterpret_cast<__nv_bfloat16*>(s.w0 + core_off(o, k, 6)) =
+            __float2bfloat16_rn(k < 36 ? p[P_W0 + o * 36 + k] : 0.f);
+    }
+    for (int i = tid; i < 64 * 64; i += 256)
+        *reinterpret_cast<__nv_bfloat16*>(s.w1 + core_off(i / 64, i % 64, 8)) = __float2bfloat16_rn(p[P_W1 + i]);
+    if (tid < 64) {
+        s.b0[tid] = p[P_B0 + tid];
+        s.b1[tid] = p[P_B1 + tid];
+        s.w2[tid] = bf16r(p[P_W2 + tid]);
+    }
+    if (tid < 4) s.b2[tid] = p[P_B2];
+}
+
 __global__ void __launch_bounds__(TC_THREADS) k_gate(GridGeom g, const double* __restrict__ u,
-                                                  const float* __restrict__ p, float thr, int8_t* __restrict__ order,
+                                                  const unsigned char* __restrict__ image, float thr,
+                                                  int8_t* __restrict__ order,
                                                   unsigned long long* __restrict__ count, int* __restrict__ list,
                                                   int* __restrict__ list_count, float* __restrict__ logits,
                                                   int* __restrict__ status, int wait_limit) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     SmemTc& s = *reinterpret_cast<SmemTc*>(smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // weights, BF16, in the K-major core-matrix layout
-    for (int i = tid; i < 64 * 48; i += TC_THREADS) {
-        const int o = i / 48, k = i % 48;
-        *reinterpret_cast<__nv_bfloat16*>(s.w0 + core_off(o, k, 6)) =
-            __float2bfloat16_rn(k < 36 ? p[P_W0 + o * 36 + k] : 0.f);
-    }
-    for (int i = tid; i < 64 * 64; i += TC_THREADS)
-        *reinterpret_cast<__nv_bfloat16*>(s.w1 + core_off(i / 64, i % 64, 8)) = __float2bfloat16_rn(p[P_W1 + i]);
-    for (int i = tid; i < 64; i += TC_THREADS) {
-        s.b0[i] = p[P_B0 + i];
-        s.b1[i] = p[P_B1 + i];
-        s.w2[i] = bf16r(p[P_W2 + i]);
-    }
-    const float b2 = p[P_B2];
+    for (int i = tid; i < TC_IMAGE / 16; i += TC_THREADS)  // lands during the first tile's features
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_raw) + 16 * i),
+                     "l"(reinterpret_cast<const char*>(image) + 16 * i)
+                     : "memory");
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s.tmem)),
                      "r"(TC_COLS));
@@ -344,6 +383,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_gate(GridGeom g, const double* _
                 *reinterpret_cast<uint4*>(s.x + core_off(tid, 8 * kc, 6)) = make_uint4(w[0], w[1], w[2], w[3]);
             }
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");
         fence_async_smem();
         if (__syncthreads_and(c)) {  // every stencil constant: nothing to gate
             if (logits && row < ncells) logits[row] = 0.f;
@@ -407,7 +447,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_gate(GridGeom g, const double* _
                 z += bf16r(fmaxf(d[j] + s.b1[o], 0.f)) * s.w2[o];
             }
         }
-        z += b2;
+        z += s.b2[0];
         bool fire = false;
         int cidx = 0;
         if (row < ncells) {
@@ -705,6 +745,7 @@ __global__ void k_adam(float* __restrict__ p, const float* __restrict__ gr, floa
 
 struct NnGate {
     float* params;
+    unsigned char* image;  // params as k_gate_image lays them out (in params' allocation)
     float thr;
     bool loaded;
     int wait_limit;  // polls of the MMA waits before a timeout (0: ~1 s); a test hook
@@ -713,10 +754,12 @@ struct NnGate {
 NnGate* nn_gate_create(const GridGeom&) {
     NnGate* n = new (std::nothrow) NnGate();
     if (!n) return nullptr;
-    if (cudaMalloc(&n->params, sizeof(float) * NN_GATE_NPARAMS) != cudaSuccess) {
+    constexpr size_t at = (sizeof(float) * NN_GATE_NPARAMS + 255) / 256 * 256;
+    if (cudaMalloc(&n->params, at + TC_IMAGE) != cudaSuccess) {
         delete n;
         return nullptr;
     }
+    n->image = reinterpret_cast<unsigned char*>(n->params) + at;
     n->thr = 0.f;
     n->loaded = false;
     return n;
@@ -731,6 +774,8 @@ void nn_gate_destroy(NnGate* n) {
 int nn_gate_set(NnGate* n, const float* params, cudaStream_t s) {
     if (cudaMemcpyAsync(n->params, params, sizeof(float) * NN_GATE_NPARAMS, cudaMemcpyHostToDevice, s) != cudaSuccess)
         return -1;
+    k_gate_image<<<1, 256, 0, s>>>(n->params, n->image);
+    if (cudaGetLastError() != cudaSuccess) return -1;
     n->loaded = true;
     return 0;
 }
@@ -756,7 +801,7 @@ int nn_gate_orders(NnGate* n, const GridGeom& g, const double* uin, int8_t* orde
     }
     // persistent: 4 CTAs per SM, each holding 128 of the SM's 512 TMEM columns
     const int blocks = (int)(tiles < 4LL * nsm ? tiles : 4LL * nsm);
-    k_gate<<<blocks, TC_THREADS, TC_SMEM, s>>>(g, uin, n->params, n->thr, order, count, list, list_count, logits,
+    k_gate<<<blocks, TC_THREADS, TC_SMEM, s>>>(g, uin, n->image, n->thr, order, count, list, list_count, logits,
                                                status, n->wait_limit);
     return cudaGetLastError() == cudaSuccess ? 1 : -1;
 }
