@@ -35,6 +35,11 @@ TMAX = 0.05
 # variables at 3 Gauss points (2*3*4*25 = 600), 3 HLLC solves (3*103 = 309)
 # and the quadrature (4*5 = 20).
 FLOPS_PER_FACE = 929
+# What the fast kernel puts on the FP64 pipe per face: 3 HLLC solves of 48
+# instructions and the quadrature's 12; its reconstruction runs in fixed point
+# on the integer pipe.  As two flops each, like the probe's FMAs: the fraction
+# of the pipe, which 929 flops would overstate.
+FP64_INSTR_PER_FACE_FAST = 156
 # Algorithmic HBM bytes per cell-update of one full SSP-RK3 step: each stage
 # reads its input (32 B) and writes its output (32 B); stages 2-3 also read U^n.
 BYTES_PER_CELL_UPDATE = 256
@@ -178,9 +183,9 @@ def measured_peaks():
 
 # DRAM bytes per face of one launch of the fast two-direction face kernel
 # (k_flux_xy_tma) on the 2048^2 Sedov first pass, from one ncu capture of this
-# workload: dram__bytes_read.sum + dram__bytes_write.sum = 136.13 MB + 208.49 MB
+# workload: dram__bytes_read.sum + dram__bytes_write.sum = 137.27 MB + 212.91 MB
 # over 8,392,704 faces.  A constant of that capture, not a live measurement.
-DRAM_BYTES_PER_FACE_NCU = 41.06
+DRAM_BYTES_PER_FACE_NCU = 41.72
 
 
 def cpu_oracle_rate(n, steps, threads):
@@ -605,15 +610,16 @@ def run_ours(args, ws, rank, local):
 
     # ---- roofline of the dominant kernel (first-pass face kernel) ----
     # one "launch" of the roofline = the first pass of one RK stage: every face
-    # of the grid (fast mode: k_flux_xy_tma + k_flux_edge; exact: the x and y kernels)
+    # of the grid (fast mode: k_flux_xy_tma; exact: k_flux_gp)
     launch_ms = tm.flux_ms / max(tm.flux_launches, 1)
     faces_per_launch = tm.flux_faces / max(tm.flux_launches, 1)
-    achieved_tflops = FLOPS_PER_FACE * faces_per_launch / (launch_ms * 1e-3) / 1e12
+    pipe_flops = 2 * FP64_INSTR_PER_FACE_FAST if fp == pkg.FP_FAST else FLOPS_PER_FACE
+    achieved_tflops = pipe_flops * faces_per_launch / (launch_ms * 1e-3) / 1e12
     peak_tflops = max(peak_fp64_gflops, peak_after_gflops) / 1e3
     tpf = DRAM_BYTES_PER_FACE_NCU if fp == pkg.FP_FAST else None  # the capture is of the fast kernel
-    kname = ("first pass of one RK stage: k_flux_xy_tma (interior, both directions, TMA-staged halo tiles) + "
-             "k_flux_edge (faces of ghost cells); GP recon + HLLC + quadrature" if fp == pkg.FP_FAST
-             else "first pass of one RK stage: k_flux_tile x and y (GP recon + HLLC + quadrature)")
+    kname = ("first pass of one RK stage: k_flux_xy_tma (both directions, TMA-staged halo tiles; GP recon in fixed "
+             "point, HLLC and quadrature in FP64)" if fp == pkg.FP_FAST
+             else "first pass of one RK stage: k_flux_gp (both directions; GP recon + HLLC + quadrature)")
     roofline = {"bound": "fp64", "kernel": kname,
                 "achieved": achieved_tflops, "peak": peak_tflops, "unit": "TFLOP/s",
                 "frac": achieved_tflops / peak_tflops,
@@ -622,7 +628,7 @@ def run_ours(args, ws, rank, local):
                                "just after the timed region, the higher reading; MEASURED_PEAKS.json has no FP64 "
                                "figure",
                 "peak_before_after": [peak_fp64_gflops / 1e3, peak_after_gflops / 1e3],
-                "flops_per_face": FLOPS_PER_FACE, "faces_per_launch": faces_per_launch,
+                "flops_per_face": pipe_flops, "algorithmic_flops_per_face": FLOPS_PER_FACE, "faces_per_launch": faces_per_launch,
                 "launch_ms": launch_ms, "share_of_step": tm.flux_ms / el_ms if el_ms else None}
     peaks = measured_peaks()
     hbm_peak = peaks.get("hbm_gbs") if peaks else 6800.0
@@ -630,7 +636,7 @@ def run_ours(args, ws, rank, local):
     roofline_hbm = {"bound": "hbm", "achieved": step_gbs, "peak": hbm_peak, "unit": "GB/s",
                     "frac": step_gbs / hbm_peak, "traffic": None,
                     "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6.8 TB/s",
-                    "note": "whole step, 256 algorithmic bytes per cell-update; the path is FP64-pipe bound"}
+                    "note": "whole step, 256 algorithmic bytes per cell-update; the path is bound by FP64 and integer issue"}
 
     forms = {}
     if args.nn:

@@ -108,7 +108,7 @@ struct GridGeom {
     int cc_col;          // NN_GP_MOOD_CC: the column l whose order-3 states are blended (-1: none)
 };
 
-// Longest troubled lists that one cluster (k_mood_loop) and one CTA (batched
+// Longest troubled lists that one cluster (k_mood_team) and one CTA (batched
 // loop) take over from all SMs; the environment variable
 // GPMOOD_MOOD_SOLO overrides both (tuning only: results do not depend on it).
 #define GPM_MOOD_TEAM_MAX 100

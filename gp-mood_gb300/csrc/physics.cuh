@@ -247,7 +247,8 @@ __device__ __forceinline__ void hllc(const double* ul, const double* ur, double*
     for (int k = 0; k < 4; k++) F[k] = Fk[k] + S * (st[k] * dStar - u[k]);
 }
 #else
-// Fast mode: HLLC in 60 FP64 instructions and no branch.  The FP64 pipe bounds
+// Fast mode: HLLC in 48 FP64 instructions and no branch (60 before the
+// reciprocals' series ran in integers, ~95 as selects over the reference's form).  The FP64 pipe bounds
 // every caller (an instruction costs an SM 16-19 cycles, an integer one half a
 // cycle), so the flux is arranged for few FP64 instructions:
 //  * the side's flux is written at the contact speed u*, F = (m, m u* + p*,
@@ -261,7 +262,8 @@ __device__ __forceinline__ void hllc(const double* ul, const double* ur, double*
 //    min(-c_L, dv - c_R) and S_R - v_R = max(c_R, c_L - dv), dv = v_R - v_L;
 //  * minima, maxima and sign tests compare bit patterns on the integer pipe
 //    (doubles of one sign order like their bits).
-// A 2048^2 first pass: 7.27 -> 6.0 ms against hllc's arithmetic with selects.
+// A 2048^2 first pass, still with FP64 reciprocals and reconstruction: 7.27 -> 6.0 ms
+// against hllc's arithmetic with selects.
 // States as (rho, normal momentum, tangential momentum, E): one side's
 // quantities, then the flux of a pair; a pair is admissible if both sides are
 // (the flux is undefined otherwise).

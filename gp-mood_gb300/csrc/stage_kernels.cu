@@ -355,7 +355,7 @@ __device__ __forceinline__ void face_global(const GridGeom& g, const GpWeights& 
 // two faces come from the mirror-symmetry components of its stencil (FixOrbit)
 // in fixed point, on the integer pipe (fixed_recon.cuh), so the FP64 pipe,
 // which bounds this kernel, runs only the Riemann solves: at order 5 with 3
-// points 192 FP64 instructions per face instead of 350 with FP64 sums.  After
+// points 156 FP64 instructions per face instead of 314 with FP64 sums.  After
 // staging, a CTA turns its tile into signed mantissas (in place) and 16-bit
 // exponents once.  Then, for x and for y: every cell's states go to shared
 // memory, its far-face (right, top) states in its own slot and its near-face
@@ -1122,7 +1122,9 @@ __device__ __forceinline__ bool mood_sync(GridBar* b, GridWait& w, bool solo) {
 //  * a face's Gauss point takes two lanes, one per side: each reconstructs its
 //    side's state and its primitive quantities; they swap them by shuffles,
 //    both run the Riemann join, and the face's lanes sum the quadrature, one
-//    variable a lane (~70 instructions in a row for ~112 on one lane);
+//    variable a lane (~70 instructions in a row for ~112 on one lane; measured
+//    in a pass of 3 cells: sums 1.9k cycles, side 1.0k, join 2.0k, quadrature 0.8k,
+//    the same through shared memory);
 //  * what a cross needs of Uin alone (the shock detector's halves, U2 in x and
 //    in y; in the team also the density bounds and which list entry takes a
 //    shared cell) runs beside the faces on warps of its own, so that after the
@@ -1134,12 +1136,14 @@ __device__ __forceinline__ bool mood_sync(GridBar* b, GridWait& w, bool solo) {
 // 8 SMs take 32 warps side by side, and CTA 0 runs the cells.  The team's lists
 // live in every member's shared memory (and in the global list, which a longer
 // one is read from), the tests' results in CTA 0's, through distributed shared
-// memory.
+// memory.  A 512x128 DMR, 30 steps, 42 ms with one-CTA passes: 22.5 ms so; 23.8
+// with 4 CTAs, 24.3 with lists of up to 160 cells here, 22.7 with up to 60.
 constexpr int TEAM = 8;                  // CTAs of the cluster
 constexpr int TEAM_CROSS = 512;          // cross cells whose tests run beside the faces (one per thread of CTA 0)
 constexpr int TEAM_LIST_CAP = 1024;
 // Up to here a cross cell is updated by four lanes (4 FP64 instructions in a row
-// for 16, the tests after it on every lane): at most two warps per SM quarter.
+// for 16, the tests after it on every lane): at most two warps per SM quarter; 128
+// is as fast.
 constexpr int TEAM_QUAD = 64;
 
 struct TeamSmem {
@@ -1148,7 +1152,6 @@ struct TeamSmem {
     bool flag[4][TEAM_CROSS];            // shock flow half, pressure-jump half, U2 smooth in x, in y
     int cross[TEAM_CROSS];               // the cross cell; -1: outside, or another entry's
     Bound lo[TEAM_CROSS], hi[TEAM_CROSS];  // its density bounds; lo > hi: none
-    alignas(16) double F[MOOD_THREADS / 32][16][4];  // a warp's fluxes at its Gauss points, for the quadrature
     double z3[4][GPM_MAXGP][5];          // order-3 weights, read by lanes of mixed faces and Gauss points
     double z1[4][GPM_MAXGP];             // order 1
 };
@@ -1169,7 +1172,7 @@ __device__ __forceinline__ bool cross_test(const GridGeom& g, const GpWeights& w
 
 // Warp task `task` of the 4*nt faces of the listed cells.
 template <int NGP>
-__device__ __forceinline__ void team_faces(const StageArgs& a, const GpWeights& w, TeamSmem& sm, const int* lst,
+__device__ __forceinline__ void team_faces(const StageArgs& a, const GpWeights& w, const TeamSmem& sm, const int* lst,
                                            int nt, int task) {
     constexpr int LPF = 2 * NGP, FPW = 32 / LPF;  // lanes per face, faces per warp
     const GridGeom& g = a.g;
@@ -1249,16 +1252,17 @@ __device__ __forceinline__ void team_faces(const StageArgs& a, const GpWeights& 
         else riemann<1>(g.num_flux, ul, ur, F);
     }
     // quadrature (quad_flux's expression): variable k on lane k of the face; two rounds of two with one Gauss point
-    double(*Fw)[4] = sm.F[threadIdx.x >> 5];
-    __syncwarp();
-    if (side == 0) st_cell(&Fw[lane >> 1][0], Cell{F[0], F[1], F[2], F[3]});
-    __syncwarp();
 #pragma unroll
     for (int k0 = 0; k0 < 4; k0 += (LPF < 4 ? LPF : 4)) {
         double acc = 0.;
 #pragma unroll
         for (int gg = 0; gg < NGP; gg++) {
-            const double x = Fw[min((base >> 1) + gg, 15)][(k0 + j) & 3];
+            double x = 0.;
+#pragma unroll
+            for (int k = 0; k < (LPF < 4 ? LPF : 4); k++) {
+                const double y = __shfl_sync(0xffffffffu, F[k0 + k], min(base + 2 * gg, 31));
+                if (j == k) x = y;
+            }
             acc = gg == 0 ? x * w.gw[0] : acc + x * w.gw[gg];
         }
 #if GPM_EXACT
