@@ -2,9 +2,9 @@
 // products, MOOD detection.  Included by stage_kernels.cu, which is compiled
 // twice: GPM_EXACT=1 with --fmad=false (every expression rounds exactly like
 // the reference's x86-64 build) and GPM_EXACT=0 with FMA contraction,
-// reciprocal reuse, Newton reciprocals and square roots from the hardware
-// approximations (fast_rcp.cuh), division-free DETECTION tests and, in the
-// first pass, an HLLC with selects instead of branches.
+// reciprocals and square roots from the hardware's approximations
+// (fast_rcp.cuh), division-free DETECTION tests and an HLLC of one formula
+// without branches.
 //
 // Reference routines: physics.f90:9-75,132-143 (Flux, c2p_local, pressure),
 // mod_HLLC.f90:11-169 (HLLC_Flux), mod_GP_MOOD.f90:58-65 (dot products),
@@ -624,7 +624,7 @@ __device__ __forceinline__ double pressure_ir(const Cell& u, double ir) {
     return (GPM_GAMMA - 1.) * (u.e - 0.5 * (u.mx * u.mx + u.my * u.my) * ir);
 }
 
-// Fast mode: the same three tests with six Newton reciprocals (gpm_fast_rcp)
+// Fast mode: the same three tests with six reciprocals (gpm_fast_rcp)
 // in place of the nineteen IEEE divisions; the quantities agree with the
 // exact form to rounding for admissible states.  A lone warp pays ~64 cycles
 // per FP64 instruction, and a short MOOD pass waits on this chain.

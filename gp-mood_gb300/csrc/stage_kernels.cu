@@ -1638,7 +1638,7 @@ __device__ __forceinline__ double cell_dt(const Cell& u, double dx, double dy) {
     return 1.0 / (1.0 / (dx / (fabs(vx) + c)) + 1.0 / (dy / (fabs(vy) + c)));
 }
 #else
-// Fast mode: dx*dy / ((|u|+c)*dy + (|v|+c)*dx) with Newton reciprocals and
+// Fast mode: dx*dy / ((|u|+c)*dy + (|v|+c)*dx) with gpm_fast_rcp and
 // the fast square root, equal to the form above up to rounding (a NaN or
 // non-positive cell still gives NaN or a non-positive value, which the
 // reduction skips).

@@ -280,11 +280,11 @@ int  gpmood_probe_fp64(double* gflops);
  * flops per half.  A mixed rate near the single ones means that the two share
  * the FP64 hardware.  Measurement only; no reference counterpart. */
 int  gpmood_probe_fp64_pipes(double* gflops3);
-/* The fast mode's reciprocal (Newton-Raphson from the hardware approximation)
+/* The fast mode's reciprocal (a series from the hardware approximation)
  * on device arrays: d_y[i] = 1/d_x[i]; for testing its accuracy. */
 int  gpmood_fast_rcp(const double* d_x, double* d_y, int n);
 /* The fast mode's square root (from the hardware's approximate reciprocal
- * square root, one coupled Newton step and a final correction) on device
+ * square root and the binomial series) on device
  * arrays: d_y[i] = sqrt(d_x[i]); for testing its accuracy. */
 int  gpmood_fast_sqrt(const double* d_x, double* d_y, int n);
 
