@@ -35,11 +35,11 @@ TMAX = 0.05
 # variables at 3 Gauss points (2*3*4*25 = 600), 3 HLLC solves (3*103 = 309)
 # and the quadrature (4*5 = 20).
 FLOPS_PER_FACE = 929
-# What the fast kernel puts on the FP64 pipe per face: 3 HLLC solves of 48
+# What the fast kernel puts on the FP64 pipe per face: 3 HLLC solves of 38
 # instructions and the quadrature's 12; its reconstruction runs in fixed point
 # on the integer pipe.  As two flops each, like the probe's FMAs: the fraction
 # of the pipe, which 929 flops would overstate.
-FP64_INSTR_PER_FACE_FAST = 156
+FP64_INSTR_PER_FACE_FAST = 126
 # Algorithmic HBM bytes per cell-update of one full SSP-RK3 step: each stage
 # reads its input (32 B) and writes its output (32 B); stages 2-3 also read U^n.
 BYTES_PER_CELL_UPDATE = 256

@@ -247,8 +247,8 @@ __device__ __forceinline__ void hllc(const double* ul, const double* ur, double*
     for (int k = 0; k < 4; k++) F[k] = Fk[k] + S * (st[k] * dStar - u[k]);
 }
 #else
-// Fast mode: HLLC in 48 FP64 instructions and no branch (60 before the
-// reciprocals' series ran in integers, ~95 as selects over the reference's form).  The FP64 pipe bounds
+// Fast mode: HLLC in 38 FP64 instructions and no branch (60 before the
+// reciprocals' and roots' series ran in integers, ~95 as selects over the reference's form).  The FP64 pipe bounds
 // every caller (an instruction costs an SM 16-19 cycles, an integer one half a
 // cycle), so the flux is arranged for few FP64 instructions:
 //  * the side's flux is written at the contact speed u*, F = (m, m u* + p*,

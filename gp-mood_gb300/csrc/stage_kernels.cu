@@ -355,7 +355,7 @@ __device__ __forceinline__ void face_global(const GridGeom& g, const GpWeights& 
 // two faces come from the mirror-symmetry components of its stencil (FixOrbit)
 // in fixed point, on the integer pipe (fixed_recon.cuh), so the FP64 pipe,
 // which bounds this kernel, runs only the Riemann solves: at order 5 with 3
-// points 156 FP64 instructions per face instead of 314 with FP64 sums.  After
+// points 126 FP64 instructions per face instead of 284 with FP64 sums.  After
 // staging, a CTA turns its tile into signed mantissas (in place) and 16-bit
 // exponents once.  Then, for x and for y: every cell's states go to shared
 // memory, its far-face (right, top) states in its own slot and its near-face
@@ -372,7 +372,8 @@ __device__ __forceinline__ void face_global(const GridGeom& g, const GpWeights& 
 //
 // Several small CTAs an SM keep some in the FP64 phase while others are in the
 // integer phase, and hide its latency: 2048^2 Sedov, order 5, 2 steps: 20.3 ms
-// with five of 4 rows, 24.5 with four, 19.6 with three of 8 rows.
+// with five of 4 rows, 24.5 with four, 19.6 with three of 8 rows (all with FP64 roots;
+// 17.4 now).
 constexpr int XT = 32, XY = 8;  // cells per tile of the batched form; XT is also the width here
 constexpr int TW = XT + 6;      // tile width with halo: 3 cells below, 3 above
 
