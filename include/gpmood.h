@@ -284,7 +284,7 @@ int  gpmood_probe_fp64_pipes(double* gflops3);
  * on device arrays: d_y[i] = 1/d_x[i]; for testing its accuracy. */
 int  gpmood_fast_rcp(const double* d_x, double* d_y, int n);
 /* The fast mode's square root (from the hardware's approximate reciprocal
- * square root and the binomial series) on device
+ * square root and the binomial series, in integers) on device
  * arrays: d_y[i] = sqrt(d_x[i]); for testing its accuracy. */
 int  gpmood_fast_sqrt(const double* d_x, double* d_y, int n);
 
