@@ -129,11 +129,12 @@ struct DevScalars {
     double t, dt, qx, qy;             // time, step, dt/dx, dt/dy
     unsigned long long detected_step; // count_detected_cell of the current step
     unsigned long long apriori_step;
+    int ntrb[2];                      // troubled-cell counts, double-buffered lists: a stage starts with both 0, as
+                                      // the start of a step and the MOOD loop's end leave them
     int status;                       // GPMOOD status bits
     int pad;                          // the fields so far are a step's own: one upload sets them (set_time)
     double tmax, cfl;
     unsigned long long dtmin_bits;    // Setdt reduction slot (bits of a positive double)
-    int ntrb[2];                      // troubled-cell counts, double-buffered lists; the MOOD loop leaves them 0
     int passes_stage[GPM_MAXST];      // MOOD passes of each RK stage of the last step (device loop)
     unsigned stamp_epoch;             // first unused pass stamp of the device MOOD loop
     int mood_cur, mood_pass;          // k_mood_loop's state for k_mood_team: the current list, the passes so far

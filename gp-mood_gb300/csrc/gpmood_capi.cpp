@@ -445,13 +445,14 @@ int run_step(gpmood_ctx* c, double* u, double* ur, bool with_cfl, bool bc_in) {
 }
 
 // Put t, dt and dt/dx, dt/dy computed on the host (IEEE, same bits) on the
-// device and clear the step's counters and flags.
+// device and clear the step's counters, list counts and flags.
 int set_time(gpmood_ctx* c, double t, double dt) {
     c->hSc->t = t;
     c->hSc->dt = dt;
     c->hSc->qx = dt / c->g.dx;
     c->hSc->qy = dt / c->g.dy;
     c->hSc->detected_step = c->hSc->apriori_step = 0;
+    c->hSc->ntrb[0] = c->hSc->ntrb[1] = 0;  // calls between steps (nn_predict, nn_gate_logits) list cells too
     c->hSc->status = 0;
     CU(cudaMemcpyAsync(c->dSc, c->hSc, offsetof(DevScalars, tmax), cudaMemcpyHostToDevice, c->stream));
     return 0;

@@ -1805,6 +1805,7 @@ __global__ void k_step_begin(GridGeom g, DevScalars* sc, double t) {
     sc->dtmin_bits = (unsigned long long)__double_as_longlong(1.0e30);
     sc->detected_step = 0;
     sc->apriori_step = 0;
+    sc->ntrb[0] = sc->ntrb[1] = 0;  // calls between steps (nn_predict, nn_gate_logits) list cells too
     sc->status = 0;
 }
 
