@@ -1487,7 +1487,10 @@ template <int NGP>
 __global__ void __launch_bounds__(MOOD_THREADS, 1) k_mood_team(StageArgs a, const __grid_constant__ GpWeights w,
                                                       const GridBar* bar, int max_pass, int stage) {
     __shared__ TeamSmem sm;
-    if (bar->err) return;  // a grid barrier ran out before: the host reports it and starts over
+    if (bar->err) {  // a grid barrier ran out: the host reports it after the step's other stages, whose lists start empty
+        if (blockIdx.x == 0 && threadIdx.x == 0) a.sc->ntrb[0] = a.sc->ntrb[1] = 0;
+        return;
+    }
     const double qx = a.sc->qx, qy = a.sc->qy;
     const unsigned epoch = a.sc->stamp_epoch;
     const int rank = (int)blockIdx.x, tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
