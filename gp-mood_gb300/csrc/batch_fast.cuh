@@ -140,9 +140,9 @@ __device__ __forceinline__ bool hllc_select(const double* ul, const double* ur, 
     uStar = (R.p - L.p) + uStar;
     const double aL = ul[0] * numerL, aR = ur[0] * numerR;
     uStar = uStar * rcp(aL - aR);
-    const bool sl_neg = negative(SL), left = sl_neg && !negative(uStar);
-    const bool right = negative(uStar) && !negative(SR);
-    const bool useL = !sl_neg || left;  // whose physical flux hllc returns or corrects
+    const bool left = negative(SL) && nonnegative(uStar);
+    const bool right = negative(uStar) && nonnegative(SR);
+    const bool useL = nonnegative(SL) || left;  // whose physical flux hllc returns or corrects
     double u[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) u[k] = useL ? ul[k] : ur[k];

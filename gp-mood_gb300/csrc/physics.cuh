@@ -67,12 +67,24 @@ __device__ __forceinline__ double key_val(long long k) {
     return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL));
 }
 
-// Comparisons of doubles that are not NaN on the integer pipe (an FP64 compare,
-// minimum or maximum costs an FP64 instruction): the same result, except that
-// a minimum of zeros of both signs is -0 and a maximum +0.
-__device__ __forceinline__ bool negative(double x) { return bits_of(x) > 0x8000000000000000ULL; }  // x < 0
-__device__ __forceinline__ double key_min(double a, double b) { return ord_key(b) < ord_key(a) ? b : a; }
-__device__ __forceinline__ double key_max(double a, double b) { return ord_key(b) > ord_key(a) ? b : a; }
+// Comparisons of arithmetic results on the integer pipe (an FP64 compare, minimum
+// or maximum costs an FP64 instruction), with the FP64 ones' answers: false for
+// NaN, and a minimum and maximum that skip a NaN as fmin and fmax do (except that
+// a minimum of zeros of both signs is -0 and a maximum +0).  An operation's NaN
+// is quiet, so the high word tells it.
+__device__ __forceinline__ bool quiet_nan(double x) { return (__double2hiint(x) & 0x7fffffff) > 0x7ff00000; }
+__device__ __forceinline__ bool negative(double x) {  // x < 0
+    return bits_of(x) > 0x8000000000000000ULL && (unsigned)__double2hiint(x) <= 0xfff00000u;
+}
+__device__ __forceinline__ bool nonnegative(double x) {  // x >= 0
+    return bits_of(x) <= 0x8000000000000000ULL && !quiet_nan(x);
+}
+__device__ __forceinline__ double key_min(double a, double b) {
+    return (ord_key(b) < ord_key(a) || quiet_nan(a)) && !quiet_nan(b) ? b : a;
+}
+__device__ __forceinline__ double key_max(double a, double b) {
+    return (ord_key(b) > ord_key(a) || quiet_nan(a)) && !quiet_nan(b) ? b : a;
+}
 
 // pressure(u), physics.f90:132-143: (y-1)*(E - 0.5*(mx^2+my^2)/rho)
 __device__ __forceinline__ double pressure(const Cell& u) {
@@ -216,7 +228,7 @@ __device__ __forceinline__ void hllc(const double* ul, const double* ur, double*
     }
     const double SL = key_min(L.vn - L.c, R.vn - R.c);
     const double SR = key_max(L.vn + L.c, R.vn + R.c);
-    if (!negative(SL)) {
+    if (nonnegative(SL)) {
         phys_flux<DIR>(ul, L, F);
         return;
     }
@@ -225,8 +237,8 @@ __device__ __forceinline__ void hllc(const double* ul, const double* ur, double*
     uStar = (R.p - L.p) + uStar;
     const double aL = ul[0] * numerL, aR = ur[0] * numerR;
     uStar = uStar / (aL - aR);
-    const bool left = !negative(uStar);
-    const bool right = !left && !negative(SR);
+    const bool left = negative(SL) && nonnegative(uStar);
+    const bool right = negative(uStar) && nonnegative(SR);
     if (!left && !right) {
         phys_flux<DIR>(ur, R, F);
         return;
@@ -386,7 +398,7 @@ __device__ __forceinline__ void hllc_join(const double* ul, const double* ur, co
     }
     const double SL = key_min(L.vn - L.c, R.vn - R.c);
     const double SR = key_max(L.vn + L.c, R.vn + R.c);
-    if (!negative(SL)) {
+    if (nonnegative(SL)) {
         phys_flux_dyn(ul, L, dir, F);
         return;
     }
@@ -395,8 +407,8 @@ __device__ __forceinline__ void hllc_join(const double* ul, const double* ur, co
     uStar = (R.p - L.p) + uStar;
     const double aL = ul[0] * numerL, aR = ur[0] * numerR;
     uStar = uStar / (aL - aR);
-    const bool left = !negative(uStar);
-    const bool right = !left && !negative(SR);
+    const bool left = negative(SL) && nonnegative(uStar);
+    const bool right = negative(uStar) && nonnegative(SR);
     if (!left && !right) {
         phys_flux_dyn(ur, R, dir, F);
         return;
