@@ -11,7 +11,9 @@
 // 1960, is evaluated on the mantissa with 8 to 10 guard bits and rounded once:
 // within 1.01 half-ulps on 4e7 samples.  ~35 integer instructions; three FP64
 // FMAs for the same series cost the 2048^2 first pass 12 of its 48 per Riemann
-// solve.  Zero, subnormal, infinite and NaN d, and |d| beyond 2^1022, give NaN.
+// solve.  From |d| = 2^1022 on, where reciprocals turn subnormal, the result is
+// the seed: 2^-1022 to its 20 bits, then a zero of d's sign.  Zero, subnormal,
+// infinite and NaN d give NaN.
 //
 // sqrt(x) in integers too: from y ~ 1/sqrt(x) (PTX rsqrt.approx.ftz.f64, low
 // word zero) the residual e = 1 - x*y^2 is exact to 2^-60 in the middle bits of
@@ -43,7 +45,8 @@ __device__ __forceinline__ double gpm_fast_rcp(double d) {
     const int s2 = 11 - __clz((int)(W >> 32));
     const unsigned long long M = (W + (1ull << (s2 - 1))) >> s2;
     const unsigned hi = (yh & 0xfff00000u) + ((unsigned)(M >> 32) - 0x100000u) + ((unsigned)(s2 - sh) << 20);
-    return ey - 1u < 2046u ? __hiloint2double((int)hi, (int)M) : __longlong_as_double(0x7ff8000000000000LL);
+    const unsigned mag = dh & 0x7fffffffu, other = mag - 0x7fd00000u < 0x200000u ? yh : 0x7ff80000u;
+    return mag - 0x100000u < 0x7fc00000u ? __hiloint2double((int)hi, (int)M) : __hiloint2double((int)other, 0);
 }
 
 __device__ __forceinline__ double gpm_fast_sqrt(double x) {
