@@ -27,8 +27,11 @@
 // next one (a recording's cudaMalloc and cudaFree calls were 1.5 ms of a 9 ms
 // gradient at 128^2).  Recordings share it with their context, so that either
 // may go first: it is freed with the context, and a recording that outlives
-// the context frees its own block.
+// the context frees its own block.  A larger block than MOST is freed at once,
+// so that no more than that is held back from other allocations: the calls are
+// under 2 % of a gradient there (256^2, 5 steps: 16.5 -> 16.8 ms).
 struct AdjPool {
+    static constexpr size_t MOST = (size_t)64 << 20;
     std::mutex mu;
     bool open = true;
     void* block = nullptr;
@@ -55,7 +58,7 @@ struct AdjPool {
         void* old;
         {
             std::lock_guard<std::mutex> lock(mu);
-            if (!open) {
+            if (!open || n > MOST) {
                 old = p;
             } else {
                 old = block;
