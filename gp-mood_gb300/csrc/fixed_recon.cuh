@@ -8,24 +8,28 @@
 // sums run on the integer pipe and FP64 is left to the Riemann solves.  Radius 1
 // (order 3, 5 points) uses the same form.
 //
-// Per variable and stencil the values share one exponent E, the largest biased
-// exponent of its cells: a double M * 2^(e-1075) becomes Q = M << 5 >> (E - e), a
-// 58-bit integer with 5 guard bits below the largest value's last place.  The
-// mirror-symmetry components (GpOrbit) are exact integer sums of up to four Q
-// (60 bits).  A weight is w * 2^58 rounded to an integer.  Both factors are
-// split as h * 2^30 + l, |l| <= 2^29, and a product keeps h*h (accumulated on
-// its own) and h*l + l*h (accumulated together); l*l, at most one unit of Q,
-// is dropped.  With sum |w| <= 4 over a state's cells (checked by the host,
-// FixOrbit::ok) neither accumulator passes 2^62 and no result 2^60.  The
-// 64-bit results, in units of 2^(E-1080), are rounded to double once.  Error:
-// at most 2^-58 of the stencil's largest binade per cell for its alignment and
-// its dropped product, and the final rounding, against one FP64 rounding per
-// multiply-add before (tests/test_fixed_recon.py measures both).
+// Per variable and stencil the values are aligned to one exponent E by what
+// they weigh: a group of mirror images (fix_group) whose weights are below 2^-k
+// takes part in E, the largest biased exponent, with e - k, and its weights are
+// stored times 2^k.  A double M * 2^(e-1075) becomes Q = M << 5 >> (E + k - e), a
+// 58-bit integer.  The mirror-symmetry components (GpOrbit) are exact integer
+// sums of up to four Q (60 bits).  A weight is w * 2^(58+k), at most 1, rounded to
+// an integer.  Both factors are split as h * 2^30 + l, |l| <= 2^29, and a product
+// keeps h*h (accumulated on its own) and h*l + l*h (accumulated together); l*l, at
+// most one unit of Q, is dropped.  With sum |w| 2^k <= 15 over a state's cells
+// (the host picks k so; sum |w| <= 4 is checked, FixOrbit::ok) neither
+// accumulator passes 2^62 and no result 2^62.  The 64-bit results, in units of
+// 2^(E-1080), are rounded to double once.  Error: a unit per cell for its
+// alignment and its dropped product, and the final rounding, against one FP64
+// rounding per multiply-add before: RMS 0.35 to 0.8 of FP64's wherever in the
+// stencil one value stands out (tests/test_fixed_recon.py,
+// tests/test_fixed_recon_groups.py).  With one exponent and no k a large value in
+// an outer cell (weight ~0.05) left the states 3 to 20 times FP64's error.
 //
-// Not representable that way, and decided per variable and stencil: a largest
-// exponent below 58 (values under 2^-965) gives zero states; one of 2040 and
-// up (values over 2^1017, infinities, NaN) gives NaN states, hence a NaN flux
-// as the FP64 sums' overflow in HLLC does.
+// Not representable that way, and decided per variable and stencil: E below 58
+// (values under 2^-965) gives zero states; 2040 and up (values over 2^1017, where
+// k lowers E up to 2^1023; infinities, NaN) gives NaN states, hence a NaN flux as
+// the FP64 sums' overflow in HLLC does.
 #pragma once
 #include <stdint.h>
 
@@ -55,6 +59,29 @@ GPM_HD long long fix_shift(long long v, unsigned n) {
 #else
     return v >> (n > 63 ? 63 : n);
 #endif
+}
+
+// The group of stencil value i (the order below): 0 the cell itself, 1 and 2 its
+// neighbours along n and t, 3 and 4 the next ones, 5 the corners.
+GPM_HD constexpr int fix_group(int i) { return i == 0 ? 0 : i < 9 ? (i + 1) / 2 : 5; }
+
+// The stencil values q(i), decoded, aligned by their exponents e and their groups'
+// k into v; returns E.
+template <int NP, class Load>
+GPM_HD int fix_align(const int* k, int* e, long long* v, Load q) {
+    int E = 0;
+#ifdef __CUDACC__
+#pragma unroll
+#endif
+    for (int i = 0; i < NP; i++) {
+        if (i) e[i] -= k[fix_group(i)];
+        E = e[i] > E ? e[i] : E;
+    }
+#ifdef __CUDACC__
+#pragma unroll
+#endif
+    for (int i = 0; i < NP; i++) v[i] = fix_shift(q(i), (unsigned)(E - e[i]));
+    return E;
 }
 
 GPM_HD long long fix_wide(int a, int b) { return (long long)a * b; }

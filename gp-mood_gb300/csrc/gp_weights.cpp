@@ -172,37 +172,71 @@ extern "C" void gpm_fix_orbits(GpWeights* w, int ngp) {
                     ok = ok && fabs(w->zt[o][far][g][mn[m]] - z) <= 1e-14 &&
                          fabs(w->zt[o][near][ngp - 1 - g][mt[m]] - z) <= 1e-14;
                 }
-            for (int mid = 0; mid < (ngp == 3 ? 2 : 1); mid++) {
-                double z[13] = {0.0}, c[13];
+            double c[2][13];  // the components' weights, of the first and the middle Gauss point
+            const int mids = ngp == 3 ? 2 : 1;
+            for (int mid = 0; mid < mids; mid++) {
+                double z[13] = {0.0};
                 for (int m = 0; m < np; m++) z[axis == 0 ? m : tr[m]] = w->zt[o][near][mid][m];  // (n, t) frame
                 // 0 (0,0), 1 (-1,0), 2 (0,1), 3 (1,0), 4 (0,-1), 5 (-1,-1), 6 (-1,1), 7 (1,1), 8 (1,-1), 9 (0,-2),
                 // 10 (-2,0), 11 (0,2), 12 (2,0)
-                c[0] = z[0];
-                c[1] = 0.5 * (z[1] + z[3]);
-                c[2] = 0.5 * (z[10] + z[12]);
-                c[3] = 0.5 * (z[4] + z[2]);
-                c[4] = 0.5 * (z[9] + z[11]);
-                c[5] = 0.25 * (z[5] + z[8] + z[6] + z[7]);
-                c[6] = 0.5 * (z[1] - z[3]);
-                c[7] = 0.5 * (z[10] - z[12]);
-                c[8] = 0.25 * (z[5] - z[8] + z[6] - z[7]);
-                c[9] = 0.5 * (z[4] - z[2]);
-                c[10] = 0.5 * (z[9] - z[11]);
-                c[11] = 0.25 * (z[5] + z[8] - z[6] - z[7]);
-                c[12] = 0.25 * (z[5] - z[8] - z[6] + z[7]);
-                static const int nc[13] = {1, 2, 2, 2, 2, 4, 2, 2, 4, 2, 2, 4, 4};  // cells in each component
+                const double k[13] = {z[0],
+                                      0.5 * (z[1] + z[3]),
+                                      0.5 * (z[10] + z[12]),
+                                      0.5 * (z[4] + z[2]),
+                                      0.5 * (z[9] + z[11]),
+                                      0.25 * (z[5] + z[8] + z[6] + z[7]),
+                                      0.5 * (z[1] - z[3]),
+                                      0.5 * (z[10] - z[12]),
+                                      0.25 * (z[5] - z[8] + z[6] - z[7]),
+                                      0.5 * (z[4] - z[2]),
+                                      0.5 * (z[9] - z[11]),
+                                      0.25 * (z[5] + z[8] - z[6] - z[7]),
+                                      0.25 * (z[5] - z[8] - z[6] + z[7])};
+                memcpy(c[mid], k, sizeof k);
+            }
+            static const int nc[13] = {1, 2, 2, 2, 2, 4, 2, 2, 4, 2, 2, 4, 4};     // cells in each component
+            static const int group[13] = {0, 1, 3, 2, 4, 5, 1, 3, 5, 2, 4, 5, 5};  // fix_group of its cells
+            // sum of absolute weights times 2^k of the larger Gauss point
+            auto sum = [&](const int* k) {
+                double most = 0.0;
+                for (int mid = 0; mid < mids; mid++) {
+                    double s = 0.0;
+                    for (int i = 0; i < 13; i++) s += ldexp(fabs(c[mid][i]) * nc[i], k[group[i]]);
+                    if (!(s <= most)) most = s;
+                }
+                return most;
+            };
+            int* k = orb.k[axis];
+            ok = ok && sum(k) <= 4.0;
+            // the largest k <= 6 (an infinity's exponent stays out of range) that leave every weight at most 1,
+            // or 1/2, ..., with the sum in the accumulators' range
+            for (double most = 1.0; ok; most *= 0.5) {
+                for (int g = 1; g < 6; g++) {
+                    double largest = 0.0;
+                    for (int mid = 0; mid < mids; mid++)
+                        for (int i = 0; i < 13; i++)
+                            if (group[i] == g) largest = fmax(largest, fabs(c[mid][i]));
+                    k[g] = 0;
+                    while (largest > 0.0 && k[g] < 6 && ldexp(largest, k[g] + 1) <= most) k[g]++;
+                }
+                if (sum(k) <= 15.0) break;
+            }
+            for (int mid = 0; ok && mid < mids; mid++) {
                 static const int all[13] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12}, five[5] = {0, 1, 3, 6, 9};
                 const int n = o == 2 ? (mid ? 9 : 13) : (mid ? 4 : 5);
-                FixWeight* fw = mid ? orb.w1[axis] : orb.w0[axis];
-                double sum = 0.0;
+                FixWeight *one = mid ? orb.w1[axis] : orb.w0[axis], *grouped = mid ? orb.g1[axis] : orb.g0[axis];
                 for (int i = 0; i < n; i++) {
-                    const int k = o == 2 ? all[i] : five[i];
-                    sum += fabs(c[k]) * nc[k];
-                    const long long v = llrint(ldexp(c[k], 58));
-                    fw[i].h = (int)((v + (1LL << 29)) >> 30);
-                    fw[i].l = (int)(v - ((long long)fw[i].h << 30));
+                    const int j = o == 2 ? all[i] : five[i];
+                    auto fixed = [&](int bits) {
+                        const long long v = llrint(ldexp(c[mid][j], bits));
+                        FixWeight f;
+                        f.h = (int)((v + (1LL << 29)) >> 30);
+                        f.l = (int)(v - ((long long)f.h << 30));
+                        return f;
+                    };
+                    one[i] = fixed(58);
+                    grouped[i] = fixed(58 + k[group[j]]);
                 }
-                ok = ok && sum <= 4.0;
             }
         }
         orb.ok = ok;

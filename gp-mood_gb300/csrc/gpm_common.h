@@ -68,12 +68,15 @@ struct GpOrbit {
 // axis's own frame (n: along it, t: across it), order 5: [Q0 Q1p Q2p Q3p Q4p
 // Q5pp | Q1m Q2m Q5mp | Q3m Q4m Q5pm | Q5mm] with Q1, Q2 the pairs along n and
 // Q3, Q4 along t; order 3: [Q0 Q1p Q3p | Q1m | Q3m].  w0 is the first Gauss
-// point's, w1 (3 points) the middle one's, whose last two groups vanish.
+// point's, w1 (3 points) the middle one's, whose last two groups vanish.  g0, g1:
+// the same times 2^k of the component's cell group (fix_group), for stencils
+// aligned by fix_align; w0, w1 are those of stencils aligned to one exponent.
 struct FixWeight {
     int h, l;
 };
 struct FixOrbit {
-    FixWeight w0[2][13], w1[2][9];
+    FixWeight w0[2][13], w1[2][9], g0[2][13], g1[2][9];
+    int k[2][6];
     int ok;  // mirror symmetric and in the fixed-point form's range; 0: the first pass runs face by face instead
     int pad;
 };

@@ -389,25 +389,21 @@ struct XySmem {
 // Variable k's states on the two faces of one axis of the cell at tile
 // position `at`; sn, st: strides in cells along and across the axis.
 template <int ORD, int NGP, class S>
-__device__ __forceinline__ void recon_axis(const S& sm, const FixWeight* w0, const FixWeight* w1, int at, int sn, int st,
-                                           int k, double* lo, double* hi) {
+__device__ __forceinline__ void recon_axis(const S& sm, const FixOrbit& o, int axis, int at, int sn, int st, int k,
+                                           double* lo, double* hi) {
     constexpr int NP = np_of(ORD);
     const int off[13] = {0, -sn, sn, -st, st, -2 * sn, 2 * sn, -2 * st, 2 * st, -sn - st, sn - st, st - sn, sn + st};
     const unsigned short* ex = reinterpret_cast<const unsigned short*>(&sm.ex[0][0] + at) + k;
     const long long* q = reinterpret_cast<const long long*>(&sm.tile[0][0] + at) + k;
-    int e[NP], E = 0;
+    int e[NP];
 #pragma unroll
-    for (int i = 0; i < NP; i++) {
-        e[i] = ex[4 * off[i]];
-        E = max(E, e[i]);
-    }
+    for (int i = 0; i < NP; i++) e[i] = ex[4 * off[i]];
     long long v[NP];
-#pragma unroll
-    for (int i = 0; i < NP; i++) v[i] = fix_shift(q[4 * off[i]], (unsigned)(E - e[i]));
+    const int E = fix_align<NP>(o.k[axis], e, v, [&](int i) { return q[4 * off[i]]; });
     FixHalves c[NP];
     fix_components<ORD>(v, c);
     long long l[NGP], h[NGP];
-    fix_family<ORD, NGP>(w0, w1, c, l, h);
+    fix_family<ORD, NGP>(o.g0[axis], o.g1[axis], c, l, h);
     const bool ok = fix_exponent_ok(E);
     const double special = __longlong_as_double(fix_special_bits(E));
 #pragma unroll
@@ -468,7 +464,7 @@ __device__ __forceinline__ void xy_tile(const GridGeom& g, const FixOrbit& o, co
 #pragma unroll 1
                 for (int k = 0; k < 4; k++) {
                     double lo[NGP], hi[NGP];
-                    recon_axis<ORD, NGP>(sm, o.w0[axis], o.w1[axis], (cy + 3) * TW + cx + 3, sn, st, k, lo, hi);
+                    recon_axis<ORD, NGP>(sm, o, axis, (cy + 3) * TW + cx + 3, sn, st, k, lo, hi);
 #pragma unroll
                     for (int gp = 0; gp < NGP; gp++) {
                         if (give) sm.near[py][px][4 * gp + k] = lo[gp];
