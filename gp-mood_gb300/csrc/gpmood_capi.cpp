@@ -95,7 +95,6 @@ struct gpmood_ctx {
     DevScalars* hSc;              // pinned mirror
     GridBar* dBar;                // barrier of the cooperative MOOD loop, directly behind dSc
     GridBar* hBar;                // pinned mirror, directly behind hSc
-    int* hCount;                  // pinned troubled count
     double t;                     // host mirror of the time
     int niter;
     bool have_state;
@@ -503,7 +502,6 @@ void free_all(gpmood_ctx* c) {
     cudaFree(c->dList[0]); cudaFree(c->dList[1]); cudaFree(c->dTests); cudaFree(c->dSc); cudaFree(c->dStageOrd);
     for (int i = 0; i < 5; i++) cudaFree(c->dRk4[i]);
     if (c->hSc) cudaFreeHost(c->hSc);
-    if (c->hCount) cudaFreeHost(c->hCount);
     if (c->nn) nn_gate_destroy(c->nn);
     if (c->nnref) nn_ref_destroy(c->nnref);
     if (c->dCcw) cudaFree(c->dCcw);
@@ -639,7 +637,6 @@ int gpmood_create(const gpmood_params* p, gpmood_ctx** out) {
     c->dBar = reinterpret_cast<GridBar*>(c->dSc + 1);
 #undef ALLOC
     if (cudaMallocHost((void**)&c->hSc, sizeof(DevScalars) + sizeof(GridBar)) != cudaSuccess ||
-        cudaMallocHost((void**)&c->hCount, sizeof(int)) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
         fail(c, GPMOOD_E_CUDA, "pinned memory / stream creation failed");
         free_all(c);
@@ -906,7 +903,6 @@ int gpmood_advance(gpmood_ctx* c, int nsteps, int* steps_done) {
         c->ghosts_done = false;
         int rc = run_step(c, c->dU, c->dUr, true, bc_in);
         if (rc) return rc;
-        if (c->hSc->status & GPM_STATUS_DT) return fail(c, GPMOOD_E_DT, "Setdt produced dt = %g", c->hSc->dt);
         c->ghosts_done = true;
         double* tmp = c->dU;                   // U = Ur
         c->dU = c->dUr;

@@ -429,21 +429,6 @@ __device__ __forceinline__ void hllc_join(const double* ul, const double* ur, co
     for (int k = 0; k < 4; k++) F[k] = Fk[k] + S * (st[k] * dStar - u[k]);
 }
 
-__device__ __forceinline__ void hllc_dyn(const double* ul, const double* ur, int dir, double* F) {
-    hllc_join(ul, ur, c2p_dyn(ul, dir), c2p_dyn(ur, dir), dir, F);
-}
-#else
-__device__ __forceinline__ void hllc_dyn(const double* ul, const double* ur, int dir, double* F) {
-    const bool y = dir != 0;
-    NormalFlux f;
-    const bool adm = hllc_normal(ul[0], y ? ul[2] : ul[1], y ? ul[1] : ul[2], ul[3], ur[0], y ? ur[2] : ur[1],
-                                 y ? ur[1] : ur[2], ur[3], f);
-    F[0] = f.r;
-    F[1] = y ? f.t : f.n;
-    F[2] = y ? f.n : f.t;
-    F[3] = f.e;
-    nan_flux(!adm, F);
-}
 #endif
 
 // Left/right wave-speed bounds and physical fluxes, as HLL_Flux and LLF_Flux
@@ -570,27 +555,12 @@ __device__ __forceinline__ void riemann(int nflux, const double* ul, const doubl
     }
 }
 
+#if GPM_EXACT
 // Face flux with Gauss quadrature, mod_FE.f90:80-98: sum_g Fg*w_g from zero.
 template <int DIR, int NGP>
 __device__ __forceinline__ void quad_flux(const double (*uL)[4], const double (*uR)[4], const double* gw, double* F,
-                                          int nflux = 100) {
+                                          int nflux) {
     double acc[4];
-#if !GPM_EXACT
-    if (nflux == 100) {  // HLLC without branches; NaN flux at an inadmissible Gauss point
-        bool adm = true;
-#pragma unroll
-        for (int g = 0; g < NGP; g++) {
-            double Fg[4];
-            adm = hllc_select<DIR>(uL[g], uR[g], Fg) && adm;
-#pragma unroll
-            for (int k = 0; k < 4; k++) acc[k] = (g == 0) ? Fg[k] * gw[0] : acc[k] + Fg[k] * gw[g];
-        }
-#pragma unroll
-        for (int k = 0; k < 4; k++) F[k] = acc[k];
-        nan_flux(!adm, F);
-        return;
-    }
-#endif
 #pragma unroll
     for (int g = 0; g < NGP; g++) {
         double Fg[4];
@@ -598,14 +568,10 @@ __device__ __forceinline__ void quad_flux(const double (*uL)[4], const double (*
 #pragma unroll
         for (int k = 0; k < 4; k++) acc[k] = (g == 0) ? Fg[k] * gw[0] : acc[k] + Fg[k] * gw[g];
     }
-#if GPM_EXACT
 #pragma unroll
     for (int k = 0; k < 4; k++) F[k] = plus_zero(acc[k]);
-#else
-#pragma unroll
-    for (int k = 0; k < 4; k++) F[k] = acc[k];
-#endif
 }
+#endif
 
 // shock_detector, mod_subroutine_MOOD.f90:191-238, on Uin around (l, n), in
 // two side-effect-free halves that the MOOD loop may evaluate on different

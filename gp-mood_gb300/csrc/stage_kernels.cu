@@ -333,20 +333,18 @@ __global__ void __launch_bounds__(128, 4) k_flux_gp(StageArgs a, const __grid_co
 // The Riemann solve and quadrature a face function uses; the batched form has
 // its own in fast mode (batch_fast.cuh).
 struct FaceMath {
+#if GPM_EXACT
     template <int DIR, int NGP>
     static __device__ __forceinline__ void quad(const double (*uL)[4], const double (*uR)[4], const double* gw,
                                                 double* F, int nflux) {
         quad_flux<DIR, NGP>(uL, uR, gw, F, nflux);
     }
+#endif
     template <int DIR>
     static __device__ __forceinline__ void solve(int nflux, const double* uL, const double* uR, double* F) {
         riemann<DIR>(nflux, uL, uR, F);
     }
 };
-
-template <int DIR, int NP, int NGP, class M = FaceMath>
-__device__ __forceinline__ void face_global(const GridGeom& g, const GpWeights& w, int o, const double* __restrict__ uin,
-                                            size_t c0, double* F);
 
 #if !GPM_EXACT
 // ---------------------------------------------------------------------------
@@ -497,6 +495,30 @@ __device__ __forceinline__ void xy_tile(const GridGeom& g, const FixOrbit& o, co
             st_cell((axis == 0 ? fx : fy) + 4 * cidx(g, l, n), Cell{F[0], F[1], F[2], F[3]});
         }
     }
+}
+
+// One face, with stencils read straight from global memory.
+template <int DIR, int NP, int NGP, class M>
+__device__ __forceinline__ void face_global(const GridGeom& g, const GpWeights& w, int o, const double* __restrict__ uin,
+                                            size_t c0, double* F) {
+    constexpr int FL = DIR == 0 ? 2 : 1;
+    constexpr int FH = DIR == 0 ? 0 : 3;
+    const ptrdiff_t row = g.nx;
+    const size_t c1 = DIR == 0 ? c0 + 1 : c0 + g.nx;
+    double uL[NGP][4], uR[NGP][4];
+    {
+        Cell q[NP];
+#pragma unroll
+        for (int m = 0; m < NP; m++) q[m] = ld_cell(uin + 4 * (c0 + st_ox(m) + row * st_oy(m)));
+        recon_face<DIR, NP, NGP>(w, o, FL, q, uL);
+    }
+    {
+        Cell q[NP];
+#pragma unroll
+        for (int m = 0; m < NP; m++) q[m] = ld_cell(uin + 4 * (c1 + st_ox(m) + row * st_oy(m)));
+        recon_face<DIR, NP, NGP>(w, o, FH, q, uR);
+    }
+    M::template quad<DIR, NGP>(uL, uR, w.gw, F, g.num_flux);
 }
 
 // Edge item: faces k0 .. k0+EDGE_T-1 of the list [x faces (0,1..nf), y faces
@@ -845,31 +867,6 @@ void launch_update_detect(const StageArgs& a, const GpWeights& w, int cur, cudaS
 
 constexpr int LIST_CTAS_PER_SM = 4;
 
-// One face of the face list at its current order (min of the two cells),
-// with stencils read straight from global memory.
-template <int DIR, int NP, int NGP, class M>
-__device__ __forceinline__ void face_global(const GridGeom& g, const GpWeights& w, int o, const double* __restrict__ uin,
-                                            size_t c0, double* F) {
-    constexpr int FL = DIR == 0 ? 2 : 1;
-    constexpr int FH = DIR == 0 ? 0 : 3;
-    const ptrdiff_t row = g.nx;
-    const size_t c1 = DIR == 0 ? c0 + 1 : c0 + g.nx;
-    double uL[NGP][4], uR[NGP][4];
-    {
-        Cell q[NP];
-#pragma unroll
-        for (int m = 0; m < NP; m++) q[m] = ld_cell(uin + 4 * (c0 + st_ox(m) + row * st_oy(m)));
-        recon_face<DIR, NP, NGP>(w, o, FL, q, uL);
-    }
-    {
-        Cell q[NP];
-#pragma unroll
-        for (int m = 0; m < NP; m++) q[m] = ld_cell(uin + 4 * (c1 + st_ox(m) + row * st_oy(m)));
-        recon_face<DIR, NP, NGP>(w, o, FH, q, uR);
-    }
-    M::template quad<DIR, NGP>(uL, uR, w.gw, F, g.num_flux);
-}
-
 // The MOOD face phase, split by Gauss point.  A pass's face list is short
 // (the faces of the cells lowered in the previous pass), so the SMs hold one
 // or two warps each and a pass waits on one warp's chain of dependent FP64
@@ -939,60 +936,6 @@ __device__ __forceinline__ void face_gp_any(const StageArgs& a, const GpWeights&
     else face_gp_states<DIR, 1>(g, w, 0, a.uin, c0, gp, uL, uR, a.ccw);
     M::template solve<DIR>(g.num_flux, uL, uR, f.F);
     f.out = (DIR == 0 ? a.fx : a.fy) + 4 * c0;
-    f.gw = w.gw;
-}
-
-// The same face item with the direction a runtime value (0: x face between
-// c0 and c0+1, 1: y face between c0 and c0+nx): the reconstruction reads the
-// weights of the face's sides by index and HLLC runs as hllc_dyn, so a warp
-// may hold x and y faces at once; in the exact mode the bits are
-// face_gp_any's.  Other Riemann solvers branch on the direction.
-__device__ __forceinline__ void face_gp_dyn(const StageArgs& a, const GpWeights& w, size_t c0, int dir, int gp,
-                                            FaceGp& f) {
-    const GridGeom& g = a.g;
-    const size_t c1 = c0 + (dir == 0 ? (size_t)1 : (size_t)g.nx);
-    const int o = min((int)a.order[c0], (int)a.order[c1]);
-    const int FL = dir == 0 ? 2 : 1, FH = dir == 0 ? 0 : 3;
-    const ptrdiff_t row = g.nx;
-    double uL[4], uR[4];
-    if (o >= 5) {
-        Cell q[13];
-#pragma unroll
-        for (int m = 0; m < 13; m++) q[m] = ld_cell(a.uin + 4 * (c0 + st_ox(m) + row * st_oy(m)));
-        gp_recon_at<13>(&w.zt[2][FL][gp][0], q, uL);
-#pragma unroll
-        for (int m = 0; m < 13; m++) q[m] = ld_cell(a.uin + 4 * (c1 + st_ox(m) + row * st_oy(m)));
-        gp_recon_at<13>(&w.zt[2][FH][gp][0], q, uR);
-    } else {
-        const int NPo = o >= 3 ? 1 : 0;  // weight set: order 3 or 1
-        Cell q[5];
-#pragma unroll
-        for (int m = 0; m < 5; m++) q[m] = ld_cell(a.uin + 4 * (c0 + st_ox(m) + row * st_oy(m)));
-        if (o >= 3) gp_recon_at<5>(&w.zt[NPo][FL][gp][0], q, uL);
-        else gp_recon_at<1>(&w.zt[0][FL][gp][0], q, uL);
-        if (a.ccw) {
-            const int l0 = (int)(c0 % (size_t)g.nx) - 3, n0 = (int)(c0 / (size_t)g.nx) - 3;
-            double v1, v2;
-            cc_weights(g, a.ccw, l0, n0, &v1, &v2);
-            if (o >= 3) cc_blend<5>(v1, v2, q[0], uL);
-            else cc_blend<1>(v1, v2, q[0], uL);
-        }
-#pragma unroll
-        for (int m = 0; m < 5; m++) q[m] = ld_cell(a.uin + 4 * (c1 + st_ox(m) + row * st_oy(m)));
-        if (o >= 3) gp_recon_at<5>(&w.zt[NPo][FH][gp][0], q, uR);
-        else gp_recon_at<1>(&w.zt[0][FH][gp][0], q, uR);
-        if (a.ccw) {
-            const int l0 = (int)(c0 % (size_t)g.nx) - 3, n0 = (int)(c0 / (size_t)g.nx) - 3;
-            double v1, v2;
-            cc_weights(g, a.ccw, l0 + (dir == 0), n0 + (dir == 1), &v1, &v2);
-            if (o >= 3) cc_blend<5>(v1, v2, q[0], uR);
-            else cc_blend<1>(v1, v2, q[0], uR);
-        }
-    }
-    if (g.num_flux == 100) hllc_dyn(uL, uR, dir, f.F);
-    else if (dir == 0) riemann<0>(g.num_flux, uL, uR, f.F);
-    else riemann<1>(g.num_flux, uL, uR, f.F);
-    f.out = (dir == 0 ? a.fx : a.fy) + 4 * c0;
     f.gw = w.gw;
 }
 
