@@ -371,7 +371,7 @@ struct FaceMath {
 // Several small CTAs an SM keep some in the FP64 phase while others are in the
 // integer phase, and hide its latency: 2048^2 Sedov, order 5, 2 steps: 20.3 ms
 // with five of 4 rows, 24.5 with four, 19.6 with three of 8 rows (all with FP64 roots;
-// 17.4 now).
+// 16.6 now).
 constexpr int XT = 32, XY = 8;  // cells per tile of the batched form; XT is also the width here
 constexpr int TW = XT + 6;      // tile width with halo: 3 cells below, 3 above
 
@@ -1765,7 +1765,8 @@ const KernelTable table = {launch_bc,       launch_flux_all, launch_update_detec
 // Batched stepping: many independent problems of uneven size (batch_common.h).
 // Every phase of an RK stage is one persistent launch over all problems'
 // work items, so a whole step has a fixed launch sequence that is captured
-// once as a CUDA graph.  Per-problem arithmetic is the single-problem path's.
+// once as a CUDA graph.  Per-problem arithmetic is the single-problem path's in
+// the exact mode, and its own in the fast mode (batch_fast.cuh).
 #include "batch_common.h"
 
 namespace GPM_NS {
@@ -2036,8 +2037,8 @@ __device__ __forceinline__ void kb_face_gp(const BatchArgs& a, int cur, int nt, 
     else face_gp_any<1, EnsMath>(sa, w, side == 0 ? c - sa.g.nx : c, gp, f);
 }
 
-// The batch's whole MOOD loop in one cooperative launch (see k_mood_loop):
-// passes run until every problem's list is empty.  ntrb[2] is the stamp epoch,
+// The batch's whole MOOD loop in one cooperative launch: passes run until every
+// problem's list is empty, on all SMs and, once it is short, in CTA 0 (mood_sync).  ntrb[2] is the stamp epoch,
 // ntrb[4] the detected-cell total, ntrb[5] the pass count of the last stage.
 template <int NGP>
 __global__ void __launch_bounds__(MOOD_THREADS, 1) kb_mood_loop(BatchArgs a, GridBar* bar, int max_pass) {
@@ -2053,7 +2054,7 @@ __global__ void __launch_bounds__(MOOD_THREADS, 1) kb_mood_loop(BatchArgs a, Gri
             if (gtid == 0) a.ntrb[3] = 1;
             break;
         }
-        if (!solo && nt <= a.mood_solo) {  // as in k_mood_loop
+        if (!solo && nt <= a.mood_solo) {
             if (blockIdx.x != 0) return;
             solo = true;
             stid = threadIdx.x;
